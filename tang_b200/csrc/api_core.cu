@@ -130,6 +130,8 @@ int tq_ctx_create(int device, void* stream, tq_ctx** out) {
   const size_t ws_bytes = (size_t)kGemvSets * kGemvMaxGrid * 2 * 128 * sizeof(unsigned long long);
   if (cudaMalloc(&ctx->gemv_ws, ws_bytes) != cudaSuccess) return bail(TQ_ECUDA);
   if (cudaMemsetAsync(ctx->gemv_ws, 0, ws_bytes, ctx->stream) != cudaSuccess) return bail(TQ_ECUDA);
+  if (cudaMalloc(&ctx->wr_part, kWrPartBytes) != cudaSuccess || cudaMalloc(&ctx->wr_counters, kWrCounters * sizeof(int)) != cudaSuccess) return bail(TQ_ECUDA);
+  if (cudaMemsetAsync(ctx->wr_counters, 0, kWrCounters * sizeof(int), ctx->stream) != cudaSuccess) return bail(TQ_ECUDA);
   if (cudaMalloc(&ctx->skg_jobs, kSkgJobs * sizeof(int)) != cudaSuccess) return bail(TQ_ECUDA);
   if (cudaHostAlloc(reinterpret_cast<void**>(&ctx->host_err), 2 * sizeof(int), cudaHostAllocMapped) != cudaSuccess) return bail(TQ_ECUDA);
   ctx->host_err[0] = ctx->host_err[1] = 0;
@@ -149,6 +151,8 @@ int tq_ctx_destroy(tq_ctx* ctx) {
   if (ctx->dev_err) cudaFree(ctx->dev_err);
   if (ctx->gemv_ws) cudaFree(ctx->gemv_ws);
   if (ctx->skg_jobs) cudaFree(ctx->skg_jobs);
+  if (ctx->wr_part) cudaFree(ctx->wr_part);
+  if (ctx->wr_counters) cudaFree(ctx->wr_counters);
   if (ctx->gemm_ws2) cudaFree(ctx->gemm_ws2);
   if (ctx->hostx_ring) cudaFree(ctx->hostx_ring);
   if (ctx->hostx_tags) cudaFree(ctx->hostx_tags);   // (the epoch word sits behind the tags)
@@ -189,6 +193,7 @@ int tq_sync(tq_ctx* ctx) {
   if (code != 0) {
     cudaMemset(ctx->dev_err, 0, (1 + kTileCounters) * sizeof(int));   // a kernel that gave up may have left tile counters half counted
     cudaMemset(ctx->gemv_ws, 0, (size_t)kGemvSets * kGemvMaxGrid * 2 * 128 * sizeof(unsigned long long));
+    cudaMemset(ctx->wr_counters, 0, kWrCounters * sizeof(int));
     if (ctx->gemm_ws2) cudaMemset(ctx->gemm_ws2, 0, ctx->gemm_ws2_bytes);   // ... or parked partial sums
     if (code == 6)   // DERR_POSITION
       return fail(ctx, TQ_EINVAL, "a sequence position outside the KV cache reached a kernel (the access was skipped): positions must stay below max_seq");

@@ -13,6 +13,8 @@
 constexpr int kTileCounters = 1024;
 constexpr int kGemvSets = 6, kGemvMaxGrid = 512;
 constexpr int kSkgJobs = 4096;
+constexpr int kWrCounters = 65536;
+constexpr size_t kWrPartBytes = 40u << 20;
 constexpr int kHostXSlots = 64;
 constexpr size_t kHostXSlotBytes = 64 * 1024;
 
@@ -31,6 +33,10 @@ struct tq_ctx {
                                  // consecutive launches rotate through the sets (at most three kernels ever have
                                  // resident CTAs at a time: a CTA slot only frees when an older kernel's CTA exits)
   unsigned gemv_seq = 0;
+  // qgemm_wr.cuh: parked pieces and, zero between launches, the tiles summed per row block.  Fixed sizes: which kernel serves
+  // a shape must not depend on what ran before, nor on whether a graph is being captured.
+  float* wr_part = nullptr;      // [kWrPartBytes]
+  int* wr_counters = nullptr;    // [kWrCounters]
   int* host_err = nullptr;       // pinned [2]: the device's status word and the number of the last tq_sync whose signal kernel ran
   int* host_err_dev = nullptr;   // ... as the device sees it
   unsigned sync_seq = 0;
@@ -136,6 +142,10 @@ int qlinear_fused(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, const Ql
 
 // silu(gate) * up over the f32 output of a gate/up projection in the interleaved row order: gu [rows][2n] -> out [rows][n].
 int launch_swiglu_interleaved(tq_ctx* ctx, const float* gu, size_t rows, size_t n, void* out, int out_dtype);
+
+// Quantised linear layer for 9 to 16 rows of bf16 activations (qgemm_wr.cu); false: the shape is not for it.
+bool launch_qgemm_wr(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size_t ldx, size_t m, void* y, int y_dtype, size_t ldy,
+                     const float* residual, bool swiglu, int* status);
 
 int ensure_xprep(tq_ctx* ctx, size_t bytes);
 int ensure_gemm_ws2(tq_ctx* ctx, size_t bytes);

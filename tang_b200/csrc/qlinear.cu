@@ -975,6 +975,10 @@ int tq_qlinear(tq_ctx* ctx, const tq_qweight* w, const void* x_dev, int x_dtype,
     const size_t rows_staged = (m < chunk ? m : chunk) * combine;
     if (int st = ensure_xprep(ctx, rows_staged * kx * 2)) return st;
   }
+  if (direct) {
+    int st = TQ_OK;
+    if (launch_qgemm_wr(ctx, w, x_dev, ldx, m, y_dev, y_dtype, ldy, residual_dev, false, &st)) return st;
+  }
   if (direct && !residual_dev && m >= (size_t)umma_min_m(y_dtype) && umma_supported(w, m))
     return launch_qgemm_umma(ctx, w, x_dev, ldx, m, y_dev, y_dtype, ldy, y_dtype == TQ_F32 ? 2 : 1, nullptr);
   const size_t xe = x_dtype == TQ_F32 ? 4 : 2, ye = y_dtype == TQ_F32 ? 4 : 2;
@@ -1219,6 +1223,10 @@ int qlinear_fused(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, const Ql
     xin = norm->xn_tmp;
   }
   if (!swiglu) return tq_qlinear(ctx, w, xin, TQ_BF16, cols, m, y, y_dtype, ldy, nullptr);
+  {
+    int st = TQ_OK;
+    if (launch_qgemm_wr(ctx, w, xin, cols, m, y, y_dtype, ldy, nullptr, true, &st)) return st;
+  }
   // many rows: the tcgen05 kernel applies silu(gate) * up to its f32 sums itself.  As for every projection, the
   // result type decides the operand terms: exact products (two terms) for f32 results, the product rounded once to
   // bf16 (at most 2^-8 relative, half a step of the result type) for bf16 results.

@@ -444,3 +444,35 @@ def test_tensor_memory_gemm_long_k(dev, orc, m):
     y = dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.F32).to_vec().reshape(m, rows)
     dev.sync()
     assert rel_err(y[sel], want) < (TOL_F32 if m <= 128 else 2e-3)
+
+
+# The 9..16 row kernel (csrc/qgemm_wr.cuh): one slab and several, a short last slab, row blocks cut by warp boundaries in every
+# way, rows that end inside a row block, and the sizes on both sides of it.  7400 tiles (16 rows x 128 k) is its smallest matrix.
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(4096, 4096), (14813, 1024), (1073, 14464), (120000, 128)])
+def test_nine_to_sixteen_rows(dev, orc, kind, rows, cols):
+    import tang_b200 as tb
+    import torch
+
+    rng = np.random.default_rng(rows + cols + kind)
+    sc, pay = make_weight(rng, kind, rows, cols)
+    w = _upload(dev, kind, sc, pay, rows, cols)
+    deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double()      # (bit-exact: test_unpack_bit_exact)
+    for m in (8, 9, 13, 16, 17):
+        xbits, xf = bf16_round(rng.standard_normal((m, cols)).astype(np.float32))
+        want = (torch.from_numpy(xf).cuda().double() @ deq.T).cpu().numpy()
+        xb = dev.upload(xbits, tb.BF16)
+        y32 = dev.qlinear(xb, w, m, tb.F32).to_vec().reshape(m, rows)
+        y16 = dev.qlinear(xb, w, m, tb.BF16).to_vec().reshape(m, rows)
+        if 9 <= m <= 16:
+            # exact products, f32 sums: K additions of at most |y|-sized terms, each within 2^-24, against 1 % of the rms
+            assert rel_err(y32, want) < 1e-4, (kind, rows, cols, m)
+            assert np.array_equal(y16, bf16_round(y32)[0])
+            res = rng.standard_normal((m, rows)).astype(np.float32)
+            rbuf = dev.upload(res)
+            got = dev.qlinear(xb, w, m, out=rbuf, residual=rbuf).to_vec().reshape(m, rows)
+            assert np.array_equal(got, y32 + res)
+            again = dev.qlinear(xb, w, m, tb.F32).to_vec().reshape(m, rows)
+            assert np.array_equal(again, y32)                          # the pieces are added in one order
+        else:
+            assert rel_err(y32, want, floor_frac=0.05) < TOL_F32       # (17 rows: scales of 24 bits in two bf16 terms)
