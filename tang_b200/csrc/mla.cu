@@ -6,6 +6,8 @@
 // are also the value.  q_lat = W_qk[h] q_nope and o = W_uv[h] o_lat are per-head int8 GEMVs
 // (tq_mla_absorb_q / tq_mla_unabsorb, grouped launches of the quantised linear kernel).
 //
+// Two kernels: mla_umma.cu on the 5th-generation tensor cores from 64 heads on where a CTA keeps enough positions, and the one
+// here for fewer heads and short contexts.
 // Kernel: grid = (splits, heads/(16 HT), batch).  A CTA owns HT = 1 or 2 tiles of 16 heads (one MMA row tile
 // each, four warps per tile) and streams 64-position cache tiles, shared by its head tiles, through a cp.async
 // double buffer.  Per cache tile, warp w of a head tile scores positions 16w..16w+15 (Q fragments by ldmatrix
@@ -27,6 +29,10 @@ int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const v
                          const int* counts, const int* offsets, int max_rows, long long x_stride, long long y_stride,
                          void* y, int y_dtype, size_t ldy, const int* active = nullptr,
                          int max_active = 0, size_t total_rows = 0);
+
+bool mla_umma_supported(const void* q, const void* cache, size_t n_heads, size_t seq_stride, size_t batch);
+int launch_mla_umma(tq_ctx* ctx, const void* q, const void* cache, const int* lens, size_t batch, size_t n_heads, size_t seq_stride, size_t max_len,
+                    float scale, int n_splits, int chunk, void* out, float* part_o, float* part_ml);
 
 constexpr int kC = 512, kR = 64, kRow = kC + kR;         // latent, rope, cache row width
 constexpr int kMlaTile = 64;
@@ -264,19 +270,45 @@ __global__ void __launch_bounds__(kMlaThreads * HT) mla_decode_kernel(const MlaP
   }
 }
 
-__global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, const float* part_ml, int n_splits,
-                                                          __nv_bfloat16* out) {
+// Merges the splits of one (sequence, head): the splits' factors are formed once, then every thread adds two columns with the
+// loads of eight splits in flight (one sequence of 4096, 32 splits: 8.7 -> 3 us behind the attention).  `unit`: the maxima's
+// unit in powers of two.
+constexpr int kMlaMaxSplits = 512;
+__global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, const float* part_ml, int n_splits, float unit, __nv_bfloat16* out) {
+  __shared__ float w[kMlaMaxSplits + 1];
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t bh = blockIdx.x;
-  float M = -FLT_MAX;
-  for (int s = 0; s < n_splits; ++s) M = fmaxf(M, part_ml[(bh * n_splits + s) * 2]);
-  float L = 0.f;
-  for (int s = 0; s < n_splits; ++s) L += part_ml[(bh * n_splits + s) * 2 + 1] * exp2f((part_ml[(bh * n_splits + s) * 2] - M) * kLog2eM);
-  for (int d = threadIdx.x; d < kC; d += 256) {
-    float O = 0.f;
-    for (int s = 0; s < n_splits; ++s)
-      O += part_o[(bh * n_splits + s) * kC + d] * exp2f((part_ml[(bh * n_splits + s) * 2] - M) * kLog2eM);
-    out[bh * kC + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + bh * n_splits;
+  if (threadIdx.x < 32) {
+    float M = -FLT_MAX, L = 0.f;
+    for (int s = threadIdx.x; s < n_splits; s += 32) M = fmaxf(M, ml[s].x);
+    M = warp_max(M);
+    for (int s = threadIdx.x; s < n_splits; s += 32) {
+      const float2 v = ml[s];
+      const float f = exp2f((v.x - M) * unit);
+      w[s] = f;
+      L += v.y * f;
+    }
+    L = warp_sum(L);
+    if (threadIdx.x == 0) w[kMlaMaxSplits] = L;
   }
+  __syncthreads();
+  const float2* src = reinterpret_cast<const float2*>(part_o + bh * n_splits * kC) + threadIdx.x;
+  float2 o = make_float2(0.f, 0.f);
+  for (int s0 = 0; s0 < n_splits; s0 += 8) {
+    float2 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = s0 + i < n_splits ? src[(size_t)(s0 + i) * (kC / 2)] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float f = s0 + i < n_splits ? w[s0 + i] : 0.f;
+      o.x += v[i].x * f;
+      o.y += v[i].y * f;
+    }
+  }
+  const float L = w[kMlaMaxSplits];
+  *reinterpret_cast<__nv_bfloat162*>(out + bh * kC + 2 * threadIdx.x) = __floats2bfloat162_rn(L > 0.f ? o.x / L : 0.f, L > 0.f ? o.y / L : 0.f);
 }
 
 __global__ void mla_place_rope_kernel(const __nv_bfloat16* q_rope, __nv_bfloat16* q_full, size_t n_bh) {
@@ -464,14 +496,30 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   TQ_REQUIRE(ctx, max_len > 0, "tq_mla_decode: max_len must bound the sequence lengths");
   const int HT = n_heads % 32 == 0 ? 2 : 1;   // head tiles per CTA
   const int B = (int)batch, HG = (int)(n_heads / (16 * HT));
-  const int tiles = ((int)max_len + kMlaTile - 1) / kMlaTile;
-  int want = (2 * ctx->sm_count + B * HG - 1) / (B * HG);
-  int max_splits = (tiles + 1) / 2;
-  if (max_splits < 1) max_splits = 1;
-  int n_splits = want < 1 ? 1 : (want > max_splits ? max_splits : want);
-  const int tps = (tiles + n_splits - 1) / n_splits;
-  n_splits = (tiles + tps - 1) / tps;
-  if (n_splits < 1) n_splits = 1;
+  // The tcgen05 kernel where every CTA of about one wave keeps eight tiles of 32 positions; below that its prologue (queries,
+  // tensor memory) costs more than it saves (one sequence of 4096, 128 heads: the layer 80.7 us with the mma.sync kernel, 87.0).
+  const int base = 2 * B * (int)((n_heads + 127) / 128), tiles32 = ((int)max_len + 31) / 32;
+  int want = ctx->sm_count / base;
+  if (want < 1) want = 1;
+  if (want > kMlaMaxSplits) want = kMlaMaxSplits;
+  const bool umma = tiles32 / want >= 8 && mla_umma_supported(q_full_bf16_dev, cache_bf16_dev, n_heads, seq_stride, batch);
+  int n_splits, chunk;
+  if (umma) {
+    const int tps = (tiles32 + want - 1) / want;
+    n_splits = (tiles32 + tps - 1) / tps;
+    chunk = tps * 32;
+  } else {
+    const int tiles = ((int)max_len + kMlaTile - 1) / kMlaTile;
+    want = (2 * ctx->sm_count + B * HG - 1) / (B * HG);
+    int max_splits = (tiles + 1) / 2;
+    if (max_splits < 1) max_splits = 1;
+    if (max_splits > kMlaMaxSplits) max_splits = kMlaMaxSplits;
+    n_splits = want < 1 ? 1 : (want > max_splits ? max_splits : want);
+    const int tps = (tiles + n_splits - 1) / n_splits;
+    n_splits = (tiles + tps - 1) / tps;
+    if (n_splits < 1) n_splits = 1;
+    chunk = (tps > 0 ? tps : 1) * kMlaTile;
+  }
   MlaParams p;
   p.q = static_cast<const __nv_bfloat16*>(q_full_bf16_dev);
   p.cache = static_cast<const __nv_bfloat16*>(cache_bf16_dev);
@@ -479,7 +527,7 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   p.seq_stride = seq_stride;
   p.n_heads = (int)n_heads;
   p.n_splits = n_splits;
-  p.chunk = (tps > 0 ? tps : 1) * kMlaTile;
+  p.chunk = chunk;
   p.scale = softmax_scale;
   p.out = static_cast<__nv_bfloat16*>(o_lat_bf16_dev);
   p.part_o = nullptr;
@@ -489,6 +537,14 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
     if (int st = ensure_scratch(ctx, n_part * (kC + 2) * sizeof(float))) return st;
     p.part_o = static_cast<float*>(ctx->scratch);
     p.part_ml = p.part_o + n_part * kC;
+  }
+  if (umma) {
+    if (int st = launch_mla_umma(ctx, q_full_bf16_dev, cache_bf16_dev, lens_dev, batch, n_heads, seq_stride, max_len, softmax_scale, n_splits, chunk,
+                                 o_lat_bf16_dev, p.part_o, p.part_ml))
+      return st;
+    if (n_splits > 1) TQ_CUDA(ctx, launch_k(ctx, mla_combine_kernel, dim3((unsigned)(batch * n_heads)), dim3(256), 0, (const float*)p.part_o,
+                                            (const float*)p.part_ml, n_splits, 1.f, p.out));
+    return TQ_OK;
   }
   static thread_local int attr_dev = -1;   // the attribute is per device
   if (attr_dev != ctx->device) {
@@ -502,9 +558,8 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   ctx->launches++;
   TQ_CUDA(ctx, cudaGetLastError());
   if (n_splits > 1) {
-    mla_combine_kernel<<<(unsigned)(batch * n_heads), 256, 0, ctx->stream>>>(p.part_o, p.part_ml, n_splits, p.out);
-    ctx->launches++;
-    TQ_CUDA(ctx, cudaGetLastError());
+    TQ_CUDA(ctx, launch_k(ctx, mla_combine_kernel, dim3((unsigned)(batch * n_heads)), dim3(256), 0, (const float*)p.part_o, (const float*)p.part_ml,
+                          n_splits, kLog2eM, p.out));
   }
   return TQ_OK;
 }

@@ -236,3 +236,38 @@ def test_mla_layer_matches_oracle(dev, orc, d, H, q_lora, B, lens):
     assert np.array_equal(out2.to_vec().reshape(B, d), got.astype(np.float32))
     g.free()
     full.destroy()
+
+
+# The attention core on the tensor cores (csrc/mla_umma.cu): heads that fill the tile and that do not, one split and several,
+# splits without positions, lengths around the 32-position tiles, flat and sharply peaked scores; what lies behind a sequence's
+# end in the cache is NaN.  The queries are given, so the result may differ by its own rounding to bf16 (at most 2^-8 = 3.9e-3 of the
+# value) and f32 sums only.
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,B,lens,sharp", [(128, 80, [256, 255, 257, 33, 32, 31, 1, 0] * 10, 1.0), (64, 3, [9000, 31, 4097], 1.0),
+                                            (144, 2, [8191, 5000], 6.0), (80, 1, [9473], 30.0), (16, 2, [9000, 77], 6.0)])
+def test_attention_core(dev, H, B, lens, sharp):
+    import ctypes as C
+
+    import tang_b200 as tb
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    rows = max(lens) + 3
+    q = (torch.randn((B, H, C_ + R_), device="cuda", generator=g) * sharp).bfloat16()
+    cache = torch.randn((B, rows, C_ + R_), device="cuda", generator=g).bfloat16()
+    for b, n in enumerate(lens):
+        cache[b, n:] = float("nan")
+    out = torch.full((B, H, C_), float("nan"), device="cuda").bfloat16()
+    lb = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    scale = 1.0 / np.sqrt(NOPE + R_)
+    dev._check(dev._L.tq_mla_decode(dev._ctx, C.c_void_p(q.data_ptr()), C.c_void_p(cache.data_ptr()), C.c_void_p(lb.data_ptr()), B, H, C_, R_,
+                                    rows * (C_ + R_), max(lens), scale, C.c_void_p(out.data_ptr())))
+    dev.sync()
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert not out[b].any()
+            continue
+        kv = cache[b, :n].double()
+        want = (q[b].double() @ kv.T * scale).softmax(-1) @ kv[:, :C_]
+        assert rel_err(out[b].double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, (b, n)
