@@ -17,6 +17,7 @@ constexpr int kWrCounters = 65536;
 constexpr size_t kWrPartBytes = 40u << 20;
 constexpr int kHostXSlots = 64;
 constexpr size_t kHostXSlotBytes = 64 * 1024;
+constexpr size_t kBounceYBytes = 1u << 20;
 
 struct tq_ctx {
   int device = 0;
@@ -68,6 +69,8 @@ struct tq_ctx {
   uint8_t* hostx_ring = nullptr;     // [kHostXSlots][kHostXSlotBytes]
   unsigned* hostx_tags = nullptr;    // [kHostXSlots]
   unsigned hostx_seq = 0;
+  uint8_t* bounce = nullptr;         // pinned [kHostXSlotBytes + kBounceYBytes]: a waiting host-vector call's x and y; made by the first such call
+  void* bounce_dev = nullptr;        // ... as the device sees it
   unsigned* hostx_epoch = nullptr;   // device word: replays of captured graphs that stage host vectors (bumped by the graph's first such call)
   bool hostx_epoch_pending = false;  // a capture is open and has not bumped the word yet
   unsigned long long ws_generation = 0;        // bumped whenever a workspace is freed and reallocated: graphs recorded
