@@ -110,9 +110,11 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
     cp_async_commit();
   };
 
-  float o[16][2];  // row g (head), d = 8*dn + 2t, +1
+  // row g (head), d = 8*dn + 2t, +1; [2], [3]: the same of the products with P's second term, which sits in the rows that a group
+  // of up to eight heads leaves empty: one mma.sync (about 32 cycles of a scheduler) for both terms.
+  float o[16][4];
 #pragma unroll
-  for (int dn = 0; dn < 16; ++dn) o[dn][0] = o[dn][1] = 0.f;
+  for (int dn = 0; dn < 16; ++dn) o[dn][0] = o[dn][1] = o[dn][2] = o[dn][3] = 0.f;
   float m_run = -FLT_MAX, l_run = 0.f;  // l_run: this lane's share of the row sum
 
   if (n_tiles > 0) load_tile(0, 0);
@@ -171,6 +173,8 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
       for (int dn = 0; dn < 16; ++dn) {
         o[dn][0] *= alpha;
         o[dn][1] *= alpha;
+        o[dn][2] *= alpha;
+        o[dn][3] *= alpha;
       }
       // P enters the tensor core as bf16; a second, residual term (p - bf16(p)) keeps 16 significant
       // bits so the result does not depend on bf16's 8-bit rounding of the probabilities.
@@ -190,16 +194,8 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
       for (int dp = 0; dp < 8; ++dp) {
         uint32_t vb[4];
         ldmatrix_x4_trans(vb, vrow + 32 * dp);
-        float acc0[4] = {o[2 * dp][0], o[2 * dp][1], 0.f, 0.f};
-        float acc1[4] = {o[2 * dp + 1][0], o[2 * dp + 1][1], 0.f, 0.f};
-        mma_bf16_16816(acc0, pa0, 0u, pa2, 0u, vb[0], vb[1]);
-        mma_bf16_16816(acc1, pa0, 0u, pa2, 0u, vb[2], vb[3]);
-        mma_bf16_16816(acc0, pb0, 0u, pb2, 0u, vb[0], vb[1]);
-        mma_bf16_16816(acc1, pb0, 0u, pb2, 0u, vb[2], vb[3]);
-        o[2 * dp][0] = acc0[0];
-        o[2 * dp][1] = acc0[1];
-        o[2 * dp + 1][0] = acc1[0];
-        o[2 * dp + 1][1] = acc1[1];
+        mma_bf16_16816(o[2 * dp], pa0, pb0, pa2, pb2, vb[0], vb[1]);
+        mma_bf16_16816(o[2 * dp + 1], pa0, pb0, pa2, pb2, vb[2], vb[3]);
       }
     }
     __syncthreads();  // everyone is done with `buf` before it is refilled
@@ -212,8 +208,8 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
   float* mml = mo + 4 * 8 * kHD;                                // [4 warps][8 rows][2]
 #pragma unroll
   for (int dn = 0; dn < 16; ++dn) {
-    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t] = o[dn][0];
-    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t + 1] = o[dn][1];
+    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t] = o[dn][0] + o[dn][2];
+    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t + 1] = o[dn][1] + o[dn][3];
   }
   if (t == 0) {
     mml[(warp * 8 + g) * 2] = m_run;
