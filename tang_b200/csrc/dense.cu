@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) dgemv_kernel(const __grid_const
 
 // ------------------------------------------------------------------------------------------------ tcgen05 GEMM
 // The weights are the UMMA M operand (128 features per tile), the activation rows the N operand (16..256), both K-major
-// in the 128-byte swizzle; D[128 x rows] in tensor memory.  Warp 0 copies, warp 1 multiplies, warps 4..11 store.
+// in the 128-byte swizzle; D[128 x rows] in tensor memory.  Warps 0 and 3 copy, warp 1 multiplies, warps 4..11 store.
 constexpr int kDuThreads = 384;
 constexpr int kDuEpiWarp0 = 4, kDuEpiWarps = 8;
 constexpr int kDuMaxStages = 12;
@@ -280,7 +280,7 @@ dgemm_umma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 2);          // the weights' copy and the activations'
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -323,16 +323,20 @@ dgemm_umma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
   auto w_row = [&](int ft, int tt) { return ft * kUmmaRows + (p.grouped ? p.grp.jobs[tt].x * (int)p.grp.group_rows : 0); };
   auto x_row = [&](int tt) { return p.grouped ? p.grp.jobs[tt].y : tt * p.ntok; };
 
-  if (warp == 0) {
+  if (warp == 0 || warp == 3) {
+    // Warp 0 copies the weights, warp 3 the activations: one thread issuing both boxes of a stage is a bound of its own (a box of
+    // 128 to 256 rows keeps the issuing thread for hundreds of cycles, a stage's products take 512 at most).
+    const bool weights = warp == 0;
     if (lane == 0) {
       // The weights of the first stages do not depend on the previous kernel: their copies start before the wait.
       int ft, tt, kb0, kbn, z;
       int pre = 0;
-      if (!p.grouped && (int)blockIdx.x < p.n_tiles) {
+      const uint32_t bytes = weights ? (uint32_t)kUmmaRows * 128u : (uint32_t)p.ntok * 128u;
+      if (weights && !p.grouped && (int)blockIdx.x < p.n_tiles) {
         coords(blockIdx.x, ft, tt, kb0, kbn, z);
         pre = min(S, kbn);
         for (int s = 0; s < pre; ++s) {
-          mbar_arrive_expect_tx(&full[s], stage_bytes);
+          mbar_arrive_expect_tx(&full[s], bytes);
           tma_load_2d(tiles_s + (size_t)s * stage_bytes, &w_map, (kb0 + s) * kUmmaK, ft * kUmmaRows, &full[s]);
         }
       }
@@ -343,18 +347,16 @@ dgemm_umma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
       const int n_tiles = tiles_total();
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         coords(tile, ft, tt, kb0, kbn, z);
-        const int wr = w_row(ft, tt), xr = x_row(tt);
+        const int row = weights ? w_row(ft, tt) : x_row(tt);
         for (int kb = 0; kb < kbn; ++kb) {
-          uint8_t* st = tiles_s + (size_t)s * stage_bytes;
           if (pre > 0) {
             --pre;
           } else {
             ok = !*failed && mbar_wait_spin(&empty[s], ph ^ 1u);
             if (!ok) { give_up(DERR_EMPTY_WAIT); break; }
-            mbar_arrive_expect_tx(&full[s], stage_bytes);
-            tma_load_2d(st, &w_map, (kb0 + kb) * kUmmaK, wr, &full[s]);
+            mbar_arrive_expect_tx(&full[s], bytes);
+            tma_load_2d(tiles_s + (size_t)s * stage_bytes + (weights ? 0 : kUmmaRows * 128), weights ? &w_map : &x_map, (kb0 + kb) * kUmmaK, row, &full[s]);
           }
-          tma_load_2d(st + kUmmaRows * 128, &x_map, (kb0 + kb) * kUmmaK, xr, &full[s]);
           if (++s == S) {
             s = 0;
             ph ^= 1u;
