@@ -33,7 +33,11 @@ int all_to_all_v(tq_ctx* ctx, tq_comm* comm, const void* send_dev, const size_t*
                  const size_t* recv_off, const size_t* recv_bytes);
 int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, size_t m_total,
                               const int* counts, const int* offsets, const int* active, int max_active, int max_rows,
-                              int expected_rows, void* y, int y_dtype, size_t ldy);
+                              int expected_rows, void* y, int y_dtype, size_t ldy, int terms = 2, int swiglu = 0);
+struct UmmaGroups;
+bool umma_supported(const tq_qweight* w, size_t m);
+int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size_t ldx, size_t m, void* y, int y_dtype,
+                      size_t ldy, int terms, const UmmaGroups* grp, int swiglu);
 bool umma_grouped_supported(const tq_qweight* w, int n_groups);
 
 // One CTA of eight warps per token; warp w computes the logits of experts w, w + 8, ...
@@ -599,12 +603,14 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   const size_t expected = n / (size_t)c.n_experts;
   const bool tensor_path = expected >= 24 && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
   if (tensor_path) {
+    // silu(gate) * up in the projection's epilogue, from the same f32 sums (two terms per weight although the result is bf16): the
+    // f32 round trip of the 2 f wide projection and its kernel are gone
     TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, n, cnt, offs, active, max_active, (int)T, (int)(expected * 3 / 2),
-                                      gu, TQ_F32, 2 * f));
+                                      act, TQ_BF16, f, 2, 2));
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_gate_up, nl, xs, d, cap, cnt, offs, (int)T, 0, 0, gu, TQ_F32, 2 * f, active, max_active, n));
+    TQ_STEP(tq_swiglu(ctx, gu, gu + f, TQ_F32, 2 * f, n, f, act, TQ_BF16));
   }
-  TQ_STEP(tq_swiglu(ctx, gu, gu + f, TQ_F32, 2 * f, n, f, act, TQ_BF16));
   if (tensor_path) {
     TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_down, nl, act, f, n, cnt, offs, active, max_active, (int)T, (int)(expected * 3 / 2), yo,
                                       TQ_F32, d));
@@ -612,8 +618,13 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_down, nl, act, f, cap, cnt, offs, (int)T, 0, 0, yo, TQ_F32, d, active, max_active, n));
   }
   for (size_t i = 0; i < m->sh_gate_up.size() && Ts > 0; ++i) {
-    TQ_STEP(tq_qlinear(ctx, m->sh_gate_up[i], h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
-    TQ_STEP(tq_swiglu(ctx, shgu, shgu + f, TQ_F32, 2 * f, Ts, f, shact, TQ_BF16));
+    // (the same epilogue where the projection fills the GPU without splitting K: below, the split form and the separate kernel)
+    if (Ts >= 1024 && m->sh_gate_up[i]->kind != TQ_I8_ROW && umma_supported(m->sh_gate_up[i], Ts) && d % 8 == 0) {
+      TQ_STEP(launch_qgemm_umma(ctx, m->sh_gate_up[i], h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
+    } else {
+      TQ_STEP(tq_qlinear(ctx, m->sh_gate_up[i], h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
+      TQ_STEP(tq_swiglu(ctx, shgu, shgu + f, TQ_F32, 2 * f, Ts, f, shact, TQ_BF16));
+    }
     TQ_STEP(tq_qlinear(ctx, m->sh_down[i], shact, TQ_BF16, f, Ts, sh + i * Ts * d, TQ_F32, d, nullptr));
   }
   moe_combine_local_kernel<<<dim3((unsigned)T, (unsigned)((d + 1023) / 1024)), 256, 0, ctx->stream>>>(yo, slot, idl, w, (c.n_shared && Ts) ? sh : nullptr, (int)c.n_shared,

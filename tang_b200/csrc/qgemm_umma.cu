@@ -38,7 +38,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.stages, RS = p.raw_stages, KT = p.kt;
-  const int rb0 = blockIdx.x * (kUmmaRows / kTileRows);        // first 16-row block
+  // the eight 16-row blocks of this CTA: neighbours, or (swiglu 2) four gate blocks with their up blocks behind each
+  auto row_block = [&](int i) {
+    return p.swiglu == 2 ? (i & 1) * (p.n_rows / (2 * kTileRows)) + (int)blockIdx.x * 4 + (i >> 1) : (int)blockIdx.x * (kUmmaRows / kTileRows) + i;
+  };
   int m0 = blockIdx.y * p.ntok * kTokTiles;                    // first token of this CTA
   int m_end = p.m_total;                                       // rows at or beyond this are not this CTA's to store
   const uint8_t* tile_base = p.tiles;
@@ -104,7 +107,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
         if (!mbar_wait_spin(&raw_empty[r], rph ^ 1u)) { give_up(DERR_EMPTY_WAIT); break; }
         mbar_arrive_expect_tx(&raw_full[r], 8u * kcs * TB);
         for (int i = 0; i < 8; ++i)
-          bulk_g2s(raw_s + ((size_t)(r * 8 + i) * KT) * TB, tile_base + ((size_t)(rb0 + i) * p.kc_total + kc_begin + t0) * TB,
+          bulk_g2s(raw_s + ((size_t)(r * 8 + i) * KT) * TB, tile_base + ((size_t)row_block(i) * p.kc_total + kc_begin + t0) * TB,
                    kcs * TB, &raw_full[r], pol_w);
         if (++r == RS) {
           r = 0;
@@ -415,15 +418,18 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
             if (m < m_end) __stcg(part + (size_t)m * p.n_rows + n, v[i]);
           }
         } else if (p.swiglu) {
-          // lane l holds output row n: gate rows are the lanes with (l & 15) < 8, their up rows sit eight lanes on
-          const int o_col = (n >> 4) * 8 + (lane & 7);
+          // A gate row's up row sits eight lanes on (interleaved rows), or sixteen (halves: lanes 0..15 hold a gate block, 16..31 its
+          // up block).  Of every two columns the gate lanes finish the first, the up lanes the second.
+          const int away = p.swiglu == 2 ? 16 : 8;
+          const bool is_up = lane & away;
+          const int o_col = p.swiglu == 2 ? (n >> 5) * 16 + (lane & 15) : (n >> 4) * 8 + (lane & 7);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float up = __shfl_down_sync(0xffffffffu, v[i], 8);
-            const int m = mt + c0 + i;
-            if ((lane & 8) == 0 && m < m_end) {
-              const float g = v[i];
-              const float act = g * (1.0f / (1.0f + expf(-g))) * up;   // the formula of swiglu_kernel, term for term
+          for (int i = 0; i < 16; i += 2) {
+            const float got = __shfl_xor_sync(0xffffffffu, is_up ? v[i] : v[i + 1], away);
+            const float g = is_up ? got : v[i], up = is_up ? v[i + 1] : got;
+            const int m = mt + c0 + i + is_up;
+            const float act = g * (1.0f / (1.0f + expf(-g))) * up;   // the formula of swiglu_kernel, term for term
+            if (m < m_end) {
               if (p.y_bf16) reinterpret_cast<__nv_bfloat16*>(p.y)[(size_t)m * p.ldy + o_col] = __float2bfloat16_rn(act);
               else reinterpret_cast<float*>(p.y)[(size_t)m * p.ldy + o_col] = act;
             }
@@ -496,7 +502,7 @@ bool umma_supported(const tq_qweight* w, size_t m) {
 // With `grp`: `grp->n_groups` weight matrices stacked by rows (experts); group e multiplies rows
 // offsets[e] .. +counts[e] of x (device arrays) and m is the total row count of x / y.
 int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size_t ldx, size_t m, void* y, int y_dtype,
-                      size_t ldy, int terms, const UmmaGroups* grp, bool swiglu) {
+                      size_t ldy, int terms, const UmmaGroups* grp, int swiglu) {
   if (w->kind == TQ_I8_ROW) terms = 1;   // exact with one term: the row scale is applied to the accumulator
   if (!encode_tiled()) return fail(ctx, TQ_EUNSUPPORTED, "cuTensorMapEncodeTiled is not available from this driver");
   TQ_REQUIRE(ctx, umma_supported(w, m), "tcgen05 GEMM: needs rows %% 128 == 0 and cols %% 128 == 0");
@@ -549,7 +555,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   // Few output tiles (narrow layers, small batches) leave most SMs idle: split K over gridDim.z.
   const int base_ctas = (int)(w->rows / kUmmaRows) * (int)n_tok_tiles;
   int splits = 1;
-  if (!grp && base_ctas < (ctx->sm_count * 3) / 4) {
+  if (!grp && swiglu != 2 && base_ctas < (ctx->sm_count * 3) / 4) {
     splits = ctx->sm_count / base_ctas;
     if (splits > w->n_kc / 4) splits = w->n_kc / 4;      // at least eight 64-k steps per CTA
     if (splits > 16) splits = 16;
@@ -610,7 +616,8 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.ts = ts;
   p.a_col0 = a_col0;
   p.y_bf16 = y_dtype == TQ_BF16;
-  p.swiglu = swiglu ? 1 : 0;
+  TQ_REQUIRE(ctx, swiglu != 2 || w->kind != TQ_I8_ROW, "tcgen05 GEMM: gate and up halves with row scales");
+  p.swiglu = swiglu;
   p.err = ctx->dev_err;
   p.splits = splits;
   p.kc_per_split = kc_per_split;
@@ -659,7 +666,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
 // Grouped entry for the other translation units: experts stacked by rows, rows of x / y grouped by expert.
 int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, size_t m_total,
                               const int* counts, const int* offsets, const int* active, int max_active, int max_rows,
-                              int expected_rows, void* y, int y_dtype, size_t ldy) {
+                              int expected_rows, void* y, int y_dtype, size_t ldy, int terms, int swiglu) {
   UmmaGroups g;
   g.n_groups = n_groups;
   g.counts = counts;
@@ -668,7 +675,7 @@ int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, co
   g.max_active = max_active;
   g.max_rows = max_rows;
   g.expected_rows = expected_rows;
-  return launch_qgemm_umma(ctx, w, x_bf16, ldx, m_total, y, y_dtype, ldy, y_dtype == TQ_F32 ? 2 : 1, &g, false);
+  return launch_qgemm_umma(ctx, w, x_bf16, ldx, m_total, y, y_dtype, ldy, terms, &g, swiglu);
 }
 
 bool umma_grouped_supported(const tq_qweight* w, int n_groups) {

@@ -156,3 +156,22 @@ def test_deepseek_v2_lite_shape_large_batches(dev, orc, T):
     want, _, _, _ = host.oracle(orc, hf[sample])
     assert_moe_close(got[sample], want, T)
     layer.destroy()
+
+
+@pytest.mark.parametrize("renorm", [False, True])
+def test_fused_gate_up_equals_the_separate_kernel(dev, renorm):
+    """Many tokens: gate and up halves meet in the projection's epilogue (csrc/qgemm_umma.cu, swiglu 2), for the routed experts
+    and, from 1024 tokens on, for the shared one.  The same tokens a few at a time take the other kernels: what differs is f32
+    summation order and, through it, single bf16 roundings of the SwiGLU output (the layer's bar above)."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(31 + renorm)
+    moe = HostMoe(rng, 256, 384, 4, 2, 1, renorm)
+    layer = moe.to_device(dev)
+    T = 1061
+    bits, _ = bf16_round(rng.standard_normal((T, 256)).astype(np.float32))
+    whole = layer.forward(dev.upload(bits, tb.BF16), T).to_vec().reshape(T, 256)
+    parts = np.concatenate([layer.forward(dev.upload(bits[t:t + 40], tb.BF16), min(40, T - t)).to_vec().reshape(-1, 256) for t in range(0, T, 40)])
+    worst, share = rel_err_profile(whole, parts)
+    assert worst < 1e-2 and share < 5e-3, (worst, share)
+    layer.destroy()
