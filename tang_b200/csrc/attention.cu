@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
   };
 
   // row g (head), d = 8*dn + 2t, +1; [2], [3]: the same of the products with P's second term, which sits in the rows that a group
-  // of up to eight heads leaves empty: one mma.sync (about 32 cycles of a scheduler) for both terms.
+  // of up to eight heads leaves empty: one mma.sync for both terms.
   float o[16][4];
 #pragma unroll
   for (int dn = 0; dn < 16; ++dn) o[dn][0] = o[dn][1] = o[dn][2] = o[dn][3] = 0.f;

@@ -442,33 +442,54 @@ dgemm_umma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
           for (int j = 0; j < 16; ++j)
             if (j < n) v[j] *= p.epi.row_scale[mb + j];
         }
-        // a half-warp's rows share a section, so the shuffles below are only ever needed by lanes that agree on the kind
+        // Sixteen values at a time without a branch between them: value by value through dense_store, with both sides of the
+        // gate formed in turn, the outputs of a 128 x 256 tile took longer than the products of 2048 k.  A half-warp's rows share
+        // a section, so the shuffles are only ever needed by lanes that agree on the kind.
         const bool glu = dst.kind == DENSE_GLU;
         if (__any_sync(0xffffffffu, glu)) {
           // lanes with (row & 8) == 0 hold gates, the others the matching ups: of every two columns the gate lanes
           // finish the first and the up lanes the second
-          const bool upper = lane & 8;
+          const int upper = (lane >> 3) & 1;
+          const bool f32 = __any_sync(0xffffffffu, glu && dst.f32);
+          float val[8];
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float give = upper ? v[j] : v[j + 1];
-            const float got = __shfl_xor_sync(0xffffffffu, give, 8);
-            if (glu) {
-              const float val = upper ? dense_glu(p.epi, got, v[j + 1]) : dense_glu(p.epi, v[j], got);
-              const int jj = upper ? j + 1 : j;
-              if (jj < n) dense_store(p.epi, dst, mb + jj, val);
-            }
+          for (int j = 0; j < 8; ++j) {
+            const float got = __shfl_xor_sync(0xffffffffu, upper ? v[2 * j] : v[2 * j + 1], 8);
+            const float gate = upper ? got : v[2 * j], up = upper ? v[2 * j + 1] : got;
+            val[j] = f32 ? dense_glu(p.epi, gate, up) : dense_glu_bf16(p.epi, gate, up);
           }
-          if (glu) continue;
+          if (glu) {
+            if (dst.base) {
+              char* at = dst.base + (long long)(mb + upper) * dst.ld;
+#pragma unroll
+              for (int j = 0; j < 8; ++j, at += 2 * dst.ld) {
+                if (2 * j + upper >= n) continue;
+                if (dst.f32) *reinterpret_cast<float*>(at) = val[j];
+                else *reinterpret_cast<__nv_bfloat16*>(at) = __float2bfloat16_rn(val[j]);
+              }
+            }
+            continue;
+          }
         }
+        if (!dst.base) continue;
         if (dst.kind == DENSE_RESID) {
-          if (dst.base) {
-            float old[16];
+          float old[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < n) old[j] = *reinterpret_cast<const float*>(dst.base + (long long)(mb + j) * dst.ld);
+          for (int j = 0; j < 16; ++j)
+            if (j < n) old[j] = *reinterpret_cast<const float*>(dst.base + (long long)(mb + j) * dst.ld);
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < n) *reinterpret_cast<float*>(dst.base + (long long)(mb + j) * dst.ld) = old[j] + p.epi.mult * v[j];
+          for (int j = 0; j < 16; ++j)
+            if (j < n) *reinterpret_cast<float*>(dst.base + (long long)(mb + j) * dst.ld) = old[j] + p.epi.mult * v[j];
+        } else if (dst.kind == DENSE_ROW && dst.act == DENSE_LINEAR) {
+          char* at = dst.base + (long long)mb * dst.ld;
+          if (dst.f32) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j, at += dst.ld)
+              if (j < n) *reinterpret_cast<float*>(at) = v[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j, at += dst.ld)
+              if (j < n) *reinterpret_cast<__nv_bfloat16*>(at) = __float2bfloat16_rn(v[j]);
           }
         } else {
 #pragma unroll

@@ -13,8 +13,7 @@
 //               exchange.  O is rescaled only when a maximum has grown by more than 2^8 (the reference of the exponentials is
 //               any number near the maximum), which is rare after the first tiles;
 // Measured, 128 heads: 16 sequences of 8.7k to 16.4k positions, the attention alone 437 us with the mma.sync kernel -> 177 us
-// (tiles of 32 positions, 1.4 us each; two stages instead of three: 296 us); mma.sync itself is the bound there, about
-// 32 cycles of a scheduler per m16n8k16.  What bounds it now is the chain copy -> scores -> softmax -> products of a tile with
+// (tiles of 32 positions, 1.4 us each; two stages instead of three: 296 us).  What bounds it now is the chain copy -> scores -> softmax -> products of a tile with
 // three tiles in flight (shared memory is full), not the 220 TFLOP/s that it reaches.
 // Splits over the positions are merged by mla_combine_kernel.  Every wait is bounded.
 #include <cfloat>
