@@ -65,6 +65,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// PAIR: both terms of the probabilities in one mma.sync, the second in the rows 8 to 15 that a group of up to eight heads leaves
+// empty, at twice the accumulators.
+template <bool PAIR>
 __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   // smem: K[2][64][272] | V[2][64][272]; reused for the warp merge at the end
@@ -110,11 +113,12 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
     cp_async_commit();
   };
 
-  // row g (head), d = 8*dn + 2t, +1; [2], [3]: the same of the products with P's second term, which sits in the rows that a group
-  // of up to eight heads leaves empty: one mma.sync for both terms.
-  float o[16][4];
+  constexpr int NO = PAIR ? 4 : 2;
+  float o[16][NO];  // row g (head), d = 8*dn + 2t, +1; [2], [3]: the same of the second term
 #pragma unroll
-  for (int dn = 0; dn < 16; ++dn) o[dn][0] = o[dn][1] = o[dn][2] = o[dn][3] = 0.f;
+  for (int dn = 0; dn < 16; ++dn)
+#pragma unroll
+    for (int c = 0; c < NO; ++c) o[dn][c] = 0.f;
   float m_run = -FLT_MAX, l_run = 0.f;  // l_run: this lane's share of the row sum
 
   if (n_tiles > 0) load_tile(0, 0);
@@ -170,12 +174,9 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
       l_run = l_run * alpha + psum;
       m_run = m_new;
 #pragma unroll
-      for (int dn = 0; dn < 16; ++dn) {
-        o[dn][0] *= alpha;
-        o[dn][1] *= alpha;
-        o[dn][2] *= alpha;
-        o[dn][3] *= alpha;
-      }
+      for (int dn = 0; dn < 16; ++dn)
+#pragma unroll
+        for (int c = 0; c < NO; ++c) o[dn][c] *= alpha;
       // P enters the tensor core as bf16; a second, residual term (p - bf16(p)) keeps 16 significant
       // bits so the result does not depend on bf16's 8-bit rounding of the probabilities.
       float ph[4], pl[4];
@@ -194,8 +195,21 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
       for (int dp = 0; dp < 8; ++dp) {
         uint32_t vb[4];
         ldmatrix_x4_trans(vb, vrow + 32 * dp);
-        mma_bf16_16816(o[2 * dp], pa0, pb0, pa2, pb2, vb[0], vb[1]);
-        mma_bf16_16816(o[2 * dp + 1], pa0, pb0, pa2, pb2, vb[2], vb[3]);
+        if constexpr (PAIR) {
+          mma_bf16_16816(o[2 * dp], pa0, pb0, pa2, pb2, vb[0], vb[1]);
+          mma_bf16_16816(o[2 * dp + 1], pa0, pb0, pa2, pb2, vb[2], vb[3]);
+        } else {
+          float acc0[4] = {o[2 * dp][0], o[2 * dp][1], 0.f, 0.f};
+          float acc1[4] = {o[2 * dp + 1][0], o[2 * dp + 1][1], 0.f, 0.f};
+          mma_bf16_16816(acc0, pa0, 0u, pa2, 0u, vb[0], vb[1]);
+          mma_bf16_16816(acc1, pa0, 0u, pa2, 0u, vb[2], vb[3]);
+          mma_bf16_16816(acc0, pb0, 0u, pb2, 0u, vb[0], vb[1]);
+          mma_bf16_16816(acc1, pb0, 0u, pb2, 0u, vb[2], vb[3]);
+          o[2 * dp][0] = acc0[0];
+          o[2 * dp][1] = acc0[1];
+          o[2 * dp + 1][0] = acc1[0];
+          o[2 * dp + 1][1] = acc1[1];
+        }
       }
     }
     __syncthreads();  // everyone is done with `buf` before it is refilled
@@ -208,8 +222,8 @@ __global__ void __launch_bounds__(kAttnThreads) gqa_decode_kernel(const GqaParam
   float* mml = mo + 4 * 8 * kHD;                                // [4 warps][8 rows][2]
 #pragma unroll
   for (int dn = 0; dn < 16; ++dn) {
-    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t] = o[dn][0] + o[dn][2];
-    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t + 1] = o[dn][1] + o[dn][3];
+    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t] = PAIR ? o[dn][0] + o[dn][NO - 2] : o[dn][0];
+    mo[((size_t)warp * 8 + g) * kHD + 8 * dn + 2 * t + 1] = PAIR ? o[dn][1] + o[dn][NO - 1] : o[dn][1];
   }
   if (t == 0) {
     mml[(warp * 8 + g) * 2] = m_run;
@@ -514,6 +528,13 @@ __global__ void kv_attention_f32_kernel(const float* q, const float* k_cache, co
   }
 }
 
+// Both terms in one instruction where several CTAs share an SM; a single wave waits for its own few tiles, and there the wider
+// accumulators cost more than they save (8B-shaped decode step: 64 sequences, 1024 CTAs, 7.25 -> 7.11 ms; one, 136 CTAs,
+// 1.762 -> 1.774).
+static auto decode_form(const tq_ctx* ctx, dim3 grid) {
+  return (long long)grid.x * grid.y * grid.z > 2LL * ctx->sm_count ? gqa_decode_kernel<true> : gqa_decode_kernel<false>;
+}
+
 int launch_gqa_decode(tq_ctx* ctx, const void* q, const void* k_cache, const void* v_cache, const int* lens, int B,
                       int n_heads, int n_kv, int head_dim, size_t seq_stride, int max_len, void* out, int out_dtype) {
   TQ_REQUIRE(ctx, head_dim == kHD, "tq_gqa_decode: head_dim must be %d", kHD);
@@ -556,11 +577,12 @@ int launch_gqa_decode(tq_ctx* ctx, const void* q, const void* k_cache, const voi
   const size_t smem = 4 * (size_t)kTileKeys * kRowBytes;
   static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the kernel
   if (!attr_set[ctx->device & 63]) {
-    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_set[ctx->device & 63] = true;
   }
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)B);
-  TQ_CUDA(ctx, launch_k(ctx, gqa_decode_kernel, grid, dim3(kAttnThreads), smem, p));
+  TQ_CUDA(ctx, launch_k(ctx, decode_form(ctx, grid), grid, dim3(kAttnThreads), smem, p));
   if (n_splits > 1)
     TQ_CUDA(ctx, launch_k(ctx, gqa_combine_kernel, dim3((unsigned)(B * n_heads)), dim3(kHD), 0, (const float*)p.part_o,
                           (const float*)p.part_ml, n_splits, out, p.out_f32));
@@ -683,7 +705,8 @@ int tq_gqa_decode_noalloc(tq_ctx* ctx, const void* q_dev, const void* k_cache_de
     void* ptr = nullptr;
     TQ_CUDA(ctx, cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
     TQ_REQUIRE(ctx, ptr != nullptr, "tq_gqa_decode_noalloc: the static scratch array has no device address");
-    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     g_noalloc_ptr[ctx->device] = ptr;
   }
   const int B = (int)batch, n_kv = (int)n_kv_heads, nh = (int)n_heads;
@@ -721,7 +744,7 @@ int tq_gqa_decode_noalloc(tq_ctx* ctx, const void* q_dev, const void* k_cache_de
   p.part_o = n_splits > 1 ? static_cast<float*>(g_noalloc_ptr[ctx->device]) : nullptr;
   p.part_ml = n_splits > 1 ? p.part_o + n_part * kHD : nullptr;
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)B);
-  gqa_decode_kernel<<<grid, kAttnThreads, smem, ctx->stream>>>(p);
+  decode_form(ctx, grid)<<<grid, kAttnThreads, smem, ctx->stream>>>(p);
   ctx->launches++;
   TQ_CUDA(ctx, cudaGetLastError());
   if (n_splits > 1) {
