@@ -9,11 +9,10 @@ constexpr int wr_depth(int kind) { return kind == Q8_F32 || kind == I8_ROW ? 4 :
 template <int KIND>
 static cudaError_t wr_launch(tq_ctx* ctx, const QWrParams& p, unsigned grid, size_t smem) {
   auto kern = qgemm_wr_kernel<KIND, wr_depth(KIND)>;
-  static size_t attr_bytes[64] = {};   // per device
-  const int dev = ctx->device & 63;
-  if (attr_bytes[dev] < smem) {
-    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
-    attr_bytes[dev] = smem;
+  static bool done[64] = {};   // per device; the same value from every thread
+  if (!done[ctx->device & 63]) {
+    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)) return e;
+    done[ctx->device & 63] = true;
   }
   return launch_k(ctx, kern, dim3(grid), dim3(32 * kWrWarps), smem, p);
 }
