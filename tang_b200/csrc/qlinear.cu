@@ -636,6 +636,9 @@ static bool launch_qgemm_skg(tq_ctx* ctx, const tq_qweight* w, int n_groups, con
   return true;
 }
 
+bool launch_qgemm_heads(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, int mx, long long x_stride, long long y_stride,
+                        void* y, int y_dtype, size_t ldy, int* status);
+
 int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, int mx,
                          const int* counts, const int* offsets, int max_rows, long long x_stride, long long y_stride,
                          void* y, int y_dtype, size_t ldy, const int* active, int max_active, size_t total_rows) {
@@ -643,6 +646,10 @@ int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const v
              "grouped qlinear: rows per group must be a multiple of 16");
   TQ_REQUIRE(ctx, w->cols == (size_t)w->n_kc * kTileK && ldx % 8 == 0 && ((uintptr_t)x_bf16 & 15) == 0 && (x_stride % 8) == 0,
              "grouped qlinear: K must be a multiple of 128 and activation rows 16-byte aligned");
+  if (!counts) {
+    int st = TQ_OK;
+    if (launch_qgemm_heads(ctx, w, n_groups, x_bf16, ldx, mx, x_stride, y_stride, y, y_dtype, ldy, &st)) return st;
+  }
   {
     int st = TQ_OK;
     if (launch_qgemm_skg(ctx, w, n_groups, static_cast<const __nv_bfloat16*>(x_bf16), ldx, mx, counts, offsets, max_rows, x_stride, y_stride, y,

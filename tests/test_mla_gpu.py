@@ -271,3 +271,38 @@ def test_attention_core(dev, H, B, lens, sharp):
         kv = cache[b, :n].double()
         want = (q[b].double() @ kv.T * scale).softmax(-1) @ kv[:, :C_]
         assert rel_err(out[b].double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, (b, n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("H,B", [(16, 1), (80, 8), (75, 9), (128, 16), (33, 33), (128, 64)])
+def test_per_head_products(dev, kind, H, B):
+    """W_UK and W_UV as grouped products of a short K (csrc/qgemm_heads.cu), row counts around the eight-row column tiles, head counts
+    whose row blocks do not fill the last CTA; exact products in f32 sums of at most 512 terms."""
+    import ctypes as C
+
+    import tang_b200 as tb
+    import torch
+    from util import make_weight
+
+    rng = np.random.default_rng(kind * 100 + H + B)
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    for rows, cols in ((C_, NOPE), (VD, C_)):
+        sc, pay = make_weight(rng, kind, H * rows, cols)
+        w = dev.upload_qarrays(kind, pay, sc, H * rows, cols)
+        deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double().view(H, rows, cols)
+        x = torch.randn((B, H, cols), device="cuda", generator=g).bfloat16()
+        rope = torch.zeros((B, H, R_), device="cuda").bfloat16()
+        torch.cuda.synchronize()
+        want = torch.einsum("bhc,hrc->bhr", x.double(), deq)
+        if rows == C_:
+            out = torch.empty((B, H, C_ + R_), device="cuda", dtype=torch.bfloat16)
+            dev._check(dev._L.tq_mla_absorb_q(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.data_ptr()), C.c_void_p(rope.data_ptr()), B, H, cols,
+                                              C.c_void_p(out.data_ptr())))
+            dev.sync()
+            assert rel_err(out[:, :, :C_].double().cpu().numpy(), want.cpu().numpy()) < 4.1e-3        # its own rounding to bf16: 2^-8
+        else:
+            out = torch.empty((B, H, VD), device="cuda")
+            dev._check(dev._L.tq_mla_unabsorb(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.data_ptr()), B, H, VD, C.c_void_p(out.data_ptr()), tb.F32))
+            dev.sync()
+            assert rel_err(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-3
