@@ -7,7 +7,7 @@
 // fragments straight from global memory (a head's rows are a few KB that its warps share in L1), and stores its results.  No
 // shared memory, no barrier, nothing to park.  Bound: the latency of two dependent loads, behind which the bytes (8.4 MB) hide.
 // The general kernel spent its time on setting up a ring per CTA for one or four tiles of K: 128 heads, one row 17.4 us for
-// [512, 128] and 8.5 for [128, 512], sixteen rows 18.4 and 19.9.
+// [512, 128] and 8.5 for [128, 512], sixteen rows 18.4 and 19.9, where the two now take 21 together (the layer 276 -> 259 us).
 #include "internal.h"
 #include "qgemm_mma.cuh"
 
