@@ -30,7 +30,7 @@ int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const v
                          void* y, int y_dtype, size_t ldy, const int* active = nullptr,
                          int max_active = 0, size_t total_rows = 0);
 
-bool mla_umma_supported(const void* q, const void* cache, size_t n_heads, size_t seq_stride, size_t batch);
+bool mla_umma_supported(const void* q, const void* cache, size_t n_heads, size_t seq_stride, size_t batch, size_t max_len);
 int launch_mla_umma(tq_ctx* ctx, const void* q, const void* cache, const int* lens, size_t batch, size_t n_heads, size_t seq_stride, size_t max_len,
                     float scale, int n_splits, int chunk, void* out, float* part_o, float* part_ml);
 
@@ -502,7 +502,7 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   int want = ctx->sm_count / base;
   if (want < 1) want = 1;
   if (want > kMlaMaxSplits) want = kMlaMaxSplits;
-  const bool umma = tiles32 / want >= 8 && mla_umma_supported(q_full_bf16_dev, cache_bf16_dev, n_heads, seq_stride, batch);
+  const bool umma = tiles32 / want >= 8 && mla_umma_supported(q_full_bf16_dev, cache_bf16_dev, n_heads, seq_stride, batch, max_len);
   int n_splits, chunk;
   if (umma) {
     const int tps = (tiles32 + want - 1) / want;

@@ -333,12 +333,14 @@ mla_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// The attention over one latent cache with `n_splits` splits of `chunk` positions each; false: the shape is not for it.
-bool mla_umma_supported(const void* q, const void* cache, size_t n_heads, size_t seq_stride, size_t batch) {
-  return n_heads >= 64 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)cache & 15) == 0 && seq_stride % 8 == 0 && seq_stride >= kMuRow && batch <= 65535 &&
+// False: the call is for the other kernel.  The tensor map wants aligned sequences that lie one behind the other: views that
+// overlap, and a stride that nobody reads because there is one sequence, stay with the kernel that forms its own addresses.
+bool mla_umma_supported(const void* q, const void* cache, size_t n_heads, size_t seq_stride, size_t batch, size_t max_len) {
+  return n_heads >= 64 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)cache & 15) == 0 && seq_stride % 8 == 0 && seq_stride >= max_len * kMuRow && batch <= 65535 &&
          encode_tiled() != nullptr;
 }
 
+// The attention over one latent cache with `n_splits` splits of `chunk` positions each.
 int launch_mla_umma(tq_ctx* ctx, const void* q, const void* cache, const int* lens, size_t batch, size_t n_heads, size_t seq_stride, size_t max_len,
                     float scale, int n_splits, int chunk, void* out, float* part_o, float* part_ml) {
   MlaUmmaParams p;
@@ -353,8 +355,7 @@ int launch_mla_umma(tq_ctx* ctx, const void* q, const void* cache, const int* le
   p.part_ml = part_ml;
   p.err = ctx->dev_err;
   CUtensorMap qm, km;
-  const size_t rows = max_len < seq_stride / kMuRow ? max_len : seq_stride / kMuRow;    // rows a box may touch
-  const cuuint64_t gdim[4] = {64, (cuuint64_t)rows, (cuuint64_t)kMuBoxes, (cuuint64_t)batch};
+  const cuuint64_t gdim[4] = {64, (cuuint64_t)max_len, (cuuint64_t)kMuBoxes, (cuuint64_t)batch};
   const cuuint64_t gstride[3] = {(cuuint64_t)kMuRow * 2, 128, (cuuint64_t)seq_stride * 2};
   const cuuint32_t box[4] = {64, (cuuint32_t)kMuTile, (cuuint32_t)kMuBoxes, 1}, estr[4] = {1, 1, 1, 1};
   if (!encode_bf16_k64(&qm, q, batch * n_heads, kMuRow, kMuRow, 128) ||

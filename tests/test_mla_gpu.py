@@ -273,6 +273,43 @@ def test_attention_core(dev, H, B, lens, sharp):
         assert rel_err(out[b].double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, (b, n)
 
 
+def attend(dev, q, cache, starts, lens, stride, max_len):
+    """tq_mla_decode on torch tensors, checked against 64 bits; `starts`: rows of `cache` at which the sequences begin.  Returns the
+    result and what it is in 64 bits."""
+    import ctypes as C
+
+    import torch
+
+    B, H = q.shape[:2]
+    out = torch.full((B, H, C_), float("nan"), device="cuda").bfloat16()
+    lb = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    scale = 1.0 / np.sqrt(NOPE + R_)
+    dev._check(dev._L.tq_mla_decode(dev._ctx, C.c_void_p(q.data_ptr()), C.c_void_p(cache.data_ptr()), C.c_void_p(lb.data_ptr()), B, H, C_, R_,
+                                    stride, max_len, scale, C.c_void_p(out.data_ptr())))
+    dev.sync()
+    want = torch.zeros((B, H, C_), device="cuda", dtype=torch.float64)
+    for b, n in enumerate(lens):
+        if n:
+            kv = cache[starts[b]:starts[b] + n].double()
+            want[b] = (q[b].double() @ kv.T * scale).softmax(-1) @ kv[:, :C_]
+    return out, want
+
+
+# Sequences that begin closer to one another than max_len rows: views of one cache that overlap, and a single sequence, whose stride says
+# nothing.  Both sizes are the tcgen05 kernel's but for the stride.  The bar is test_attention_core's.
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,n,step", [(40, 300, 100), (40, 300, 299), (1, 19000, 1), (1, 19000, 0)])
+def test_attention_core_over_close_sequences(dev, B, n, step):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(B + step)
+    q = torch.randn((B, 128, C_ + R_), device="cuda", generator=g).bfloat16()
+    cache = torch.randn(((B - 1) * step + n, C_ + R_), device="cuda", generator=g).bfloat16()
+    got, want = attend(dev, q, cache, [b * step for b in range(B)], [n - b % 7 for b in range(B)], step * (C_ + R_), n)
+    assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", [0, 1, 2, 3])
 @pytest.mark.parametrize("H,B", [(16, 1), (80, 8), (75, 9), (128, 16), (33, 33), (128, 64)])
