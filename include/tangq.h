@@ -128,7 +128,8 @@ TQ_API int tq_qlinear(tq_ctx* ctx, const tq_qweight* w, const void* x_dev, int x
 /* The reference call itself: q4_matvec(&QuantizedQ4, &[f64]) -> Vec<f64> (quantize.rs:256) and
  * q8_matvec (quantize.rs:227), with HOST vectors.  x_host [m, cols], y_host [m, rows]; dtype is
  * TQ_F64 (the reference's), TQ_F32 or TQ_BF16 (bit patterns) for both.  f64 input is narrowed to
- * f32 (on the device, after upload).  Synchronises. */
+ * f32.  Synchronises.  A pageable x_host is read when the call is made, a pinned one (two pinned f32 or bf16 vectors of few
+ * rows aside: tq_q_matvec_host_async) in its turn on the context's stream. */
 TQ_API int tq_q_matvec_host(tq_ctx* ctx, const tq_qweight* w, const void* x_host, void* y_host, int dtype, size_t m);
 
 /* The same call without the final wait, for a caller with several matvecs to run (a list of layers, a batch of

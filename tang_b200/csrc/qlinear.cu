@@ -1082,11 +1082,20 @@ __global__ void __launch_bounds__(256) stage_host_x_kernel(const void* x, int dt
   pdl_wait();   // kernels of a stream still complete in launch order
 }
 
-static void* pinned_alias(const void* host) {
+// What CUDA knows about a host vector: its device alias when it is pinned, and whether it is ordinary pageable memory.
+struct HostVector {
+  void* alias = nullptr;
+  bool pageable = false;
+};
+static HostVector host_vector(const void* host) {
+  HostVector v;
   cudaPointerAttributes attr;
-  if (cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer) return attr.devicePointer;
+  if (cudaPointerGetAttributes(&attr, host) == cudaSuccess) {
+    if (attr.type == cudaMemoryTypeHost) v.alias = attr.devicePointer;
+    v.pageable = attr.type == cudaMemoryTypeUnregistered;
+  }
   cudaGetLastError();   // an unregistered pointer is not an error here
-  return nullptr;
+  return v;
 }
 
 // Host vectors in pinned memory, bf16 or f32, up to eight staged rows: no copy is queued on the stream at all.  A
@@ -1142,10 +1151,11 @@ static bool matvec_host_pinned(tq_ctx* ctx, const tq_qweight* w, const void* xa,
   return true;
 }
 
-// A waiting call with ordinary (pageable) vectors, f64 among them: the values go through pinned buffers of the context's own,
+// A waiting call with an ordinary (pageable) x and a pageable or pinned y, f64 among them: the values go through pinned buffers of the context's own,
 // narrowed and widened by the host on the way, so that the call is the staging kernel, the matvec and the wait's signal instead
 // of two driver copies, two conversion kernels, a staging and a matvec (576 x 576 Q8, f64 vectors: 49.8 -> 30.7 us a call).  The
-// buffers are free again when the call returns.  Rows are padded to whole 128-k chunks, which the staging kernel reads 16 bytes
+// buffers are free again when the call returns.  The host reads x when the call is made: nothing queued on the stream can still be
+// writing pageable memory, but a pinned x may be the result of a call before, and waits for its turn on the stream.  Rows are padded to whole 128-k chunks, which the staging kernel reads 16 bytes
 // at a time.
 static bool matvec_host_bounce(tq_ctx* ctx, const tq_qweight* w, const void* x_host, void* y_host, int dtype, size_t m, int* status) {
   const size_t kx = (size_t)w->n_kc * kTileK, ny = m * w->rows;
@@ -1196,11 +1206,10 @@ static int matvec_host(tq_ctx* ctx, const tq_qweight* w, const void* x_host, voi
   TQ_REQUIRE(ctx, x_host && y_host, "tq_q_matvec_host: null vector");
   if (hostx_fits(ctx, w, dtype, m)) {
     int st = TQ_OK;
-    void* xa = dtype == TQ_F64 ? nullptr : pinned_alias(x_host);
-    void* ya = xa ? pinned_alias(y_host) : nullptr;
-    if (ya) {
-      if (matvec_host_pinned(ctx, w, xa, w->cols, ya, dtype, m, &st)) return st != TQ_OK ? st : (wait ? tq_sync(ctx) : TQ_OK);
-    } else if (wait && !ctx->capturing && matvec_host_bounce(ctx, w, x_host, y_host, dtype, m, &st)) {
+    const HostVector x = host_vector(x_host), y = host_vector(y_host);
+    if (x.alias && y.alias && dtype != TQ_F64) {
+      if (matvec_host_pinned(ctx, w, x.alias, w->cols, y.alias, dtype, m, &st)) return st != TQ_OK ? st : (wait ? tq_sync(ctx) : TQ_OK);
+    } else if (x.pageable && (y.pageable || y.alias) && wait && !ctx->capturing && matvec_host_bounce(ctx, w, x_host, y_host, dtype, m, &st)) {
       return st;
     }
   }
@@ -1223,12 +1232,10 @@ static int matvec_host(tq_ctx* ctx, const tq_qweight* w, const void* x_host, voi
   if (dtype != TQ_F64) {
     // A pinned result vector is visible to the device: the kernel stores y straight into it (posted writes over
     // the bus) and the separate device-to-host copy disappears.  x is still copied once: every CTA reads all of it.
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, y_host) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer) {
-      if (int st = tq_qlinear(ctx, w, xd, dev_dt, 0, m, attr.devicePointer, dev_dt, 0, nullptr)) return st;
+    if (void* ya = host_vector(y_host).alias) {
+      if (int st = tq_qlinear(ctx, w, xd, dev_dt, 0, m, ya, dev_dt, 0, nullptr)) return st;
       return wait ? tq_sync(ctx) : TQ_OK;
     }
-    cudaGetLastError();   // an unregistered pointer is not an error here
   }
   if (int st = tq_qlinear(ctx, w, xd, dev_dt, 0, m, s + off_y, dev_dt, 0, nullptr)) return st;
   const void* yd = s + off_y;

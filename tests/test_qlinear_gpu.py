@@ -330,6 +330,66 @@ def test_host_matvec_into_pinned_memory(dev, orc):
         assert np.array_equal(y_pinned, y_pageable)
 
 
+def test_host_matvec_reads_x_in_stream_order(dev, orc):
+    """A pinned x that queued work still writes, a pageable or f64 y: the waiting call sees what that work leaves behind."""
+    import ctypes as C
+
+    import torch
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(34)
+    first, second = (_upload(dev, 2, *make_weight(rng, 2, r, c), r, c) for r, c in ((512, 1024), (384, 512)))
+    slow, many = _upload(dev, 1, *make_weight(rng, 1, 4096, 8192), 4096, 8192), dev.alloc(2048 * 8192, tb.BF16)
+    out = dev.alloc(2048 * 4096, tb.F32)
+    for dt, tdt in ((tb.F32, torch.float32), (tb.BF16, torch.bfloat16), (tb.F64, torch.float64)):
+        xh = torch.from_numpy(rng.standard_normal(1024)).to(tdt).pin_memory()
+        mid = torch.zeros(512, dtype=tdt).pin_memory()
+        raw = mid.view(torch.int16).numpy().view(np.uint16) if dt == tb.BF16 else mid.numpy()   # (the same memory)
+        dev.q_matvec_host_async(first, xh.data_ptr(), mid.data_ptr(), dt, 1)
+        dev.sync()
+        want = dev._matvec_host(second, raw.copy(), 1)
+        got = np.zeros_like(want)
+        mid.zero_()
+        for _ in range(20):
+            dev.qlinear(many, slow, 2048, out=out)       # (milliseconds)
+        dev.q_matvec_host_async(first, xh.data_ptr(), mid.data_ptr(), dt, 1)
+        dev._check(dev._L.tq_q_matvec_host(dev._ctx, C.c_void_p(second.handle), C.c_void_p(mid.data_ptr()), C.c_void_p(got.ctypes.data), dt, 1))
+        assert np.abs(want.astype(np.float64)).max() > 0 and np.array_equal(got, want), dt
+
+
+# Pageable vectors through the context's pinned buffers: rows whose columns are no whole 128-k chunk, two f64 and f32 rows, results on
+# both sides of the buffers' 1 MB (the larger ones are copied by the driver), beside replays of a graph that stages its own vectors.
+@pytest.mark.parametrize("rows,cols,m", [(96, 100, 2), (33, 1056, 1), (262144, 64, 1), (262160, 64, 1), (131072, 32, 2), (131088, 32, 2)])
+def test_pageable_host_matvec(dev, orc, rows, cols, m):
+    import torch
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(rows + cols)
+    sc, pay = make_weight(rng, 2, rows, cols)
+    w = _upload(dev, 2, sc, pay, rows, cols)
+    small = _upload(dev, 1, *make_weight(rng, 1, 256, 1024), 256, 1024)
+    gx, gy = torch.from_numpy(rng.standard_normal(1024).astype(np.float32)).pin_memory(), torch.zeros(256).pin_memory()
+    dev.q_matvec_host_async(small, gx.data_ptr(), gy.data_ptr(), tb.F32, 1)
+    dev.sync()
+    graph_want = gy.numpy().copy()
+    dev.begin_capture()
+    dev.q_matvec_host_async(small, gx.data_ptr(), gy.data_ptr(), tb.F32, 1)
+    g = dev.end_capture()
+    x = rng.standard_normal((m, cols))
+    x32 = x.astype(np.float32)
+    bits, xb = bf16_round(x32)
+    deq = dev.dequantize(w)[0].astype(np.float64)
+    for v, vals, tol in ((x, x32, 1e-5), (x32, x32, 1e-5), (bits, xb, 4e-3)):   # f32 sums of up to 1056 exact products; the result's bf16
+        want = vals.astype(np.float64) @ deq.T
+        gy.zero_()
+        g.launch()
+        got = dev.q_matmul_host(w, v, m)
+        assert np.array_equal(gy.numpy(), graph_want)
+        gotf = (got.astype(np.uint32) << 16).view(np.float32) if got.dtype == np.uint16 else got
+        assert rel_err(gotf.astype(np.float64), want, floor_frac=1.0) < tol, v.dtype
+    g.free()
+
+
 def test_host_matvec_async_queue(dev, orc):
     """Several host-vector calls queued without a wait, one tq_sync at the end: every pinned result equals the
     waiting call's, bit for bit, whatever mix of weights and vector types was queued."""
