@@ -450,13 +450,11 @@ dgemm_umma_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
           // lanes with (row & 8) == 0 hold gates, the others the matching ups: of every two columns the gate lanes
           // finish the first and the up lanes the second
           const int upper = (lane >> 3) & 1;
-          const bool f32 = __any_sync(0xffffffffu, glu && dst.f32);
           float val[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float got = __shfl_xor_sync(0xffffffffu, upper ? v[2 * j] : v[2 * j + 1], 8);
-            const float gate = upper ? got : v[2 * j], up = upper ? v[2 * j + 1] : got;
-            val[j] = f32 ? dense_glu(p.epi, gate, up) : dense_glu_bf16(p.epi, gate, up);
+            val[j] = dense_glu(p.epi, upper ? got : v[2 * j], upper ? v[2 * j + 1] : got);
           }
           if (glu) {
             if (dst.base) {

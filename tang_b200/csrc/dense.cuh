@@ -132,14 +132,6 @@ __device__ __forceinline__ float dense_glu(const DenseEpilogue& e, float gate, f
   return e.glu == DENSE_GLU_SILU ? gate / (1.0f + expf(-gate)) * up : clamped_glu(gate, up, e.glu_limit, e.glu_alpha);
 }
 
-// The same with an approximate reciprocal (2 ulp of f32) in place of the division, which branches: several values interleave.
-// For results that are rounded to bf16 next.
-__device__ __forceinline__ float dense_glu_bf16(const DenseEpilogue& e, float gate, float up) {
-  const bool silu = e.glu == DENSE_GLU_SILU;
-  const float g = silu ? gate : fminf(gate, e.glu_limit), u = silu ? up : fminf(fmaxf(up, -e.glu_limit), e.glu_limit) + 1.0f;
-  return g * __fdividef(1.0f, 1.0f + expf(silu ? -g : -e.glu_alpha * g)) * u;
-}
-
 __device__ __forceinline__ void dense_store(const DenseEpilogue& e, const DenseDst& d, int m, float v) {
   if (!d.base) return;
   long long idx = m;

@@ -349,6 +349,39 @@ def test_grouped_linear(dev, dt, chunk, cols, feat, glu):
     L.tq_dweight_free(dev._ctx, h)
 
 
+@pytest.mark.parametrize("chunk", [8, 16, 48, 256])
+def test_grouped_glu_rounds_once(dev, chunk):
+    """A bf16 result of the gated unit is its f32 result rounded, whichever kernel a row count takes, also where the exponential nears
+    the end of f32: gates of -60 to -88.5 (from about -87.4 on 1 + e^-gate has no normal reciprocal) with ups as large."""
+    L, rows, cols, feat = dev._L, 300, 128, 40
+    rng = np.random.default_rng(chunk)
+    group = 2 * pad8(feat)
+    h = C.c_void_p()
+    dev._check(L.tq_dweight_create(dev._ctx, group, cols, BF16, C.byref(h)))
+    wg, wu = (np.ascontiguousarray(bf16_round((rng.standard_normal((feat, cols)) * 0.2).astype(np.float32))[1].astype(np.float32)) for _ in range(2))
+    wg[:, 0], wu[:, 0] = -1.0, 1.0
+    for i, w in enumerate((wg, wu)):
+        dev._check(L.tq_dweight_put(dev._ctx, h, C.c_void_p(w.ctypes.data), F32, feat, cols, 0, 0, i + 1))
+    xs = rng.standard_normal((rows, cols))
+    xs[:120] = 0
+    xs[:120, 0] = 60 + 0.5 * (np.arange(120) % 58)
+    x, xv = up(dev, xs, BF16)
+    jobs = [(0, i, min(chunk, rows - i), 0) for i in range(0, rows, chunk)]
+    got = []
+    for dt in (F32, BF16):
+        y = dev.alloc(rows * group // 2, dt)
+        dev._check(L.tq_dlinear_grouped(dev._ctx, h, ptr(x), cols, rows, ptr(ints(dev, jobs)), ptr(ints(dev, [len(jobs)])), len(jobs), chunk, group, None, None,
+                                        1000.0, 1.0, ptr(y), dt, group // 2))
+        got.append(y.to_vec().reshape(rows, group // 2)[:, :feat])
+    L.tq_dweight_free(dev._ctx, h)
+    assert np.array_equal(got[1], bf16_round(got[0])[0])
+    g, u = xv[:, :cols] @ wg.T.astype(np.float64), xv[:, :cols] @ wu.T.astype(np.float64)
+    want = g / (1 + np.exp(-g)) * (u + 1)
+    # exact gates and ups in the first rows: expf within 2 ulp, a reciprocal of 2^-128 keeps 21 bits; f32 sums of 128 products in the others
+    assert (np.abs(got[0] - want)[:120] <= 2e-6 * np.abs(want[:120])).all()
+    assert (np.abs(got[0] - want)[120:] <= 3e-5 * (1 + np.abs(want[120:]))).all()
+
+
 def test_bad_arguments_are_refused(dev):
     import tang_b200 as tb
 
