@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "qlayout.cuh"
+#include "qtile.cuh"
 
 namespace tq {
 
@@ -64,14 +65,6 @@ __host__ __device__ inline size_t qg_smem_bytes(int kind, int nt, int wr, int wk
   size_t pipe = (size_t)stages * qg_stage_bytes(kind, wr, wk * tpw, mx);
   size_t epi = (size_t)qg_epilogue_bytes(wr, wk, nt);
   return kQgHeaderBytes + qg_x_stride(wk * tpw) + (pipe > epi ? pipe : epi);
-}
-
-// mma with a zero accumulator input (the compiler then needs no registers for it)
-__device__ __forceinline__ void mma_bf16_16816_z(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                 uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 template <int KIND, int NT>

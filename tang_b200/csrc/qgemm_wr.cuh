@@ -11,17 +11,21 @@
 //     range alone: it copies its own tiles into its own ring (cp.async, D stages), so there is no barrier between warps and no
 //     producer, and every warp has D - 1 tiles in flight;
 //   * a fragment tile is read from the ring as the A operand (qlayout.cuh), unpacked to exact bf16 integers, multiplied
-//     with mma.sync, and the 32-block's scale multiplies the f32 partial sum: products are exact, only f32 sums round;
+//     with mma.sync, and the 32-block's scale multiplies the f32 partial sum: products are exact, only f32 sums round (qtile.cuh);
 //   * a (row block, slab) piece that does not hold all of K is parked as f32 fragments; the warp whose tiles complete a row
 //     block (a counter of tiles) adds the parked pieces in slab order, then in warp order: the same bits whoever that is.
 //     Nobody waits for anybody.  (Pieces of one CTA meeting in shared memory behind a CTA barrier at the end measured slower:
 //     18.5 against 16.0 us at 14336 x 4096, 24.1 against 18.9 at 4096 x 14336.)
-// Measured, 12 rows, f32 results, against the general kernel: 14336 x 4096 Q4 22.1 -> 16.0 us, 4096 x 14336 27.7 -> 18.9,
-// 6144 x 4096 17.0 -> 10.3, int8 24576 x 1536 32.3 -> 14.7, int8 7168 x 16384 67.9 -> 36.9.
+// Measured, 12 rows, f32 results, against the general kernel: 14336 x 4096 Q4 22.1 -> 16.6 us, 4096 x 14336 27.7 -> 17.2,
+// 6144 x 4096 17.0 -> 11.0, int8 24576 x 1536 32.3 -> 15.4, int8 7168 x 16384 67.9 -> 34.2.  Errors against 64 bits, relative to the
+// result's norm, Q4: 1.11e-7 -> 7.6e-8, 1.46e-7 -> 7.9e-8, 9.3e-8 -> 6.5e-8; int8 6.3e-8 -> 6.2e-8, 14336 x 4096 8.3e-8 -> 6.9e-8.
 #pragma once
+
+#include <cfloat>
 
 #include "common.cuh"
 #include "qlayout.cuh"
+#include "qtile.cuh"
 
 namespace tq {
 
@@ -62,12 +66,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
-__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
-}
-
 // Stores a finished row block: acc[i][c] holds row g (c < 2) or g + 8 of it, activation rows 8 i + 2 t + c % 2.
 template <int KIND>
 __device__ __forceinline__ void wr_store(const QWrParams& p, float (&acc)[kWrNT][4], int rb, int g, int t) {
@@ -204,35 +202,20 @@ __global__ void __launch_bounds__(32 * kWrWarps, 1) qgemm_wr_kernel(const QWrPar
       w4[0] = lds128(tile + 16 * lane);
       w4[1] = lds128(tile + 512 + 16 * lane);
     }
+    tile_sums<KIND, NT>(
+        acc, sc,
+        [&](int j, uint32_t (&a)[2][4]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t a[2][4];                 // [row half][k pairs (0,1) (2,3) (4,5) (6,7) of this lane's eight]
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if constexpr (kIs8) {
-          const uint2 v = lds64(tile + h * 1024 + (j >> 1) * 512 + 16 * lane + 8 * (j & 1));
-          dequant_i8_words(v.x, v.y, a[h]);
-        } else {
-          dequant_q4_word(j == 0 ? w4[h].x : j == 1 ? w4[h].y : j == 2 ? w4[h].z : w4[h].w, a[h]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const uint4 b = lds128(xk + (uint32_t)(8 * i * xs_stride + 64 * j));
-        if constexpr (KIND == I8_ROW) {
-          mma_bf16_16816(acc[i], a[0][0], a[1][0], a[0][1], a[1][1], b.x, b.y);
-          mma_bf16_16816(acc[i], a[0][2], a[1][2], a[0][3], a[1][3], b.z, b.w);
-        } else {
-          float d[4];
-          mma_bf16_zero(d, a[0][0], a[1][0], a[0][1], a[1][1], b.x, b.y);
-          mma_bf16_16816(d, a[0][2], a[1][2], a[0][3], a[1][3], b.z, b.w);
-          acc[i][0] = fmaf(sc[0][j], d[0], acc[i][0]);
-          acc[i][1] = fmaf(sc[0][j], d[1], acc[i][1]);
-          acc[i][2] = fmaf(sc[1][j], d[2], acc[i][2]);
-          acc[i][3] = fmaf(sc[1][j], d[3], acc[i][3]);
-        }
-      }
-    }
+          for (int h = 0; h < 2; ++h) {
+            if constexpr (kIs8) {
+              const uint2 v = lds64(tile + h * 1024 + (j >> 1) * 512 + 16 * lane + 8 * (j & 1));
+              dequant_i8_words(v.x, v.y, a[h]);
+            } else {
+              dequant_q4_word(j == 0 ? w4[h].x : j == 1 ? w4[h].y : j == 2 ? w4[h].z : w4[h].w, a[h]);
+            }
+          }
+        },
+        [&](int i, int j) { return lds128(xk + (uint32_t)(8 * i * xs_stride + 64 * j)); });
     if (++slot == D) slot = 0;
     ++done;
     if (++kc < skc && u + 1 < hi) continue;
@@ -254,22 +237,52 @@ __global__ void __launch_bounds__(32 * kWrWarps, 1) qgemm_wr_kernel(const QWrPar
         __threadfence();
         if (lane == 0) p.counters[rb] = 0;
         clear();
-        for (int s = 0; s < p.n_slabs; ++s) {
-          const int ks = min(p.skc, p.kc_total - s * p.skc);
-          const long long tot = (long long)p.n_rb * ks, f0 = (long long)rb * ks;
-          const int w0 = (int)(((f0 + 1) * n_w - 1) / tot), w1 = (int)(((f0 + ks) * n_w - 1) / tot);   // owners of the first and last tile
-          for (int wi = w0; wi <= w1; ++wi) {
+        // What each addition rounds away is kept aside and added last (two-sum, Knuth): the pieces of a sum without cancellation
+        // are as large as the result, and up to a dozen of them one after the other would cost more than all additions before.
+        float lost[NT][4] = {};
+        auto add = [&](float& a, float& low, float v) {
+          const float sum = a + v, b = sum - a;
+          low += (a - (sum - b)) + (v - b);
+          a = sum;
+        };
+        int first_w = 0, last_w = 0;          // of slab `lane` of these 32: owners of the first and the last tile of the row block
+        int s = 0, w0 = 0, w1 = 0, wi = 0;    // the next piece: slab s, warp wi of w0 .. w1
+        auto enter = [&]() {
+          if ((s & 31) == 0) {
+            const int ks = min(p.skc, p.kc_total - min(s + lane, p.n_slabs - 1) * p.skc);
+            const long long tot = (long long)p.n_rb * ks, f0 = (long long)rb * ks;
+            first_w = (int)(((f0 + 1) * n_w - 1) / tot);
+            last_w = (int)(((f0 + ks) * n_w - 1) / tot);
+          }
+          wi = w0 = __shfl_sync(0xffffffffu, first_w, s & 31);
+          w1 = __shfl_sync(0xffffffffu, last_w, s & 31);
+        };
+        enter();
+        while (s < p.n_slabs) {
+          float4 v[4][NT];                    // four pieces in flight
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool any = s < p.n_slabs;
             const float* src = p.part + (wi == w0 ? (size_t)s * p.n_rb + rb : heads + (size_t)s * n_w + wi) * kWrPiece + 4 * lane;
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-              const float4 v = __ldcg(reinterpret_cast<const float4*>(src + i * 128));
-              acc[i][0] += v.x;
-              acc[i][1] += v.y;
-              acc[i][2] += v.z;
-              acc[i][3] += v.w;
-            }
+            for (int i = 0; i < NT; ++i) v[k][i] = any ? __ldcg(reinterpret_cast<const float4*>(src + i * 128)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (any && ++wi > w1 && ++s < p.n_slabs) enter();
           }
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+              add(acc[i][0], lost[i][0], v[k][i].x);
+              add(acc[i][1], lost[i][1], v[k][i].y);
+              add(acc[i][2], lost[i][2], v[k][i].z);
+              add(acc[i][3], lost[i][3], v[k][i].w);
+            }
         }
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (fabsf(acc[i][c]) <= FLT_MAX) acc[i][c] += lost[i][c];      // (behind an infinity `lost` is NaN)
       }
     }
     if (mine) wr_store<KIND>(p, acc, rb, g, t);

@@ -536,3 +536,32 @@ def test_nine_to_sixteen_rows(dev, orc, kind, rows, cols):
             assert np.array_equal(again, y32)                          # the pieces are added in one order
         else:
             assert rel_err(y32, want, floor_frac=0.05) < TOL_F32       # (17 rows: scales of 24 bits in two bf16 terms)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(4096, 4096), (1536, 16384)])
+def test_nine_to_sixteen_rows_have_no_bias(dev, kind, rows, cols):
+    """Sums of positive terms: the tensor core truncates when it adds, so an accumulator that stayed there for all of K would be low by
+    its number of steps.  A 32-block's two steps lose less than 2^-23 of it each (1.2e-7 on average), f32 additions none."""
+    import tang_b200 as tb
+    import torch
+
+    rng = np.random.default_rng(cols + kind)
+    sc = rng.uniform(0.5, 1.5, rows if kind == 3 else (rows, cols // 32)).astype(np.float32)
+    if kind < 2:
+        lo, hi = (rng.integers(9, 16, (rows, cols // 2), dtype=np.uint8) for _ in range(2))
+        pay, sc = lo | (hi << 4), sc.astype(np.float16).view(np.uint16) if kind == 1 else sc
+    else:
+        pay = rng.integers(1, 128, (rows, cols), dtype=np.int8)
+    w = _upload(dev, kind, sc, pay, rows, cols)
+    deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double()
+    for m in (9, 16):
+        xbits, xf = bf16_round(np.abs(rng.standard_normal((m, cols))).astype(np.float32))   # (of all exponents: every addition rounds)
+        want = (torch.from_numpy(xf).cuda().double() @ deq.T).cpu().numpy()
+        y = dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.F32).to_vec().reshape(m, rows)
+        err = y / want - 1
+        # (rms: a result's own rounding 2.5e-8, sums of up to 24 tiles in a row, the pieces' sums rounded once)
+        assert abs(err.mean()) < 1.3e-7 and np.sqrt((err * err).mean()) < 7e-8, (err.mean(), np.sqrt((err * err).mean()))
+        xbits[1, cols // 2 + 1] = 0x7F80
+        y = dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.F32).to_vec().reshape(m, rows)
+        assert (y[1] == np.inf).all() and np.isfinite(np.delete(y, 1, 0)).all()
