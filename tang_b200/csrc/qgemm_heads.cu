@@ -3,13 +3,15 @@
 //
 //     y[m, e, n] = sum_k x[m, e, k] * q[e, n, k] * scale[e, n, k / 32]      (crates/tang-infer/src/quantize.rs:227-289, per head)
 //
-// A warp owns one 16-row block of one weight and all of its K: it reads the fragment tiles straight into registers, the activation
-// fragments straight from global memory (a head's rows are a few KB that its warps share in L1), and stores its results.  No
-// shared memory, no barrier, nothing to park.  Bound: the latency of two dependent loads, behind which the bytes (8.4 MB) hide.
-// The general kernel spent its time on setting up a ring per CTA for one or four tiles of K: 128 heads, one row 17.4 us for
-// [512, 128] and 8.5 for [128, 512], sixteen rows 18.4 and 19.9, where the two now take 21 together (the layer 276 -> 259 us).
+// A warp owns one 16-row block of one weight, up to sixteen activation rows and all of K: it reads the fragment tiles straight into
+// registers, the activation fragments straight from global memory (a head's rows are a few KB that its warps share in L1), and stores
+// its results.  No shared memory, no barrier, nothing to park.  Bound: the latency of two dependent loads, behind which the bytes
+// (8.4 MB) hide.  More rows are more CTAs that read the tiles from L2: all of 64 rows in one warp took 18.6 and 17.8 us (registers).
+// The general kernel spends its time on setting up a ring per CTA for one or four tiles of K.  int8, [512, 128] and [128, 512], us, the
+// general kernel -> this one: 128 heads, one row 8.1 / 6.6 -> 4.8 / 3.1, sixteen 16.9 / 15.3 -> 6.4 / 7.4, 64 54.7 / 46.6 -> 15.7 / 15.4;
+// 16 heads, one row, [512, 128] 4.6 -> 3.3.  Errors of f32 results of K = 512 against 64 bits 5.3e-8 -> 5.0e-8.
 #include "internal.h"
-#include "qgemm_mma.cuh"
+#include "qtile.cuh"
 
 namespace tq {
 
@@ -24,7 +26,8 @@ struct QHeadsParams {
 
 constexpr int kHeadsWarps = 8;
 
-template <int KIND, int NT>
+// ONE: K is one chunk
+template <int KIND, int NT, bool ONE>
 __global__ void __launch_bounds__(32 * kHeadsWarps) qgemm_heads_kernel(const QHeadsParams p) {
   constexpr bool kIs8 = KIND == Q8_F32 || KIND == I8_ROW;
   constexpr int WB = kIs8 ? 2048 : 1024, TB = WB + (KIND == Q4_F16 ? 128 : KIND == I8_ROW ? 0 : 256), NV = WB / 512;
@@ -42,12 +45,13 @@ __global__ void __launch_bounds__(32 * kHeadsWarps) qgemm_heads_kernel(const QHe
   pdl_wait();
   pdl_launch_dependents();
   if (!live) return;
+  const int m0 = 16 * blockIdx.y;
   const __nv_bfloat16* x = p.x + (size_t)e * p.x_stride + 8 * t;
   float acc[NT][4];
 #pragma unroll
   for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
 #pragma unroll 1
-  for (int kc = 0; kc < p.n_kc; ++kc, tile += TB) {
+  for (int kc = 0; kc < (ONE ? 1 : p.n_kc); ++kc, tile += TB) {
     float sc[2][4];
     if constexpr (KIND == Q4_F16) {
 #pragma unroll
@@ -63,37 +67,24 @@ __global__ void __launch_bounds__(32 * kHeadsWarps) qgemm_heads_kernel(const QHe
         sc[h][0] = v.x; sc[h][1] = v.y; sc[h][2] = v.z; sc[h][3] = v.w;
       }
     }
+    tile_sums<KIND, NT, ONE>(
+        acc, sc,
+        [&](int j, uint32_t (&a)[2][4]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t a[2][4];             // [row half][k pairs (0,1) (2,3) (4,5) (6,7) of this lane's eight]
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if constexpr (kIs8) {
-          const uint4& v = w[2 * h + (j >> 1)];
-          dequant_i8_words(j & 1 ? v.z : v.x, j & 1 ? v.w : v.y, a[h]);
-        } else {
-          const uint4& v = w[h];
-          dequant_q4_word(j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w, a[h]);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const uint4 b = 8 * i + g < p.mx ? *reinterpret_cast<const uint4*>(x + (size_t)(8 * i + g) * p.ldx + kc * kTileK + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (KIND == I8_ROW) {
-          mma_bf16_16816(acc[i], a[0][0], a[1][0], a[0][1], a[1][1], b.x, b.y);
-          mma_bf16_16816(acc[i], a[0][2], a[1][2], a[0][3], a[1][3], b.z, b.w);
-        } else {
-          float d[4];
-          mma_bf16_16816_z(d, a[0][0], a[1][0], a[0][1], a[1][1], b.x, b.y);
-          mma_bf16_16816(d, a[0][2], a[1][2], a[0][3], a[1][3], b.z, b.w);
-          acc[i][0] = fmaf(sc[0][j], d[0], acc[i][0]);
-          acc[i][1] = fmaf(sc[0][j], d[1], acc[i][1]);
-          acc[i][2] = fmaf(sc[1][j], d[2], acc[i][2]);
-          acc[i][3] = fmaf(sc[1][j], d[3], acc[i][3]);
-        }
-      }
-    }
-    if (kc + 1 < p.n_kc) load(tile + TB);
+          for (int h = 0; h < 2; ++h) {
+            if constexpr (kIs8) {
+              const uint4& v = w[2 * h + (j >> 1)];
+              dequant_i8_words(j & 1 ? v.z : v.x, j & 1 ? v.w : v.y, a[h]);
+            } else {
+              const uint4& v = w[h];
+              dequant_q4_word(j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w, a[h]);
+            }
+          }
+        },
+        [&](int i, int j) {
+          return m0 + 8 * i + g < p.mx ? *reinterpret_cast<const uint4*>(x + (size_t)(m0 + 8 * i + g) * p.ldx + kc * kTileK + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+        });
+    if (!ONE && kc + 1 < p.n_kc) load(tile + TB);
   }
   const int n0 = 16 * rb + g;
   float s[2] = {1.f, 1.f};
@@ -105,7 +96,7 @@ __global__ void __launch_bounds__(32 * kHeadsWarps) qgemm_heads_kernel(const QHe
   for (int i = 0; i < NT; ++i)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int m = 8 * i + 2 * t + (c & 1);
+      const int m = m0 + 8 * i + 2 * t + (c & 1);
       if (m >= p.mx) continue;
       const size_t o = (size_t)m * p.ldy + (size_t)e * p.y_stride + n0 + 8 * (c >> 1);
       const float v = acc[i][c] * s[c >> 1];
@@ -114,13 +105,15 @@ __global__ void __launch_bounds__(32 * kHeadsWarps) qgemm_heads_kernel(const QHe
     }
 }
 
+template <int KIND, bool ONE>
+static cudaError_t heads_launch(tq_ctx* ctx, const QHeadsParams& p) {
+  const dim3 grid((unsigned)((p.n_blocks + kHeadsWarps - 1) / kHeadsWarps), (unsigned)((p.mx + 15) / 16)), block(32 * kHeadsWarps);
+  if (p.mx <= 8) return launch_k(ctx, qgemm_heads_kernel<KIND, 1, ONE>, grid, block, 0, p);
+  return launch_k(ctx, qgemm_heads_kernel<KIND, 2, ONE>, grid, block, 0, p);
+}
 template <int KIND>
 static cudaError_t heads_launch(tq_ctx* ctx, const QHeadsParams& p) {
-  const dim3 grid((unsigned)((p.n_blocks + kHeadsWarps - 1) / kHeadsWarps)), block(32 * kHeadsWarps);
-  if (p.mx <= 8) return launch_k(ctx, qgemm_heads_kernel<KIND, 1>, grid, block, 0, p);
-  if (p.mx <= 16) return launch_k(ctx, qgemm_heads_kernel<KIND, 2>, grid, block, 0, p);
-  if (p.mx <= 32) return launch_k(ctx, qgemm_heads_kernel<KIND, 4>, grid, block, 0, p);
-  return launch_k(ctx, qgemm_heads_kernel<KIND, 8>, grid, block, 0, p);
+  return p.n_kc == 1 ? heads_launch<KIND, true>(ctx, p) : heads_launch<KIND, false>(ctx, p);
 }
 
 // `n_groups` weights stacked by rows (a multiple of 16 each), group e's rows start x_stride / y_stride elements into x / y; x 16-byte

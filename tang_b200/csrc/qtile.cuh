@@ -14,12 +14,12 @@ __device__ __forceinline__ void mma_bf16_16816_z(float (&d)[4], uint32_t a0, uin
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// acc += the tile's products.  words(j, a): the integers of block j as bf16 pairs, a[row half][k pairs (0,1) (2,3) (4,5) (6,7) of this
-// lane's eight]; rows(i, j): the same k of activation row 8 i + g; sc[row half][block]: the scales (not read for I8_ROW).
+// acc += the tile's products (FRESH: acc = them).  words(j, a): the integers of block j as bf16 pairs, a[row half][k pairs (0,1) (2,3) (4,5)
+// (6,7) of this lane's eight]; rows(i, j): the same k of activation row 8 i + g; sc[row half][block]: the scales (not read for I8_ROW).
 // mma.sync truncates when it adds to its accumulator, so only the two steps of a 32-block share one; the blocks of a tile are
 // added in f32 first, and the tile's sum to acc: one accumulator over all of K had a bias of 2e-7 of the int8 results, the blocks
 // added to acc one by one errors up to 1.25 times the general kernel's (24576 x 1536: 7.7e-8 there, 9.7e-8 one by one).
-template <int KIND, int NT, class Words, class Rows>
+template <int KIND, int NT, bool FRESH = false, class Words, class Rows>
 __device__ __forceinline__ void tile_sums(float (&acc)[NT][4], const float (&sc)[2][4], Words words, Rows rows) {
   float sum[NT][4];
 #pragma unroll
@@ -42,7 +42,7 @@ __device__ __forceinline__ void tile_sums(float (&acc)[NT][4], const float (&sc)
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[i][c] += sum[i][c];
+    for (int c = 0; c < 4; ++c) acc[i][c] = FRESH ? sum[i][c] : acc[i][c] + sum[i][c];
 }
 
 }  // namespace tq

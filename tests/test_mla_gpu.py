@@ -330,16 +330,48 @@ def test_per_head_products(dev, kind, H, B):
         deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double().view(H, rows, cols)
         x = torch.randn((B, H, cols), device="cuda", generator=g).bfloat16()
         rope = torch.zeros((B, H, R_), device="cuda").bfloat16()
-        torch.cuda.synchronize()
         want = torch.einsum("bhc,hrc->bhr", x.double(), deq)
         if rows == C_:
             out = torch.empty((B, H, C_ + R_), device="cuda", dtype=torch.bfloat16)
+            torch.cuda.synchronize()   # (`out` may be memory that the products above still use, on torch's stream)
             dev._check(dev._L.tq_mla_absorb_q(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.data_ptr()), C.c_void_p(rope.data_ptr()), B, H, cols,
                                               C.c_void_p(out.data_ptr())))
             dev.sync()
             assert rel_err(out[:, :, :C_].double().cpu().numpy(), want.cpu().numpy()) < 4.1e-3        # its own rounding to bf16: 2^-8
         else:
             out = torch.empty((B, H, VD), device="cuda")
+            torch.cuda.synchronize()
             dev._check(dev._L.tq_mla_unabsorb(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.data_ptr()), B, H, VD, C.c_void_p(out.data_ptr()), tb.F32))
             dev.sync()
             assert rel_err(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("H,B", [(16, 3), (128, 16)])
+def test_per_head_products_have_no_bias(dev, kind, H, B):
+    """W_UV's products as f32 results of positive terms: the tensor core truncates when it adds, so an accumulator that stayed there for all
+    of K would be low by its number of steps; a 32-block's two steps lose less than 2^-23 of it each, f32 additions none on average."""
+    import ctypes as C
+
+    import tang_b200 as tb
+    import torch
+
+    rng = np.random.default_rng(kind + H)
+    rows = H * VD
+    sc = rng.uniform(0.5, 1.5, rows if kind == 3 else (rows, C_ // 32)).astype(np.float32)
+    if kind < 2:
+        lo, hi = (rng.integers(9, 16, (rows, C_ // 2), dtype=np.uint8) for _ in range(2))
+        pay, sc = lo | (hi << 4), sc.astype(np.float16).view(np.uint16) if kind == 1 else sc
+    else:
+        pay = rng.integers(1, 128, (rows, C_), dtype=np.int8)
+    w = dev.upload_qarrays(kind, pay, sc, rows, C_)
+    deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double().view(H, VD, C_)
+    x = torch.randn((B, H, C_), device="cuda", generator=torch.Generator(device="cuda").manual_seed(H)).abs().bfloat16()
+    out = torch.empty((B, H, VD), device="cuda")
+    torch.cuda.synchronize()
+    dev._check(dev._L.tq_mla_unabsorb(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.data_ptr()), B, H, VD, C.c_void_p(out.data_ptr()), tb.F32))
+    dev.sync()
+    err = out.double() / torch.einsum("bhc,hrc->bhr", x.double(), deq) - 1
+    # (rms: a result's own rounding 2.5e-8, three additions of tiles)
+    assert abs(err.mean().item()) < 1.3e-7 and err.square().mean().sqrt().item() < 6e-8, (err.mean(), err.square().mean().sqrt())
