@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(kMlaThreads * HT) mla_decode_kernel(const MlaP
 // loads of eight splits in flight (one sequence of 4096, 32 splits: 8.7 -> 3 us behind the attention).  `unit`: the maxima's
 // unit in powers of two.
 constexpr int kMlaMaxSplits = 512;
+constexpr int kMlaMaxSplitTiles = 128;                    // tiles of 32 positions that one tensor-memory accumulator takes
 __global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, const float* part_ml, int n_splits, float unit, __nv_bfloat16* out) {
   __shared__ float w[kMlaMaxSplits + 1];
   pdl_wait();
@@ -501,6 +502,12 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   const int base = 2 * B * (int)((n_heads + 127) / 128), tiles32 = ((int)max_len + 31) / 32;
   int want = ctx->sm_count / base;
   if (want < 1) want = 1;
+  // The tensor core truncates when it adds, about 6e-9 of the sum for each position that an accumulator takes (mma.sync the same; mean
+  // signed error of values of one sign): at most 4096 positions a split, so that 38 sequences of 32768 have 2.2e-5 and not 2.1e-4
+  // (9.7e-5 with the other kernel).  It takes them from 1218 to 681 us, 64 of 32768 from 1225 to 1024, 64 of 8192 from 328 to 361; at
+  // most 2048 would cost 16 of 16384 182 -> 198 us for 1.1e-5 less, against 1.1e-3 of a result's rounding to bf16.
+  const int least = (tiles32 + kMlaMaxSplitTiles - 1) / kMlaMaxSplitTiles;
+  if (want < least) want = least;
   if (want > kMlaMaxSplits) want = kMlaMaxSplits;
   const bool umma = tiles32 / want >= 8 && mla_umma_supported(q_full_bf16_dev, cache_bf16_dev, n_heads, seq_stride, batch, max_len);
   int n_splits, chunk;

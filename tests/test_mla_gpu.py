@@ -311,6 +311,25 @@ def test_attention_core_over_close_sequences(dev, B, n, step):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,n", [(38, 32768), (40, 6000), (16, 16384)])
+def test_attention_core_has_no_bias(dev, B, n):
+    """Values of one sign: the tensor core truncates when it adds, about 6e-9 of the sum for a position, so a split takes 4096 positions at
+    most: 2.6e-5 (all of 32768 in one had 2.1e-4).  The rounding of 512 x 128 results a sequence to bf16, 1.1e-3 each and the heads' not
+    independent, leaves some 3e-6 in the mean."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(B)
+    q = (torch.randn((B, 128, C_ + R_), device="cuda", generator=g) * 0.2).bfloat16()
+    mean = torch.rand((B, 1, C_ + R_), device="cuda", generator=g) + 1
+    cache = torch.empty((B, n, C_ + R_), device="cuda", dtype=torch.bfloat16)
+    for b in range(B):
+        cache[b] = (mean[b] + torch.rand((n, C_ + R_), device="cuda", generator=g)).bfloat16()
+    got, want = attend(dev, q, cache.view(-1, C_ + R_), [b * n for b in range(B)], [n - 17 * b for b in range(B)], n * (C_ + R_), n)
+    bias = (got.double() / want - 1).mean().item()
+    assert abs(bias) < 3.5e-5, bias
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", [0, 1, 2, 3])
 @pytest.mark.parametrize("H,B", [(16, 1), (80, 8), (75, 9), (128, 16), (33, 33), (128, 64)])
 def test_per_head_products(dev, kind, H, B):
