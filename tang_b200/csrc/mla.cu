@@ -504,8 +504,8 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   if (want < 1) want = 1;
   // The tensor core truncates when it adds, about 6e-9 of the sum for each position that an accumulator takes (mma.sync the same; mean
   // signed error of values of one sign): at most 4096 positions a split, so that 38 sequences of 32768 have 2.2e-5 and not 2.1e-4
-  // (9.7e-5 with the other kernel).  It takes them from 1218 to 681 us, 64 of 32768 from 1225 to 1024, 64 of 8192 from 328 to 361; at
-  // most 2048 would cost 16 of 16384 182 -> 198 us for 1.1e-5 less, against 1.1e-3 of a result's rounding to bf16.
+  // (9.7e-5 with the other kernel).  It takes them from 1218 to 648 us, 64 of 32768 from 1225 to 986, 64 of 8192 from 328 to 341; at
+  // most 2048 would cost 16 of 16384 a tenth for 1.1e-5 less, against 1.1e-3 of a result's rounding to bf16.
   const int least = (tiles32 + kMlaMaxSplitTiles - 1) / kMlaMaxSplitTiles;
   if (want < least) want = least;
   if (want > kMlaMaxSplits) want = kMlaMaxSplits;

@@ -5,15 +5,16 @@
 // one half of the latent columns (256) and forms the scores for itself; the two CTAs of a pair are neighbours in the grid and
 // read the same cache rows, the second time from L2.  Per tile of 32 positions:
 //   warp 0      TMA: nine groups of 32 rows x 64 columns (128-byte swizzle) in one copy into one of three stages; the queries once (the first 256
-//               columns go to tensor memory, which leaves room for the third stage: with two the copies' latency was the bound);
+//               columns go to tensor memory, which leaves room for the third stage: with two the copies' latency was the bound).
+//               The rows of a last tile that is not full come by cp.async, zeros behind them: nothing behind a sequence's end is read;
 //   warp 1      issues S = Q K^T (36 MMAs of 128 x 32 x 16), then, a tile behind, O += P V (V are the same boxes, read
 //               N-major): the probabilities come from tensor memory as two bf16 terms (hi + lo, 16 significant bits, as in
 //               the mma.sync kernel), one MMA of 128 x 256 x 16 each;
 //   warps 4..7  a thread owns one head: it reads the head's 32 scores, takes the maximum, forms P and the row sum without any
 //               exchange.  O is rescaled only when a maximum has grown by more than 2^8 (the reference of the exponentials is
 //               any number near the maximum), which is rare after the first tiles;
-// Measured, 128 heads: 16 sequences of 8.7k to 16.4k positions, the attention alone 437 us with the mma.sync kernel -> 177 us
-// (tiles of 32 positions, 1.4 us each; two stages instead of three: 296 us).  What bounds it now is the chain copy -> scores -> softmax -> products of a tile with
+// Measured, 128 heads: 16 sequences of 8.7k to 16.4k positions, the attention and its merge 454 us with the mma.sync kernel -> 171 us
+// (tiles of 32 positions, 1.3 us each; with two stages instead of three the attention took 296 us where it took 177).  What bounds it now is the chain copy -> scores -> softmax -> products of a tile with
 // three tiles in flight (shared memory is full), not the 220 TFLOP/s that it reaches.
 // Splits over the positions are merged by mla_combine_kernel.  Every wait is bounded.
 #include <cfloat>
@@ -37,6 +38,8 @@ constexpr float kMuGrow = 8.f;                                       // log2 of 
 
 struct MlaUmmaParams {
   const __nv_bfloat16* q;         // [B][H][576]
+  const __nv_bfloat16* cache;     // sequence b from b * seq_stride on
+  size_t seq_stride;
   const int* lens;
   int n_heads, n_splits, chunk;   // chunk: positions per split, a multiple of the tile
   float scale;                    // softmax scale times log2(e)
@@ -120,13 +123,14 @@ mla_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant
   };
 
   if (warp == 0) {
+    const int whole = tail < kMuTile ? n - 1 : n;
     if (lane == 0 && n) {
       mbar_arrive_expect_tx(q_full, (kMuBoxes - kMuQTmem) * kMuQBox);
       for (int i = kMuQTmem; i < kMuBoxes; ++i)
         tma_load_2d(q_s + (size_t)(i - kMuQTmem) * kMuQBox, &q_map, 64 * i, b * p.n_heads + 128 * hg, q_full);
       int s = 0;
       uint32_t ph = 0;
-      for (int i = 0; i < n && !*failed; ++i) {
+      for (int i = 0; i < whole && !*failed; ++i) {
         if (!mbar_wait_spin(&k_empty[s], ph ^ 1u)) { give_up(DERR_EMPTY_WAIT); break; }
         mbar_arrive_expect_tx(&k_full[s], kMuStage);
         mu_load_4d(k_s + (size_t)s * kMuStage, &k_map, 0, k_begin + i * kMuTile, 0, b, &k_full[s]);   // all nine groups of 64 columns
@@ -134,6 +138,29 @@ mla_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant
           s = 0;
           ph ^= 1u;
         }
+      }
+    }
+    __syncwarp();
+    if (whole < n) {
+      // a last tile of `tail` rows: what the cache holds behind them may not be memory, and would not stay out of the products
+      // (0 x NaN is NaN)
+      const int s = whole % kMuStages;
+      const bool ok = __all_sync(0xffffffffu, !*failed && mbar_wait_spin(&k_empty[s], ((whole / kMuStages) & 1) ^ 1u));
+      if (ok) {
+        const __nv_bfloat16* src = p.cache + (size_t)b * p.seq_stride + (size_t)(k_begin + whole * kMuTile) * kMuRow;
+        const uint32_t dst = smem_u32(k_s + (size_t)s * kMuStage);
+#pragma unroll 4
+        for (int j = lane; j < kMuTile * kMuBoxes * 8; j += 32) {                    // pieces of 16 bytes
+          const int r = j / (kMuBoxes * 8), c = j - r * (kMuBoxes * 8);
+          const uint32_t at = dst + (uint32_t)((c >> 3) * kMuKBox + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src + (r < tail ? r * kMuRow + 8 * c : 0)), "r"(r < tail ? 16u : 0u) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&k_full[s]);
+      } else {
+        give_up(DERR_EMPTY_WAIT);
       }
     }
     __syncwarp();
@@ -150,15 +177,6 @@ mla_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant
         const int s = i & 1;
         ok = mbar_wait_spin(&k_full[ks], kph) && mbar_wait_spin(&s_empty[s], ((i >> 1) & 1) ^ 1u);
         if (!ok) break;
-        if (i == n - 1 && tail < kMuTile) {
-          // whatever the cache holds behind the sequence's end stays out of the products (0 x NaN is NaN)
-          uint8_t* st = k_s + (size_t)ks * kMuStage;
-          const int pieces = (kMuTile - tail) * 8;                              // of 16 bytes, in each box
-          for (int j = lane; j < kMuBoxes * pieces; j += 32)
-            *reinterpret_cast<uint4*>(st + (size_t)(j / pieces) * kMuKBox + tail * 128 + (j % pieces) * 16) = make_uint4(0u, 0u, 0u, 0u);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-        }
         tc_fence_after();
         if (leader) {
           const uint32_t d = tmem + (uint32_t)(kMuColS + s * kMuTile);
@@ -345,6 +363,8 @@ int launch_mla_umma(tq_ctx* ctx, const void* q, const void* cache, const int* le
                     float scale, int n_splits, int chunk, void* out, float* part_o, float* part_ml) {
   MlaUmmaParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
+  p.cache = static_cast<const __nv_bfloat16*>(cache);
+  p.seq_stride = seq_stride;
   p.lens = lens;
   p.n_heads = (int)n_heads;
   p.n_splits = n_splits;

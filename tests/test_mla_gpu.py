@@ -311,6 +311,20 @@ def test_attention_core_over_close_sequences(dev, B, n, step):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,short", [(1, 19969), (3, 9017), (40, 224), (40, 1)])
+def test_attention_core_reads_no_row_behind_the_end(dev, B, short):
+    """max_len and the stride leave room for more rows than the last sequence has, and its memory ends with it."""
+    import torch
+
+    n = 20001 if B == 1 else 9601 if B == 3 else 320
+    g = torch.Generator(device="cuda").manual_seed(short)
+    q = torch.randn((B, 128, C_ + R_), device="cuda", generator=g).bfloat16()
+    cache = torch.randn(((B - 1) * n + short, C_ + R_), device="cuda", generator=g).bfloat16()
+    got, want = attend(dev, q, cache, [b * n for b in range(B)], [n - b for b in range(B - 1)] + [short], n * (C_ + R_), n)
+    assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("B,n", [(38, 32768), (40, 6000), (16, 16384)])
 def test_attention_core_has_no_bias(dev, B, n):
     """Values of one sign: the tensor core truncates when it adds, about 6e-9 of the sum for a position, so a split takes 4096 positions at
