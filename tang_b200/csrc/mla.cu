@@ -309,7 +309,14 @@ __global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, c
     }
   }
   const float L = w[kMlaMaxSplits];
-  *reinterpret_cast<__nv_bfloat162*>(out + bh * kC + 2 * threadIdx.x) = __floats2bfloat162_rn(L > 0.f ? o.x / L : 0.f, L > 0.f ? o.y / L : 0.f);
+  const __nv_bfloat162 r = __floats2bfloat162_rn(L > 0.f ? o.x / L : 0.f, L > 0.f ? o.y / L : 0.f);
+  __nv_bfloat16* dst = out + bh * kC + 2 * threadIdx.x;
+  if (((uintptr_t)out & 3) == 0) {
+    *reinterpret_cast<__nv_bfloat162*>(dst) = r;
+  } else {                            // (results may begin at any bf16)
+    dst[0] = r.x;
+    dst[1] = r.y;
+  }
 }
 
 __global__ void mla_place_rope_kernel(const __nv_bfloat16* q_rope, __nv_bfloat16* q_full, size_t n_bh) {

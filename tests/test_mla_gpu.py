@@ -273,15 +273,15 @@ def test_attention_core(dev, H, B, lens, sharp):
         assert rel_err(out[b].double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, (b, n)
 
 
-def attend(dev, q, cache, starts, lens, stride, max_len):
-    """tq_mla_decode on torch tensors, checked against 64 bits; `starts`: rows of `cache` at which the sequences begin.  Returns the
-    result and what it is in 64 bits."""
+def attend(dev, q, cache, starts, lens, stride, max_len, shift=0):
+    """tq_mla_decode on torch tensors; `starts`: rows of `cache` at which the sequences begin; the result begins `shift` elements into
+    its memory.  Returns the result and what it is in 64 bits."""
     import ctypes as C
 
     import torch
 
     B, H = q.shape[:2]
-    out = torch.full((B, H, C_), float("nan"), device="cuda").bfloat16()
+    out = torch.full((B * H * C_ + shift,), float("nan"), device="cuda").bfloat16()[shift:].view(B, H, C_)
     lb = torch.tensor(lens, dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
     scale = 1.0 / np.sqrt(NOPE + R_)
@@ -322,6 +322,20 @@ def test_attention_core_reads_no_row_behind_the_end(dev, B, short):
     cache = torch.randn(((B - 1) * n + short, C_ + R_), device="cuda", generator=g).bfloat16()
     got, want = attend(dev, q, cache, [b * n for b in range(B)], [n - b for b in range(B - 1)] + [short], n * (C_ + R_), n)
     assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,B,n", [(16, 2, 500), (128, 3, 9600)])
+def test_merged_results_begin_anywhere(dev, H, B, n):
+    """The merge of the splits of either kernel stores to a result at an odd multiple of two bytes."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    q = torch.randn((B, H, C_ + R_), device="cuda", generator=g).bfloat16()
+    cache = torch.randn((B * n, C_ + R_), device="cuda", generator=g).bfloat16()
+    for shift in (0, 1, 2):
+        got, want = attend(dev, q, cache, [b * n for b in range(B)], [n] * B, n * (C_ + R_), n, shift)
+        assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, shift
 
 
 @pytest.mark.gpu
