@@ -619,10 +619,12 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   }
   for (size_t i = 0; i < m->sh_gate_up.size() && Ts > 0; ++i) {
     // (the same epilogue where the projection fills the GPU without splitting K: below, the split form and the separate kernel)
-    if (Ts >= 1024 && m->sh_gate_up[i]->kind != TQ_I8_ROW && umma_supported(m->sh_gate_up[i], Ts) && d % 8 == 0) {
-      TQ_STEP(launch_qgemm_umma(ctx, m->sh_gate_up[i], h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
+    const tq_qweight* gate_up = m->sh_gate_up[i];
+    const bool sized = gate_up->rows == 2 * f && gate_up->cols == d;      // (any other size is for tq_qlinear to refuse)
+    if (Ts >= 1024 && sized && gate_up->kind != TQ_I8_ROW && umma_supported(gate_up, Ts)) {
+      TQ_STEP(launch_qgemm_umma(ctx, gate_up, h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
     } else {
-      TQ_STEP(tq_qlinear(ctx, m->sh_gate_up[i], h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
+      TQ_STEP(tq_qlinear(ctx, gate_up, h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
       TQ_STEP(tq_swiglu(ctx, shgu, shgu + f, TQ_F32, 2 * f, Ts, f, shact, TQ_BF16));
     }
     TQ_STEP(tq_qlinear(ctx, m->sh_down[i], shact, TQ_BF16, f, Ts, sh + i * Ts * d, TQ_F32, d, nullptr));

@@ -175,3 +175,23 @@ def test_fused_gate_up_equals_the_separate_kernel(dev, renorm):
     worst, share = rel_err_profile(whole, parts)
     assert worst < 1e-2 and share < 5e-3, (worst, share)
     layer.destroy()
+
+
+@pytest.mark.parametrize("rows,cols", [(768 + 128, 256), (768, 384)])
+@pytest.mark.parametrize("T", [40, 1061])
+def test_shared_experts_of_another_size_are_refused(dev, rows, cols, T):
+    """A shared gate/up projection with more rows or columns than the layer's: an error at every token count, whichever kernel would
+    have run."""
+    import tang_b200 as tb
+    from util import make_weight
+
+    rng = np.random.default_rng(rows + T)
+    moe = HostMoe(rng, 256, 384, 4, 2, 0)
+    up = lambda r, c: dev.upload_qarrays(1, *make_weight(rng, 1, r, c)[::-1], r, c)
+    layer = tb.MoeLayer(dev, tb.MoeConfig(256, 384, 4, 2, 1, 0, 0, 1), dev.upload(moe.wg_bits, tb.BF16), up(4 * 768, 256), up(4 * 256, 384), [up(rows, cols)],
+                        [up(256, 384)])
+    x = dev.upload(bf16_round(rng.standard_normal((T, 256)).astype(np.float32))[0], tb.BF16)
+    with pytest.raises(tb.TangqError):
+        layer.forward(x, T)
+    dev.sync()
+    layer.destroy()
