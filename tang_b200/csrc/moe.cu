@@ -36,6 +36,8 @@ int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, co
                               int expected_rows, void* y, int y_dtype, size_t ldy, int terms = 2, int swiglu = 0);
 struct UmmaGroups;
 bool umma_supported(const tq_qweight* w, size_t m);
+bool umma_fills_gpu(const tq_ctx* ctx, const tq_qweight* w, size_t m);
+int umma_min_m(int y_dtype);
 int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size_t ldx, size_t m, void* y, int y_dtype,
                       size_t ldy, int terms, const UmmaGroups* grp, int swiglu);
 bool umma_grouped_supported(const tq_qweight* w, int n_groups);
@@ -618,10 +620,13 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_down, nl, act, f, cap, cnt, offs, (int)T, 0, 0, yo, TQ_F32, d, active, max_active, n));
   }
   for (size_t i = 0; i < m->sh_gate_up.size() && Ts > 0; ++i) {
-    // (the same epilogue where the projection fills the GPU without splitting K: below, the split form and the separate kernel)
+    // The same epilogue where K would not be split anyway (d 2048: f 1408 at 641 tokens 37.5 -> 33.1 us a shared expert, at 1000 60.1 ->
+    // 52.6; f 4096 at 512 76.1 -> 66.6; 4096 x 14336 at 256 207 -> 181), and for many tokens of a narrow expert, where the f32
+    // partials cost more than the idle SMs (1061 tokens, f 384 31.0 -> 28.4; 2048 45.5 -> 40.7; f 128 38.2 -> 36.0).
     const tq_qweight* gate_up = m->sh_gate_up[i];
     const bool sized = gate_up->rows == 2 * f && gate_up->cols == d;      // (any other size is for tq_qlinear to refuse)
-    if (Ts >= 1024 && sized && gate_up->kind != TQ_I8_ROW && umma_supported(gate_up, Ts)) {
+    const bool many = Ts >= 1024 || (Ts >= (size_t)umma_min_m(TQ_F32) && umma_fills_gpu(ctx, gate_up, Ts));
+    if (sized && many && gate_up->kind != TQ_I8_ROW && umma_supported(gate_up, Ts)) {
       TQ_STEP(launch_qgemm_umma(ctx, gate_up, h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
     } else {
       TQ_STEP(tq_qlinear(ctx, gate_up, h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));

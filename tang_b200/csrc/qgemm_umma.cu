@@ -498,6 +498,15 @@ bool umma_supported(const tq_qweight* w, size_t m) {
          w->cols % kTileK == 0 && m >= 1;
 }
 
+// Fewer output tiles than this leave SMs idle, and K is split.
+static bool umma_few_tiles(const tq_ctx* ctx, long long ctas) { return ctas < (ctx->sm_count * 3) / 4; }
+constexpr int kUmmaTwoTermTokens = 128;   // token tile of two-term products: what tensor memory leaves beside the weights
+
+// Whether two-term products of m rows run without a split of K.
+bool umma_fills_gpu(const tq_ctx* ctx, const tq_qweight* w, size_t m) {
+  return !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)((m + kUmmaTwoTermTokens - 1) / kUmmaTwoTermTokens));
+}
+
 // y[m, rows] = x[m, cols] . W^T through the tcgen05 kernel.  x: bf16, 16-byte aligned rows.
 // With `grp`: `grp->n_groups` weight matrices stacked by rows (experts); group e multiplies rows
 // offsets[e] .. +counts[e] of x (device arrays) and m is the total row count of x / y.
@@ -523,7 +532,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   // more of them, i.e. more conversions of the same weights (2048 rows: 9 tiles of 228 against 11 of 192 measured
   // the same; 512 rows, three tiles either way: 95 -> 77 us).
   const size_t m_basis = grp ? (size_t)grp->expected_rows : m;
-  const int ts_cap = terms == 2 ? 128 : 192;
+  const int ts_cap = terms == 2 ? kUmmaTwoTermTokens : 192;
   // Many rows, one term: a CTA takes TWO token tiles (each MMA issuer multiplies every stage with its own tile's
   // activations), so the weights are converted once per 2 x <= 192 tokens; the accumulators are 2 x 192 columns, the
   // weights 128.  Only where that still gives about a wave of CTAs (no K split in this form).
@@ -536,7 +545,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
     if (cap >= 64) {
       n_pairs = (m + 2 * (size_t)cap - 1) / (2 * (size_t)cap);
       dual_ntok = (int)(((m + 2 * n_pairs - 1) / (2 * n_pairs) + 15) / 16 * 16);
-      dual = (long long)(w->rows / kUmmaRows) * (long long)n_pairs >= (ctx->sm_count * 3) / 4;
+      dual = !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)n_pairs);
     }
   }
   const int ts = (dual || terms == 2 || (m_basis + ts_cap - 1) / ts_cap <= (m_basis + ntok_max - 1) / ntok_max) ? 1 : 0;
@@ -555,7 +564,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   // Few output tiles (narrow layers, small batches) leave most SMs idle: split K over gridDim.z.
   const int base_ctas = (int)(w->rows / kUmmaRows) * (int)n_tok_tiles;
   int splits = 1;
-  if (!grp && swiglu != 2 && base_ctas < (ctx->sm_count * 3) / 4) {
+  if (!grp && swiglu != 2 && umma_few_tiles(ctx, base_ctas)) {
     splits = ctx->sm_count / base_ctas;
     if (splits > w->n_kc / 4) splits = w->n_kc / 4;      // at least eight 64-k steps per CTA
     if (splits > 16) splits = 16;

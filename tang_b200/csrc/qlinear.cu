@@ -712,7 +712,7 @@ __global__ void swiglu_interleaved_kernel(const float* gu, size_t rows, size_t n
 // Activation rows from which the tcgen05 kernel takes over from the mma.sync kernel.
 // Rows from which the tcgen05 kernel takes over from the mma.sync kernel (Llama-3-8B decode step, 32 layers, f32
 // outputs: 4.87 against 4.98 ms at 16 rows, 5.63 against 5.30 ms at 20, 6.10 against 5.50 ms at 24).
-static int umma_min_m(int y_dtype) {
+int umma_min_m(int y_dtype) {
   (void)y_dtype;
   return 17;
 }

@@ -195,3 +195,37 @@ def test_shared_experts_of_another_size_are_refused(dev, rows, cols, T):
         layer.forward(x, T)
     dev.sync()
     layer.destroy()
+
+
+@pytest.mark.parametrize("d,f,T", [(256, 128, 1023), (256, 128, 1024), (512, 2048, 384), (512, 2048, 385), (256, 1408, 640), (256, 1408, 641), (256, 14336, 16), (256, 14336, 17)])
+def test_shared_expert_on_both_sides_of_its_rule(dev, d, f, T):
+    """Narrow and wide shared experts around the token counts where gate and up begin to meet in the projection's epilogue, against 64
+    bits with the one rounding that the layer has, of the gated product to bf16.  A product within an f32 sum's error of a rounding tie
+    (one in some thousand) may round the other way, 2^-8 of itself: about 1e-4 of the result's norm."""
+    import tang_b200 as tb
+    import torch
+
+    rng = np.random.default_rng(f + T)
+    moe = HostMoe(rng, d, f, 4, 2, 1)
+    layer = moe.to_device(dev)
+    bits, x = bf16_round(rng.standard_normal((T, d)).astype(np.float32))
+    got = layer.forward(dev.upload(bits, tb.BF16), T).to_vec().reshape(T, d)
+    layer.destroy()
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda().double()
+
+    def weight(w):
+        pay, sc = t(np.stack((w[1] & 15, w[1] >> 4), 2).reshape(w[2], -1).astype(np.int8) - 8), t(w[0].view(np.float16).astype(np.float32))
+        return (pay.view(w[2], -1, 32) * sc[:, :, None]).view(w[2], -1)[:, :w[3]]
+
+    def expert(e, h):
+        g, u = h @ weight(e["gate"]).T, h @ weight(e["up"]).T
+        return (g * torch.sigmoid(g) * u).bfloat16().double() @ weight(e["down"]).T
+
+    h = t(x)
+    top, idx = (h @ t(moe.wg).T).softmax(1).topk(2, 1)
+    want = expert(moe.experts[4], h)
+    for e in range(4):
+        rows, c = (idx == e).nonzero(as_tuple=True)
+        want[rows] += top[rows, c][:, None] * expert(moe.experts[e], h[rows])
+    d_ = torch.from_numpy(got).cuda().double() - want
+    assert (d_.norm() / want.norm()).item() < 5e-4, (d_.norm() / want.norm()).item()
