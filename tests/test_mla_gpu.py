@@ -238,8 +238,8 @@ def test_mla_layer_matches_oracle(dev, orc, d, H, q_lora, B, lens):
     full.destroy()
 
 
-# The attention core on the tensor cores (csrc/mla_umma.cu): heads that fill the tile and that do not, one split and several,
-# splits without positions, lengths around the 32-position tiles, flat and sharply peaked scores; what lies behind a sequence's
+# The attention core on the tensor cores (csrc/mla_umma.cu; 80 heads of one sequence and 16 heads: the mma.sync kernel): heads that fill the
+# tile and that do not, one split and several, splits without positions, lengths around the 32-position tiles, flat and sharply peaked scores; what lies behind a sequence's
 # end in the cache is NaN.  The queries are given, so the result may differ by its own rounding to bf16 (at most 2^-8 = 3.9e-3 of the
 # value) and f32 sums only.
 @pytest.mark.gpu
@@ -322,6 +322,69 @@ def test_attention_core_reads_no_row_behind_the_end(dev, B, short):
     cache = torch.randn(((B - 1) * n + short, C_ + R_), device="cuda", generator=g).bfloat16()
     got, want = attend(dev, q, cache, [b * n for b in range(B)], [n - b for b in range(B - 1)] + [short], n * (C_ + R_), n)
     assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3
+
+
+def tcgen05_length(B, H, tiles=8):
+    """The shortest max_len from which tq_mla_decode takes the tcgen05 kernel: `tiles` (eight at least) tiles of 32 positions for every CTA
+    of one wave (csrc/mla.cu)."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return 32 * tiles * max(1, sms // (2 * B * ((H + 127) // 128)))
+
+
+# Peaked scores that grow along the sequence, so that the reference of the exponentials moves, and the outputs are rescaled beside a
+# pending product, in late tiles too; heads that leave rows of the last 128 empty; sequences with room between them.
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,B,sharp", [(80, 4, 30.0), (64, 40, 30.0), (144, 3, 6.0), (128, 1, 30.0)])
+def test_attention_core_with_growing_scores(dev, H, B, sharp):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    n = tcgen05_length(B, H, 11) + 5
+    ramp = torch.linspace(0, 1, n, device="cuda")[:, None]
+    u = torch.randn((C_ + R_,), device="cuda", generator=g)
+    q = ((torch.randn((B, H, C_ + R_), device="cuda", generator=g) + u) * sharp / 24).bfloat16()
+    cache = (torch.randn((B, n, C_ + R_), device="cuda", generator=g) * 0.3 + ramp * u).bfloat16()
+    rows = torch.full((B, n + 37, C_ + R_), float("nan"), device="cuda", dtype=torch.bfloat16)
+    rows[:, :n] = cache
+    lens = [n - 33 * b for b in range(B)]
+    got, want = attend(dev, q, rows.view(-1, C_ + R_), [b * (n + 37) for b in range(B)], lens, (n + 37) * (C_ + R_), n)
+    assert rel_err(got.double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,B", [(128, 40), (64, 6)])
+def test_attention_core_replayed_while_sequences_grow(dev, H, B):
+    """One recorded call, the lengths raised between the replays: through full tiles, past them, and into splits that had no positions."""
+    import ctypes as C
+
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(H)
+    n = tcgen05_length(B, H, 9)
+    q = torch.randn((B, H, C_ + R_), device="cuda", generator=g).bfloat16()
+    cache = torch.randn((B, n, C_ + R_), device="cuda", generator=g).bfloat16()
+    out = torch.zeros((B, H, C_), device="cuda", dtype=torch.bfloat16)
+    lens = torch.zeros((B,), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    call = lambda: dev._check(dev._L.tq_mla_decode(dev._ctx, C.c_void_p(q.data_ptr()), C.c_void_p(cache.data_ptr()), C.c_void_p(lens.data_ptr()), B, H, C_, R_,
+                                                   n * (C_ + R_), n, 1.0 / np.sqrt(NOPE + R_), C.c_void_p(out.data_ptr())))
+    call()                     # (sizes the workspace)
+    dev.sync()
+    dev.begin_capture()
+    call()
+    graph = dev.end_capture()
+    for base in (1, 31, 32, 33, n // 2, n - B):
+        lens.copy_(torch.arange(B, dtype=torch.int32, device="cuda") + base)
+        torch.cuda.synchronize()
+        graph.launch()
+        dev.sync()
+        for b in range(0, B, 5):
+            kv = cache[b, :base + b].double()
+            want = (q[b].double() @ kv.T / np.sqrt(NOPE + R_)).softmax(-1) @ kv[:, :C_]
+            assert rel_err(out[b].double().cpu().numpy(), want.cpu().numpy(), floor_frac=1.0) < 4.1e-3, (base, b)
+    graph.free()
 
 
 @pytest.mark.gpu
