@@ -24,12 +24,13 @@ bool launch_qgemm_wr(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size_
   // against 23.2 here at 24 rows and 28.0 at 32 (14336 x 4096).
   if (m < 9 || m > (size_t)kWrRows || w->cols != (size_t)w->n_kc * kTileK || ldx % 8 != 0 || ((uintptr_t)x_bf16 & 15) != 0 || w->n_rb > kWrCounters)
     return false;
-  // Little to stream: the general kernel, which parks nothing and counts nothing (2048 x 2048 Q4 4.0 us against 6.7,
-  // 1536 x 7168 int8 8.8 against 12.2; 4096 x 4096 Q4 11.4 against 10.7, int8 12.4 against 11.1).
+  // Little to stream: the general kernel, which parks nothing and counts nothing (12 rows: 2048 x 2048 Q4 4.0 us against 7.4, 1536 x 7168
+  // int8 8.7 against 13.2; at 42 tiles per SM, 3072 x 4096, 10.9 against 10.1 and 11.7 against 10.7, but at 9 rows 6.3 against 9.9).
+  // Its launcher has a rule for larger ones too (qlinear.cu).
   if ((long long)w->n_rb * w->n_kc < 50LL * ctx->sm_count) return false;
   QWrParams p;
-  // The widest slabs that fit: every slab boundary is one more piece to park per row block (14336 x 4096: 16.0 us with one slab,
-  // 22 with four; 7168 x 16384 int8: 37 us with four, 71 with sixteen).
+  // The widest slabs that fit: every slab boundary is one more piece to park per row block (12 rows, Q4 14336 x 4096: 16.6 us with
+  // the two slabs that fit, 20.3 with four, 27.4 with eight; int8 7168 x 16384: 34.2 with six, 41.2 with twelve, 67.7 with 24).
   const size_t ring = (size_t)kWrWarps * wr_depth(w->kind) * qk_tile_bytes(w->kind);
   const int skc_max = (int)(((227 * 1024 - ring) / kWrRows - 64) / (2 * kTileK));
   p.n_slabs = (w->n_kc + skc_max - 1) / skc_max;

@@ -192,6 +192,20 @@ static QgConfig choose_config(const tq_ctx* ctx, const tq_qweight* w, int mx, in
   return c;
 }
 
+// Whether the general kernel is the faster one at nine to sixteen rows (the other: qgemm_wr.cuh): where its CTAs, at most two of them
+// on an SM, make one wave of few turns of their rings, it has no pieces to park and nothing to set up.  12 rows, Q4: 2048 x 8192
+// 9.1 us against 12.7, 2048 x 12288 12.4 against 14.6, 1536 x 16384 (16 turns) 15.4 against 14.2; two row blocks a CTA, 9472 x 3072
+// 9.6 against 10.6, 9472 x 4096 (8 turns) 11.7 against 12.3, 14208 x 4096 (two waves) 20.0 against 16.3; 9 rows of Q4 with f16 scales
+// (two CTAs on an SM) 4096 x 4096 6.8 against 10.3, 4096 x 14336 (14 turns) 17.1 against 16.9.  Two waves win with four turns only
+// (9 rows, 8192 x 2048 8.7 against 10.3, x 3072 10.9 against 10.4).
+static bool general_kernel_is_faster(const tq_ctx* ctx, const tq_qweight* w, int mx) {
+  const QgConfig c = choose_config(ctx, w, mx, w->n_rb, 1);
+  const size_t smem = qg_smem_bytes(w->kind, c.nt, c.wr, c.wk, c.tpw, c.stages, mx);
+  const int per_sm = 233472 / (smem + 1024) >= 2 ? 2 : 1, ctas = (w->n_rb + c.wr - 1) / c.wr;
+  const int waves = (ctas + per_sm * ctx->sm_count - 1) / (per_sm * ctx->sm_count), turns = (w->n_kc + c.wk * c.tpw - 1) / (c.wk * c.tpw);
+  return waves == 1 ? turns <= (c.wr == 1 ? 12 : 8) : waves == 2 && turns <= 2;
+}
+
 struct QgGroup {
   int n_groups = 1;
   const int* counts = nullptr;    // device: rows routed to each group (expert batches)
@@ -982,7 +996,7 @@ int tq_qlinear(tq_ctx* ctx, const tq_qweight* w, const void* x_dev, int x_dtype,
     const size_t rows_staged = (m < chunk ? m : chunk) * combine;
     if (int st = ensure_xprep(ctx, rows_staged * kx * 2)) return st;
   }
-  if (direct) {
+  if (direct && m > 8 && m <= 16 && !general_kernel_is_faster(ctx, w, (int)m)) {
     int st = TQ_OK;
     if (launch_qgemm_wr(ctx, w, x_dev, ldx, m, y_dev, y_dtype, ldy, residual_dev, false, &st)) return st;
   }

@@ -565,3 +565,25 @@ def test_nine_to_sixteen_rows_have_no_bias(dev, kind, rows, cols):
         xbits[1, cols // 2 + 1] = 0x7F80
         y = dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.F32).to_vec().reshape(m, rows)
         assert (y[1] == np.inf).all() and np.isfinite(np.delete(y, 1, 0)).all()
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(2048, 8192), (2368, 6656), (2384, 6656), (1536, 12288), (1536, 12416), (4736, 4096), (4752, 4096), (9472, 2048), (9488, 2048),
+                                       (8192, 2048), (9472, 4096), (9472, 4224)])
+def test_nine_to_sixteen_rows_on_both_sides_of_the_waves(dev, kind, rows, cols):
+    """Sizes around which the general kernel stops fitting one wave, or takes one turn of its ring too many, and the kernel of a ring per
+    warp takes over: the same products, f32 sums, and bf16 results that are those rounded."""
+    import tang_b200 as tb
+    import torch
+
+    rng = np.random.default_rng(rows + cols + kind)
+    sc, pay = make_weight(rng, kind, rows, cols)
+    w = _upload(dev, kind, sc, pay, rows, cols)
+    deq = torch.from_numpy(dev.dequantize(w)[0]).cuda().double()
+    for m in (9, 12, 16):
+        xbits, xf = bf16_round(rng.standard_normal((m, cols)).astype(np.float32))
+        want = (torch.from_numpy(xf).cuda().double() @ deq.T).cpu().numpy()
+        xb = dev.upload(xbits, tb.BF16)
+        y = dev.qlinear(xb, w, m, tb.F32).to_vec().reshape(m, rows)
+        assert np.linalg.norm(y - want) / np.linalg.norm(want) < 2.5e-7, m       # (random signs: the general kernel has up to 1.5e-7)
+        assert np.array_equal(dev.qlinear(xb, w, m, tb.BF16).to_vec().reshape(m, rows), bf16_round(y)[0])
