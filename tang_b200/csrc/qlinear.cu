@@ -1174,7 +1174,9 @@ static bool matvec_host_pinned(tq_ctx* ctx, const tq_qweight* w, const void* xa,
 static bool matvec_host_bounce(tq_ctx* ctx, const tq_qweight* w, const void* x_host, void* y_host, int dtype, size_t m, int* status) {
   const size_t kx = (size_t)w->n_kc * kTileK, ny = m * w->rows;
   const int dt = dtype == TQ_F64 ? TQ_F32 : dtype;
-  if (ny * dtype_size(dt) > kBounceYBytes) return false;     // (m * kx elements fit: hostx_fits)
+  // (m * kx elements fit: hostx_fits.)  Widening more results than this on the host takes longer than the driver's copy of the f64
+  // values: 12288 results 52 us against 55 to 62, 32768 83 against 67 to 77, 131072 254 against 147; f32 gains up to the buffer's end.
+  if (ny * dtype_size(dt) > kBounceYBytes || (dtype == TQ_F64 && ny > 16384)) return false;
   if (!ctx->bounce) {
     void* p = nullptr;
     if (cudaHostAlloc(&p, kHostXSlotBytes + kBounceYBytes, cudaHostAllocMapped) != cudaSuccess ||

@@ -358,8 +358,8 @@ def test_host_matvec_reads_x_in_stream_order(dev, orc):
 
 
 # Pageable vectors through the context's pinned buffers: rows whose columns are no whole 128-k chunk, two f64 and f32 rows, results on
-# both sides of the buffers' 1 MB (the larger ones are copied by the driver), beside replays of a graph that stages its own vectors.
-@pytest.mark.parametrize("rows,cols,m", [(96, 100, 2), (33, 1056, 1), (262144, 64, 1), (262160, 64, 1), (131072, 32, 2), (131088, 32, 2)])
+# both sides of the buffers' 1 MB and of the 16384 f64 results (the larger ones are copied by the driver), beside replays of a graph that stages its own vectors.
+@pytest.mark.parametrize("rows,cols,m", [(96, 100, 2), (33, 1056, 1), (16384, 64, 1), (8200, 64, 2), (262144, 64, 1), (262160, 64, 1), (131072, 32, 2), (131088, 32, 2)])
 def test_pageable_host_matvec(dev, orc, rows, cols, m):
     import torch
     import tang_b200 as tb
