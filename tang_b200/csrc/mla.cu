@@ -504,8 +504,12 @@ int tq_mla_decode(tq_ctx* ctx, const void* q_full_bf16_dev, const void* cache_bf
   TQ_REQUIRE(ctx, max_len > 0, "tq_mla_decode: max_len must bound the sequence lengths");
   const int HT = n_heads % 32 == 0 ? 2 : 1;   // head tiles per CTA
   const int B = (int)batch, HG = (int)(n_heads / (16 * HT));
-  // The tcgen05 kernel where every CTA of about one wave keeps eight tiles of 32 positions; below that its prologue (queries,
-  // tensor memory) costs more than it saves (one sequence of 4096, 128 heads: the layer 80.7 us with the mma.sync kernel, 87.0).
+  // The tcgen05 kernel where every CTA of about one wave keeps eight tiles of 32 positions: below that its prologue (queries, tensor
+  // memory) costs more than it saves.  Attention alone, this kernel against the mma.sync one: 64 heads, four tiles 22.3 us against
+  // 17.2, seven 27.6 against 30.7, eight 27.1 against 30.4; 128 heads, one tile 26.4 against 17.9, four 25.1 against 32.0, eight
+  // 29.7 against 47.7.  Heads (mla_umma_supported): rows of a CTA that are no head cost as much as those that are, so 16 and 32 heads
+  // are slower (16 sequences of 16384 160 us against 93, 165 against 134), 64 (165 against 235) and 80 (167 against 366) faster, and 144,
+  // two CTAs deep, still (324 against 716).  48 heads, one head tile a CTA there, would be faster too (165 against 220).
   const int base = 2 * B * (int)((n_heads + 127) / 128), tiles32 = ((int)max_len + 31) / 32;
   int want = ctx->sm_count / base;
   if (want < 1) want = 1;
