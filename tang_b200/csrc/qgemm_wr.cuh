@@ -3,8 +3,8 @@
 //
 //     y[m, n] = sum_k x[m, k] * q[n, k] * scale[n, k / 32]        (crates/tang-infer/src/quantize.rs:227-289)
 //
-// Bound: instructions and their latencies rather than bytes (14336 x 4096 at 12 rows under ncu: issue slots 49 % busy, ALU 33 %,
-// tensor pipe 20 %, DRAM 19 %).  So what stands around the products is kept short:
+// Bound: instructions and their latencies rather than bytes (14336 x 4096 at 12 rows under ncu: issue slots 48 % busy, ALU 34 %,
+// tensor pipe 20 %, DRAM 18 %).  So what stands around the products is kept short:
 //   * K is cut into slabs of `skc` 128-k chunks (one slab where the activations fit); a CTA belongs to one slab and keeps its
 //     slab of the activation rows in shared memory for its whole life: one read of x per CTA, no activation pipeline;
 //   * the slab's tiles, numbered (row block, chunk), are cut evenly over all WARPS of its CTAs.  A warp walks its contiguous
@@ -15,7 +15,7 @@
 //   * a (row block, slab) piece that does not hold all of K is parked as f32 fragments; the warp whose tiles complete a row
 //     block (a counter of tiles) adds the parked pieces in slab order, then in warp order: the same bits whoever that is.
 //     Nobody waits for anybody.  (Pieces of one CTA meeting in shared memory behind a CTA barrier at the end measured slower:
-//     18.5 against 16.0 us at 14336 x 4096, 24.1 against 18.9 at 4096 x 14336.)
+//     18.5 against 16.0 us at 14336 x 4096, 24.1 against 18.9 at 4096 x 14336, where it now takes 16.6 and 17.2.)
 // Measured, 12 rows, f32 results, against the general kernel: 14336 x 4096 Q4 22.1 -> 16.6 us, 4096 x 14336 27.7 -> 17.2,
 // 6144 x 4096 17.0 -> 11.0, int8 24576 x 1536 32.3 -> 15.4, int8 7168 x 16384 67.9 -> 34.2.  Errors against 64 bits, relative to the
 // result's norm, Q4: 1.11e-7 -> 7.6e-8, 1.46e-7 -> 7.9e-8, 9.3e-8 -> 6.5e-8; int8 6.3e-8 -> 6.2e-8, 14336 x 4096 8.3e-8 -> 6.9e-8.
