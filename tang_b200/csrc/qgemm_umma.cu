@@ -8,18 +8,19 @@
 
 namespace tq {
 
-template <int KIND, int TERMS, bool TS = false, bool DUAL = false>
+template <int KIND, int TERMS, bool DUAL = false>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
-qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p) {
+qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ UmmaParams p) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int TB = (KIND == I8_ROW) ? 2048 : (KIND == Q8_F32) ? 2304 : (KIND == Q4_F16) ? 1152 : 1280;
   constexpr bool kIs8 = KIND == I8_ROW || KIND == Q8_F32;
+  constexpr int kTileLines = TB / 128;   // 128-byte lines of a tile: its weights, then its scales
   static_assert(KIND != I8_ROW || TERMS == 1, "int8 rows carry no scale into the operand: one exact term");
   // DUAL: the CTA covers two token tiles of p.ntok rows with one conversion of the weights: issuer warp 1 multiplies
   // every stage with the first tile's activations, warp 3 with the second tile's, each into one accumulator
-  static_assert(!DUAL || (TS && TERMS == 1), "two token tiles per CTA: single-term weights in tensor memory");
+  static_assert(!DUAL || TERMS == 1, "two token tiles per CTA: single-term weights");
   constexpr int kTokTiles = DUAL ? 2 : 1;
-  constexpr int kMaxStages = 6;
+  constexpr int kMaxStages = kUmmaMaxStages;
   // ---- shared-memory carve-up (operand tiles need 1024-byte alignment for the 128-byte swizzle)
   uint8_t* smem = smem_raw;
   uint64_t* x_full = reinterpret_cast<uint64_t*>(smem);       // [stages] activation box landed
@@ -32,19 +33,16 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t base_u32 = smem_u32(smem_raw);
   uint8_t* tiles_s = smem_raw + kUmmaHeader + ((1024 - ((base_u32 + kUmmaHeader) & 1023)) & 1023);  // 1024-aligned
-  const size_t stage_bytes = umma_stage_bytes(TERMS, p.ntok, TS ? 1 : 0) * kTokTiles;
-  constexpr int kBOff = TS ? 0 : TERMS * kUmmaRows * 128;   // the activation box inside a stage
+  const size_t stage_bytes = umma_stage_bytes(p.ntok) * kTokTiles;
   uint8_t* raw_s = tiles_s + (size_t)p.stages * stage_bytes;   // [raw stages][8 tiles]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = p.stages, RS = p.raw_stages, KT = p.kt;
-  // the eight 16-row blocks of this CTA: neighbours, or (swiglu 2) four gate blocks with their up blocks behind each
-  auto row_block = [&](int i) {
-    return p.swiglu == 2 ? (i & 1) * (p.n_rows / (2 * kTileRows)) + (int)blockIdx.x * 4 + (i >> 1) : (int)blockIdx.x * (kUmmaRows / kTileRows) + i;
-  };
+  // The eight 16-row blocks of this CTA come in two boxes of four: neighbours, or (swiglu 2) gate blocks and their up blocks
+  int rb_first = (int)blockIdx.x * (p.swiglu == 2 ? 4 : 8);
+  const int rb_away = p.swiglu == 2 ? p.n_rows / (2 * kTileRows) : 4;
   int m0 = blockIdx.y * p.ntok * kTokTiles;                    // first token of this CTA
   int m_end = p.m_total;                                       // rows at or beyond this are not this CTA's to store
-  const uint8_t* tile_base = p.tiles;
   const float* row_scales = p.row_scales;   // TQ_I8_ROW: per output row, applied to the accumulator
   if (p.g_counts) {
     // grouped (experts): blockIdx.z picks the group, whose rows are g_offsets[e] .. +g_counts[e] of x and y and
@@ -59,7 +57,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     if (m0 >= cnt) return;
     m_end = p.g_offsets[e] + cnt;
     m0 += p.g_offsets[e];
-    tile_base += (size_t)e * p.g_tile_stride;
+    rb_first += e * (p.n_rows / kTileRows);
     row_scales += (size_t)e * p.n_rows;
   }
   const int kc_begin = p.g_counts ? 0 : blockIdx.z * p.kc_per_split;   // this CTA's slice of K, in 128-k tiles
@@ -80,7 +78,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     *failed = 0;
     mbar_init_fence();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, (uint32_t)p.tmem_cols);
+  if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -100,15 +98,14 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
       const uint64_t pol_w = l2_policy_evict_first();
       int r = 0;
       uint32_t rph = 0;
-      // one ring slot = KT consecutive k-tiles of the CTA's eight row blocks: eight copies of KT tiles each (the
-      // copy engine takes about as long over one tile as over four, so small copies cannot keep up with HBM)
+      // one ring slot = KT consecutive k-tiles of the CTA's eight row blocks, in two boxes of 128-byte lines (tiles behind
+      // the matrix's last read as zeros and are not looked at)
       for (int t0 = 0; t0 < kc_len && !*failed; t0 += KT) {
-        const uint32_t kcs = (uint32_t)min(KT, kc_len - t0);
         if (!mbar_wait_spin(&raw_empty[r], rph ^ 1u)) { give_up(DERR_EMPTY_WAIT); break; }
-        mbar_arrive_expect_tx(&raw_full[r], 8u * kcs * TB);
-        for (int i = 0; i < 8; ++i)
-          bulk_g2s(raw_s + ((size_t)(r * 8 + i) * KT) * TB, tile_base + ((size_t)row_block(i) * p.kc_total + kc_begin + t0) * TB,
-                   kcs * TB, &raw_full[r], pol_w);
+        mbar_arrive_expect_tx(&raw_full[r], 8u * KT * TB);
+        uint8_t* slot = raw_s + (size_t)r * 8 * KT * TB;
+        tma_load_3d(slot, &w_map, 0, (kc_begin + t0) * kTileLines, rb_first, &raw_full[r], pol_w);
+        tma_load_3d(slot + 4 * KT * TB, &w_map, 0, (kc_begin + t0) * kTileLines, rb_first + rb_away, &raw_full[r], pol_w);
         if (++r == RS) {
           r = 0;
           rph ^= 1u;
@@ -123,7 +120,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
       for (int kb = 0; kb < n_kb && !*failed; ++kb) {
         if (!mbar_wait_spin(&empty[s], ph ^ 1u)) { give_up(DERR_EMPTY_WAIT); break; }
         mbar_arrive_expect_tx(&x_full[s], (uint32_t)(p.ntok * kTokTiles) * 128u);
-        tma_load_2d(tiles_s + (size_t)s * stage_bytes + (size_t)kBOff, &x_map,
+        tma_load_2d(tiles_s + (size_t)s * stage_bytes, &x_map,
                     (kc_begin * 2 + kb) * kUmmaK, m0, &x_full[s]);
         if constexpr (DUAL)     // (rows beyond the matrix read as zeros, a box entirely beyond it too)
           tma_load_2d(tiles_s + (size_t)s * stage_bytes + (size_t)p.ntok * 128, &x_map, (kc_begin * 2 + kb) * kUmmaK,
@@ -146,7 +143,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     const bool leader = elect_one();
     const uint32_t idesc = umma_idesc_bf16(p.ntok);
     const uint64_t desc0 = umma_desc_sw128(tiles_s);
-    const uint32_t stage_u = (uint32_t)(stage_bytes >> 4), b_off_u = (uint32_t)(kBOff >> 4);
+    const uint32_t stage_u = (uint32_t)(stage_bytes >> 4);
     bool ok = true;
     const int odd = warp == 3;
     // Each issuer rotates over n_acc / 2 accumulators: the tensor core truncates every f32 addition, an error that
@@ -177,16 +174,11 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
       if (leader) {
 #pragma unroll
         for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
-          const uint64_t bd = ad + b_off_u + tile_off_u + 2 * k16;
-          if constexpr (TS) {
-            // the stage's weights sit in tensor memory: 32 columns (64 k) of the hi term, then 32 of the lo term
-            const uint32_t a_t = tmem_d + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS) + 8 * k16);
-            umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
-            if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
-          } else {
-            umma_f16(acc, ad + 2 * k16, bd, idesc, fresh | (k16 != 0));
-            if (TERMS == 2) umma_f16(acc, ad + (kUmmaRows * 128 >> 4) + 2 * k16, bd, idesc, 1u);
-          }
+          const uint64_t bd = ad + tile_off_u + 2 * k16;
+          // the stage's weights sit in tensor memory: 32 columns (64 k) of the hi term, then 32 of the lo term
+          const uint32_t a_t = tmem_d + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS) + 8 * k16);
+          umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
+          if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
         }
       }
       if (leader) umma_commit(&empty[s_cur]);   // arrives when the MMAs above have finished reading the stage
@@ -207,20 +199,12 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     // stores and fence is long; the groups overlap it).  G is even, so a group always reads the same
     // half (c = g & 1) of its 128-k packed tiles.
     const int group = (warp - kUmmaFirstDqWarp) / kUmmaGroupWarps;
-    const int tid = threadIdx.x - 32 * kUmmaFirstDqWarp - group * 32 * kUmmaGroupWarps;
-    constexpr int kCombos = 512 / (32 * kUmmaGroupWarps);
-    int src_off[kCombos], sc_off[kCombos], dst_off[kCombos][2];
-#pragma unroll
-    for (int i = 0; i < kCombos; ++i) {
-      const int combo = tid + 32 * kUmmaGroupWarps * i;            // (row block, half, lane of the tile layout)
-      const int rbi = combo >> 6, h = (combo >> 5) & 1, L = combo & 31;
-      const int g = L >> 2, t = L & 3;
-      const int row = rbi * 16 + g + 8 * h;
-      src_off[i] = rbi * KT * TB + (kIs8 ? h * 1024 : h * 512) + 16 * L;
-      sc_off[i] = rbi * KT * TB + (kIs8 ? 2048 : 1024) + (KIND == Q4_F16 ? h * 64 + g * 8 : h * 128 + g * 16);
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) dst_off[i][jj] = row * 128 + (((4 * jj + t) ^ (row & 7)) << 4);
-    }
+    // This thread owns output row 32 * (warp % 4) + lane, i.e. that lane of tensor memory: row g + 8 h of tile rbi of the slot.  In
+    // a tile the row's nibbles are 64 contiguous bytes (its four k quarters of 16 bytes, each holding one word per 32-block), its
+    // scales 8 or 16 contiguous bytes.  The copy swizzles: bits 7..9 of a byte's place in the slot are added (xor) to
+    // bits 4..6, so that the eight rows that a quarter warp reads, 64 bytes apart, lie in all 32 banks instead of in eight.
+    const int q4 = warp & 3;
+    const int rbi = p.swiglu == 2 ? (lane >> 4) * 4 + q4 : 2 * q4 + (lane >> 4), h = (lane >> 3) & 1, g = lane & 7;
     bool ok = true;
     const int c = group & 1;                                    // which 64-k half of the 128-k tile
     int s = group, r = 0, within = group >> 1;                   // A/B slot; packed-tile slot and the tile inside it
@@ -232,10 +216,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     uint32_t tok_raw = mbar_test(&raw_full[r], rph), tok_empty = mbar_test(&empty[s], ph ^ 1u);
 #pragma unroll 1
     for (int kb = group; kb < n_kb && ok; kb += kUmmaGroups) {
-      // (with two terms in tensor memory the stage is only waited for when the first half of the row is converted:
+      // (with two terms the stage is only waited for when the first half of the row is converted:
       // the MMAs that last read it have that long to finish -- decode step at batch 64 8.27 -> 8.11 ms; with one term
       // the conversion is too short for that and the early wait measured 3 % better)
-      constexpr bool kLateWait = TS && TERMS == 2;
+      constexpr bool kLateWait = TERMS == 2;
       ok = !*failed && mbar_wait_token(&raw_full[r], rph, tok_raw) && (kLateWait || mbar_wait_token(&empty[s], ph ^ 1u, tok_empty));
       if (!ok) { give_up(DERR_FULL_WAIT); break; }
       const int s_cur = s, r_cur = r, within_cur = within;
@@ -254,125 +238,73 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
           rph ^= 1u;
         }
       }
-      uint8_t* a_hi = tiles_s + (size_t)s_cur * stage_bytes;
-      uint8_t* a_lo = a_hi + kUmmaRows * 128;
-      const uint8_t* raw = raw_s + ((size_t)r_cur * 8 * KT + within_cur) * TB;
-      if constexpr (TS) {
-        // ---- weights to tensor memory: this thread owns output row 32 * (warp % 4) + lane, i.e. that lane, and
-        // converts the row's 64 k of the stage.  In a fragment tile the row's nibbles are 64 contiguous bytes (its
-        // four k quarters of 16 bytes, each holding one word per 32-block), its scales 8 or 16 contiguous bytes.
-        if (!kLateWait) tc_fence_after();          // the stage's columns were last read by MMAs whose commit was waited for
-        const int q4 = warp & 3;
-        const int rbi = 2 * q4 + (lane >> 4), h = (lane >> 3) & 1, g = lane & 7;
-        const uint8_t* wrow = raw + rbi * KT * TB + (kIs8 ? h * 1024 + 512 * c : h * 512 + 8 * c) + g * 64;
-        const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS));
-        uint32_t sh = 0, sl = 0;
-        if constexpr (KIND != I8_ROW) {
-          const uint8_t* srow = raw + rbi * KT * TB + (kIs8 ? 2048 : 1024);
-          float2 f;
-          if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(srow + h * 64 + g * 8 + 4 * c));
-          else f = *reinterpret_cast<const float2*>(srow + h * 128 + g * 16 + 8 * c);
-          const __nv_bfloat162 shb = __floats2bfloat162_rn(f.x, f.y);
-          sh = *reinterpret_cast<const uint32_t*>(&shb);
-          const __nv_bfloat162 slb = __floats2bfloat162_rn(f.x - __uint_as_float(sh << 16), f.y - __uint_as_float(sh & 0xFFFF0000u));
-          sl = *reinterpret_cast<const uint32_t*>(&slb);
-        }
-        uint32_t wq[4][4];                         // [k quarter][word]: Q4 uses words 0, 1 (blocks 2c, 2c+1)
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          if constexpr (kIs8) {
-            const uint4 v = *reinterpret_cast<const uint4*>(wrow + 16 * t);
-            wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = v.z; wq[t][3] = v.w;
-          } else {
-            const uint2 v = *reinterpret_cast<const uint2*>(wrow + 16 * t);
-            wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = 0u; wq[t][3] = 0u;
-          }
-        }
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          uint32_t hi[16], lo[16];
-          const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u);
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t q[4];                         // (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t, exact ints
-            if constexpr (kIs8) dequant_i8_words(wq[t][2 * jj], wq[t][2 * jj + 1], q);
-            else dequant_q4_word(wq[t][jj], q);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if constexpr (KIND == I8_ROW) {
-                hi[4 * t + e] = q[e];
-              } else {
-                const uint32_t tt = bf16x2_mul(q[e], s_lo);
-                hi[4 * t + e] = bf16x2_fma(q[e], s_hi, tt);
-                if (TERMS == 2) lo[4 * t + e] = bf16x2_add(bf16x2_fma(q[e], s_hi, hi[4 * t + e] ^ 0x80008000u), tt);
-              }
-            }
-          }
-          if (kLateWait && jj == 0) {
-            // the stage's columns were last read by MMAs whose commit is waited for here
-            ok = __all_sync(0xffffffffu, mbar_wait_token(&empty[s_cur], ph_cur ^ 1u, tok_empty));
-            tc_fence_after();
-          }
-          if (ok) {
-            tmem_st16(a_t + (uint32_t)(16 * jj), hi);
-            if (TERMS == 2) tmem_st16(a_t + (uint32_t)(32 + 16 * jj), lo);
-          }
-        }
-        if (!ok) { give_up(DERR_EMPTY_WAIT); break; }
-        tmem_st_wait();
-        tc_fence_before();
-      } else {
-#pragma unroll
-      for (int i = 0; i < kCombos; ++i) {
-        if constexpr (KIND == I8_ROW) {
-          // int8 with one scale per output row: the integers go into the operand as they are (exact in bf16) and the
-          // row scale multiplies the accumulator in the epilogue -- an exact product with a single term
-          const uint4 w4 = *reinterpret_cast<const uint4*>(raw + src_off[i] + 512 * c);   // [even k | odd k] of blocks 2c, 2c+1
-#pragma unroll
-          for (int jj = 0; jj < 2; ++jj) {
-            uint32_t q[4];
-            dequant_i8_words(jj ? w4.z : w4.x, jj ? w4.w : w4.y, q);
-            *reinterpret_cast<uint4*>(a_hi + dst_off[i][jj]) = make_uint4(q[0], q[1], q[2], q[3]);
-          }
-          continue;
-        }
-        // blocks 2c, 2c+1: eight nibbles per word (Q4), or the [even k | odd k] byte planes of both blocks (Q8)
-        uint2 w2 = make_uint2(0u, 0u);
-        uint4 w8 = make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (KIND == Q8_F32) w8 = *reinterpret_cast<const uint4*>(raw + src_off[i] + 512 * c);
-        else w2 = *reinterpret_cast<const uint2*>(raw + src_off[i] + 8 * c);
+      const uint8_t* slot = raw_s + (size_t)r_cur * 8 * KT * TB;
+      const int tile_line = (rbi * KT + within_cur) * kTileLines;      // the tile's first line in the slot
+      if (!kLateWait) tc_fence_after();          // the stage's columns were last read by MMAs whose commit was waited for
+      const int line = tile_line + (kIs8 ? 8 * h + 4 * c : 4 * h) + (g >> 1);
+      const uint8_t* wrow = slot + line * 128 + (kIs8 ? 0 : 8 * c);
+      const int chunk0 = ((g & 1) * 4) ^ (line & 7);
+      const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS));
+      uint32_t sh = 0, sl = 0;
+      if constexpr (KIND != I8_ROW) {
         // The scale as s_hi + s_lo, two bf16 numbers (exact for an f16 scale: 11 = 8 + 3 significant bits).
         // With t = q*s_lo (7 bits, exact in bf16), hi = fma(q, s_hi, t) is the exact product rounded once;
-        // lo = fma(q, s_hi, -hi) + t = q*scale - hi, both steps exact, so hi + lo reproduces the product.
+        // lo = t - fma(q, -s_hi, hi) = q*scale - hi, both steps exact, so hi + lo reproduces the product.
         // (f32 scales keep their first 16 significant bits this way, and with int8 values t itself is rounded to 8
         // bits: hi + lo is then the product to within 2^-15 relative.)
         float2 f;
-        if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(raw + sc_off[i] + 4 * c));
-        else f = *reinterpret_cast<const float2*>(raw + sc_off[i] + 8 * c);
+        const int s_line = tile_line + (kIs8 ? 16 : 8) + (KIND == Q4_F16 ? 0 : h);
+        if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(slot + s_line * 128 + (((4 * h + (g >> 1)) ^ (s_line & 7)) << 4) + 8 * (g & 1) + 4 * c));
+        else f = *reinterpret_cast<const float2*>(slot + s_line * 128 + ((g ^ (s_line & 7)) << 4) + 8 * c);
         const __nv_bfloat162 shb = __floats2bfloat162_rn(f.x, f.y);
-        const uint32_t sh = *reinterpret_cast<const uint32_t*>(&shb);
+        sh = *reinterpret_cast<const uint32_t*>(&shb);
         const __nv_bfloat162 slb = __floats2bfloat162_rn(f.x - __uint_as_float(sh << 16), f.y - __uint_as_float(sh & 0xFFFF0000u));
-        const uint32_t sl = *reinterpret_cast<const uint32_t*>(&slb);
+        sl = *reinterpret_cast<const uint32_t*>(&slb);
+      }
+      uint32_t wq[4][4];                         // [k quarter][word]: Q4 uses words 0, 1 (blocks 2c, 2c+1)
 #pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-          const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u);
-          uint32_t q[4];
-          // (k0,k1) (k2,k3) (k4,k5) (k6,k7), exact ints
-          if constexpr (KIND == Q8_F32) dequant_i8_words(jj ? w8.z : w8.x, jj ? w8.w : w8.y, q);
-          else dequant_q4_word(jj ? w2.y : w2.x, q);
-          uint32_t hi[4], lo[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t t = bf16x2_mul(q[e], s_lo);
-            hi[e] = bf16x2_fma(q[e], s_hi, t);
-            if (TERMS == 2) lo[e] = bf16x2_add(bf16x2_fma(q[e], s_hi, hi[e] ^ 0x80008000u), t);
-          }
-          *reinterpret_cast<uint4*>(a_hi + dst_off[i][jj]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          if (TERMS == 2) *reinterpret_cast<uint4*>(a_lo + dst_off[i][jj]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      for (int t = 0; t < 4; ++t) {
+        if constexpr (kIs8) {
+          const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((chunk0 ^ t) << 4));
+          wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = v.z; wq[t][3] = v.w;
+        } else {
+          const uint2 v = *reinterpret_cast<const uint2*>(wrow + ((chunk0 ^ t) << 4));
+          wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = 0u; wq[t][3] = 0u;
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> visible to the MMA
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        uint32_t hi[16], lo[16];
+        const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u), minus_s_hi = s_hi ^ 0x80008000u;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          uint32_t q[4];                         // (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t, exact ints
+          if constexpr (kIs8) dequant_i8_words(wq[t][2 * jj], wq[t][2 * jj + 1], q);
+          else dequant_q4_word(wq[t][jj], q);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if constexpr (KIND == I8_ROW) {
+              hi[4 * t + e] = q[e];
+            } else {
+              const uint32_t tt = bf16x2_mul(q[e], s_lo);
+              hi[4 * t + e] = bf16x2_fma(q[e], s_hi, tt);
+              if (TERMS == 2) lo[4 * t + e] = bf16x2_sub(tt, bf16x2_fma(q[e], minus_s_hi, hi[4 * t + e]));
+            }
+          }
+        }
+        if (kLateWait && jj == 0) {
+          // the stage's columns were last read by MMAs whose commit is waited for here
+          ok = __all_sync(0xffffffffu, mbar_wait_token(&empty[s_cur], ph_cur ^ 1u, tok_empty));
+          tc_fence_after();
+        }
+        if (ok) {
+          tmem_st16(a_t + (uint32_t)(16 * jj), hi);
+          if (TERMS == 2) tmem_st16(a_t + (uint32_t)(32 + 16 * jj), lo);
+        }
       }
+      if (!ok) { give_up(DERR_EMPTY_WAIT); break; }
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) {                                                // one arrival per warp
         mbar_arrive(&a_full[s_cur]);
@@ -388,7 +320,6 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
     if (!ok) give_up(DERR_TMEM);
     tc_fence_after();
     if (ok) {
-      const int q4 = warp & 3;                                 // tensor-memory lane quarter this warp may read
       const int n = blockIdx.x * kUmmaRows + 32 * q4 + lane;
       // two warps share a lane quarter and alternate over the 16-column chunks
       for (int tile = 0; tile < kTokTiles; ++tile)
@@ -449,7 +380,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const UmmaParams p)
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_d, (uint32_t)p.tmem_cols);
+  if (warp == 1) tmem_dealloc(tmem_d, 512);
   if (p.splits > 1) {
     // Deterministic split-K meet: every CTA of the tile counts in after its partial is visible; the one
     // that counts in last sums the partials in split order (so the result does not depend on which CTA
@@ -518,21 +449,12 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   TQ_REQUIRE(ctx, ((uintptr_t)x_bf16 & 15) == 0 && (ldx * 2) % 16 == 0, "tcgen05 GEMM: activation rows must be 16-byte aligned");
   // Ring sizes.  Two rules come from the dequant groups running ahead of one another (a parity wait
   // is only sound when the waiter is at most one phase ahead of the barrier): at least kUmmaGroups
-  // A/B stages, and an even number of packed-tile slots whenever slots are reused.  The token tile is
-  // the widest that leaves room for four stages and four packed tiles, then evened out over the tiles.
+  // stages, and an even number of packed-tile slots whenever slots are reused.  Four stages of weights take 32
+  // columns of tensor memory per term each; the rest holds the accumulators, two at least (one per issuing warp): token
+  // tiles up to 128 with two terms, up to 192 with one, evened out over the tiles.
   const size_t kSmemMax = 227 * 1024, raw_tile = 8 * (size_t)qk_tile_bytes(w->kind);
   const size_t budget = kSmemMax - kUmmaHeader - 1024;
-  int ntok_max = (int)(((budget - 4 * raw_tile) / kUmmaGroups - (size_t)terms * kUmmaRows * 128) / 128) / 16 * 16;
-  if (ntok_max > 256) ntok_max = 256;
-  // The dequantised weights in tensor memory instead of shared memory: writing them there and having the tensor core
-  // read them back is what fills the shared-memory pipe (32 KB written + 32 KB read per 64-k step with two terms).
-  // Four stages of weights take 32 columns per term each; the rest holds the accumulators, two at least (one per
-  // issuing warp): token tiles up to 128 with two terms, up to 192 with one.
-  // With one term the shared-memory operand allows wider token tiles: it stays where the narrower tiles would mean
-  // more of them, i.e. more conversions of the same weights (2048 rows: 9 tiles of 228 against 11 of 192 measured
-  // the same; 512 rows, three tiles either way: 95 -> 77 us).
-  const size_t m_basis = grp ? (size_t)grp->expected_rows : m;
-  const int ts_cap = terms == 2 ? kUmmaTwoTermTokens : 192;
+  const int ntok_max = terms == 2 ? kUmmaTwoTermTokens : 192;
   // Many rows, one term: a CTA takes TWO token tiles (each MMA issuer multiplies every stage with its own tile's
   // activations), so the weights are converted once per 2 x <= 192 tokens; the accumulators are 2 x 192 columns, the
   // weights 128.  Only where that still gives about a wave of CTAs (no K split in this form).
@@ -548,8 +470,6 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
       dual = !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)n_pairs);
     }
   }
-  const int ts = (dual || terms == 2 || (m_basis + ts_cap - 1) / ts_cap <= (m_basis + ntok_max - 1) / ntok_max) ? 1 : 0;
-  if (ts && (ntok_max > ts_cap || terms == 2)) ntok_max = ts_cap;
   const size_t rows_g = grp ? w->rows / grp->n_groups : w->rows;       // output features per group
   if (grp) TQ_REQUIRE(ctx, grp->n_groups > 0 && w->rows % grp->n_groups == 0 && rows_g % kUmmaRows == 0 && grp->counts && grp->offsets,
                       "tcgen05 GEMM: every group needs a multiple of 128 output features");
@@ -577,27 +497,31 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   splits = (w->n_kc + kc_per_split - 1) / kc_per_split;
   int acc_stride = 32;
   while (acc_stride < ntok) acc_stride <<= 1;
-  if (ts && ntok > 128) acc_stride = 192;
-  const int acc_cols = ts ? 512 - 128 * terms : 512;
-  int n_acc = 2;                       // a power of two: 16 accumulators up to 32 tokens, 8 at 64, 4 at 128, 2 at 256 in
-  while (!dual && n_acc < 16 && 2 * n_acc * acc_stride <= acc_cols) n_acc <<= 1;   // all of tensor memory, fewer beside the weights
-  const int tmem_cols = ts ? 512 : n_acc * acc_stride;
+  if (ntok > 128) acc_stride = 192;
+  const int acc_cols = 512 - 128 * terms;
+  int n_acc = 2;                       // a power of two, as many as tensor memory holds beside the weights
+  while (!dual && n_acc < 16 && 2 * n_acc * acc_stride <= acc_cols) n_acc <<= 1;
   // Four A/B stages are what the dequant groups need; everything else goes to the packed-tile ring, because
   // the bytes in flight from HBM (ring slots not being read) are what hides its latency.  A ring slot holds
-  // KT = 4 k-tiles of the eight row blocks (eight 4.6 KB copies) when three such slots fit, else KT = 2.
+  // KT = 4 k-tiles of the eight row blocks (two copies of 18 KB) when three such slots fit, else KT = 2.
   int stages = kUmmaGroups;
   // Two terms and up to 32 tokens: four accumulators take 128 columns, which leaves room for SIX stages of weights, so
   // that a converting group need not wait for the MMAs of its own previous stage (decode step at 20 / 32 rows:
   // 5.16 -> 5.06 ms / 5.82 -> 5.71 ms).
   int a_col0 = acc_cols;
-  if (ts && terms == 2 && acc_stride == 32) {
+  if (terms == 2 && acc_stride == 32) {
     stages = 6;
     n_acc = 4;
     a_col0 = 128;
   }
-  if ((budget - 4 * raw_tile) / umma_stage_bytes(terms, ntok_stage, ts) < (size_t)stages)
+  // One term and up to 64 tokens: eight stages (28672 x 4096 at 64 rows 45.2 -> 42.0 us).
+  if (terms == 1 && acc_stride <= 64) {
+    stages = 8;
+    a_col0 = 256;
+  }
+  if ((budget - 4 * raw_tile) / umma_stage_bytes(ntok_stage) < (size_t)stages)
     return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: token tile of %d does not fit", ntok);
-  const size_t avail = budget - (size_t)stages * umma_stage_bytes(terms, ntok_stage, ts);
+  const size_t avail = budget - (size_t)stages * umma_stage_bytes(ntok_stage);
   int kt = avail / (4 * raw_tile) >= 3 ? 4 : 2;
   int raw_stages = (int)(avail / ((size_t)kt * raw_tile));
   if (raw_stages > kUmmaMaxRawStages) raw_stages = kUmmaMaxRawStages;
@@ -606,8 +530,10 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   if (stages < kUmmaGroups || raw_stages < 1) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: ring sizes %d/%d", stages, raw_stages);
   CUtensorMap map;
   if (!encode_bf16_k64(&map, x_bf16, m, w->cols, ldx, (unsigned)ntok)) return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
+  CUtensorMap w_map;   // the packed tiles as 128-byte lines, boxes of kt tiles of four row blocks
+  if (!encode_lines128(&w_map, w->tiles, (size_t)w->n_kc * (qk_tile_bytes(w->kind) / 128), (size_t)w->n_rb, (unsigned)(kt * (qk_tile_bytes(w->kind) / 128)), 4))
+    return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
   UmmaParams p;
-  p.tiles = w->tiles;
   p.row_scales = w->row_scales;
   p.y = y;
   p.ldy = (long long)ldy;
@@ -616,13 +542,10 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.g_counts = grp ? grp->counts : nullptr;
   p.g_offsets = grp ? grp->offsets : nullptr;
   p.g_active = grp ? grp->active : nullptr;
-  p.g_tile_stride = (long long)(rows_g / kTileRows) * w->n_kc * qk_tile_bytes(w->kind);
   p.kc_total = w->n_kc;
   p.ntok = ntok;
-  p.tmem_cols = tmem_cols;
   p.acc_stride = acc_stride;
   p.n_acc = n_acc;
-  p.ts = ts;
   p.a_col0 = a_col0;
   p.y_bf16 = y_dtype == TQ_BF16;
   TQ_REQUIRE(ctx, swiglu != 2 || w->kind != TQ_I8_ROW, "tcgen05 GEMM: gate and up halves with row scales");
@@ -640,7 +563,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.stages = stages;
   p.raw_stages = raw_stages;
   p.kt = kt;
-  const size_t smem = umma_smem_bytes(w->kind, terms, ntok_stage, stages, raw_stages * kt, ts);
+  const size_t smem = umma_smem_bytes(w->kind, ntok_stage, stages, raw_stages * kt);
   if (smem > kSmemMax) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
   dim3 grid((unsigned)(rows_g / kUmmaRows), (unsigned)((m + ntok_stage - 1) / ntok_stage), (unsigned)splits);
   if (grp) {
@@ -650,20 +573,15 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_k(ctx, kern, grid, dim3(kUmmaThreads), smem, map, p);
+    return launch_k(ctx, kern, grid, dim3(kUmmaThreads), smem, map, w_map, p);
   };
   cudaError_t e;
   if (dual) {
     if (splits != 1) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: two token tiles per CTA with K split");
-    if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1, true, true>);
-    else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 1, true, true>);
-    else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 1, true, true>);
-    else e = go(qgemm_umma_kernel<Q4_F32, 1, true, true>);
-  } else if (ts) {
     if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1, true>);
-    else if (w->kind == TQ_Q4_F16) e = terms == 2 ? go(qgemm_umma_kernel<Q4_F16, 2, true>) : go(qgemm_umma_kernel<Q4_F16, 1, true>);
-    else if (w->kind == TQ_Q8_F32) e = terms == 2 ? go(qgemm_umma_kernel<Q8_F32, 2, true>) : go(qgemm_umma_kernel<Q8_F32, 1, true>);
-    else e = terms == 2 ? go(qgemm_umma_kernel<Q4_F32, 2, true>) : go(qgemm_umma_kernel<Q4_F32, 1, true>);
+    else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 1, true>);
+    else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 1, true>);
+    else e = go(qgemm_umma_kernel<Q4_F32, 1, true>);
   } else if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1>);
   else if (w->kind == TQ_Q4_F16) e = terms == 2 ? go(qgemm_umma_kernel<Q4_F16, 2>) : go(qgemm_umma_kernel<Q4_F16, 1>);
   else if (w->kind == TQ_Q8_F32) e = terms == 2 ? go(qgemm_umma_kernel<Q8_F32, 2>) : go(qgemm_umma_kernel<Q8_F32, 1>);

@@ -46,7 +46,6 @@ constexpr int kUmmaFirstDqWarp = 4;   // warps 0..3: weight producer, MMA issuer
 constexpr int kUmmaThreads = 32 * (kUmmaFirstDqWarp + kUmmaDqWarps);
 
 struct UmmaParams {
-  const uint8_t* tiles;   // fragment tiles [n_row_blocks][kc_total][tile_bytes]
   const float* row_scales;   // TQ_I8_ROW: one scale per output row (applied to the accumulator), else unused
   void* y;                // [M][ldy] f32 or bf16
   long long ldy;
@@ -54,12 +53,8 @@ struct UmmaParams {
   int n_rows;             // output features (multiple of 128)
   int kc_total;           // K / 128
   int ntok;               // tokens per CTA tile = UMMA N (multiple of 16, <= 256)
-  int tmem_cols;          // allocation: n_acc accumulators, power of two
   int acc_stride;         // columns between accumulators
-  int ts;                 // 1: the dequantised weights go to tensor memory (columns a_col0 ..: stages x terms x 32), not to
-                          //    shared memory, and the MMA reads them from there; a stage in shared memory is then the
-                          //    activation box alone
-  int a_col0;
+  int a_col0;             // tensor-memory columns of the converted weights: stages x terms x 32 from here on
   int n_acc;              // accumulators (2, 4, 8 or 16): step kb adds into number (kb & 1) + 2 * ((kb >> 1) % (n_acc / 2))
   int stages;             // A/B ring depth
   int raw_stages;         // packed-tile ring depth (slots of kt tiles of 128 k): what keeps the HBM stream in flight
@@ -75,7 +70,6 @@ struct UmmaParams {
   const int* g_counts;    // grouped launches (experts stacked by rows): rows of x / y per group, or null
   const int* g_offsets;   // first row of each group
   const int* g_active;    // optional list of group ids with rows (-1 = unused entry); blockIdx.z indexes it
-  long long g_tile_stride;   // bytes between the groups' fragment tiles
   int* err;
 };
 
@@ -90,13 +84,11 @@ struct UmmaGroups {
   int expected_rows = 0;   // typical counts[e]: sets the token tile
 };
 
-__host__ __device__ inline size_t umma_stage_bytes(int terms, int ntok, int ts = 0) {
-  return (ts ? 0 : (size_t)terms * kUmmaRows * 128) + (size_t)ntok * 128;   // A tiles + B tile, all 1024-aligned sizes
-}
-constexpr int kUmmaMaxRawStages = 16;
+__host__ __device__ inline size_t umma_stage_bytes(int ntok) { return (size_t)ntok * 128; }   // an activation box
+constexpr int kUmmaMaxRawStages = 16, kUmmaMaxStages = 8;
 constexpr int kUmmaHeader = 1024;
-__host__ __device__ inline size_t umma_smem_bytes(int kind, int terms, int ntok, int stages, int raw_tiles, int ts = 0) {
-  return kUmmaHeader + 1024 /*alignment slack*/ + (size_t)stages * umma_stage_bytes(terms, ntok, ts) +
+__host__ __device__ inline size_t umma_smem_bytes(int kind, int ntok, int stages, int raw_tiles) {
+  return kUmmaHeader + 1024 /*alignment slack*/ + (size_t)stages * umma_stage_bytes(ntok) +
          (size_t)raw_tiles * 8 * qk_tile_bytes(kind);
 }
 
@@ -106,6 +98,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
           smem_u32(dst)),
       "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot_smem, uint32_t ncols) {

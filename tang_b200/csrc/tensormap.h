@@ -38,4 +38,17 @@ inline bool encode_bf16_k64(CUtensorMap* map, const void* base, size_t rows, siz
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Bytes [blocks][lines][128], boxes of `box_lines` lines of `box_blocks` blocks in the 128-byte swizzle (16-byte chunk c of line l
+// of a 1024-byte aligned destination lands at chunk c ^ (l & 7)); lines behind a block's last read as zeros.
+inline bool encode_lines128(CUtensorMap* map, const void* base, size_t lines, size_t blocks, unsigned box_lines, unsigned box_blocks) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t gdim[3] = {128, (cuuint64_t)lines, (cuuint64_t)blocks};
+  const cuuint64_t gstride[2] = {128, (cuuint64_t)lines * 128};
+  const cuuint32_t box[3] = {128, box_lines, box_blocks};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace tq
