@@ -229,6 +229,16 @@ __device__ __forceinline__ void dequant_q4_word(uint32_t w, uint32_t (&out)[4]) 
   out[3] = bf16x2_sub(lop3_and_or(w >> 12, kMask, kMagic), kBias);
 }
 
+// The same unpacking, 24 + q instead of q (the nibble in the upper bits of the mantissa of 16.0, exact): 24 has two significant bits, so
+// that fma(24 + q, s, -24 s) = q s is exact wherever s has at most six and the product at most eight.
+__device__ __forceinline__ void dequant_q4_word_24(uint32_t w, uint32_t (&out)[4]) {
+  constexpr uint32_t kMask = 0x00780078u, kMagic = 0x41804180u;
+  out[0] = lop3_and_or(w << 3, kMask, kMagic);
+  out[1] = lop3_and_or(w >> 1, kMask, kMagic);
+  out[2] = lop3_and_or(w >> 5, kMask, kMagic);
+  out[3] = lop3_and_or(w >> 9, kMask, kMagic);
+}
+
 // The same unpacking without the bias removal: out holds 128 + n = 136 + q.  A contraction over these
 // is corrected by one more MMA whose A operand is the constant -136 (kNeg136x2 in every register):
 // sum (136 + q) x + sum (-136) x = sum q x, with every product still exact in f32.

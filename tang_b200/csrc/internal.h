@@ -24,8 +24,8 @@ struct tq_ctx {
   cudaStream_t stream = nullptr;
   bool owns_stream = false;
   int* dev_err = nullptr;        // device status word written by kernels that give up a bounded wait,
-                                 // followed by kTileCounters zeroed tile counters (split-K meets of the tcgen05
-                                 // GEMM and the MoE router) and kTileCounters more for the persistent GEMV
+                                 // followed by kTileCounters zeroed tile counters (split-K meets of the dense
+                                 // tcgen05 GEMM and the MoE router) and kTileCounters more for the persistent GEMV
   int* skg_jobs = nullptr;                 // [kSkgJobs] job list of a grouped persistent launch (rebuilt by every such launch)
   unsigned long long* gemm_ws2 = nullptr;  // the several-row persistent kernel's per-(slab, row block) parked sums (zero between launches)
   size_t gemm_ws2_bytes = 0;
@@ -48,6 +48,7 @@ struct tq_ctx {
   void* splitk = nullptr;        // f32 partials of split-K GEMMs; separate because callers that carve
   size_t splitk_bytes = 0;       // their own buffers out of `scratch` run linear layers in between
   int sm_count = 148;
+  int umma_clusters[9] = {};     // clusters of that many CTAs of the tcgen05 GEMM that run at once (0: not asked yet, -1: none)
   // Kernels that may still be running when the next kernel launched with the programmatic-launch attribute
   // starts: either exactly the previous one, with unknown outputs (`inflight_unknown`; every kernel but the
   // persistent GEMV waits for its predecessor before it lets its successor be scheduled), or a run of
@@ -177,9 +178,9 @@ inline cudaError_t launch_k(tq_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
-// The same for a kernel whose blocks form clusters of `cluster` along x.
+// The same for a kernel whose blocks form clusters.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k_cluster(tq_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, Args... args) {
+inline cudaError_t launch_k_cluster(tq_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, dim3 cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -187,8 +188,9 @@ inline cudaError_t launch_k_cluster(tq_ctx* ctx, void (*kern)(KArgs...), dim3 gr
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.x = cluster.x;
+  attr[0].val.clusterDim.y = cluster.y;
+  attr[0].val.clusterDim.z = cluster.z;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;

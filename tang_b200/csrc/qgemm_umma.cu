@@ -8,12 +8,41 @@
 
 namespace tq {
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The sum of the four floats at `mine` over the first n CTAs of the cluster, in their order.
+__device__ __forceinline__ float4 cluster_sum(const float* mine, int n) {
+  const uint32_t a = smem_u32(mine);
+  float4 v[kUmmaMaxSplits];
+#pragma unroll
+  for (int z = 0; z < kUmmaMaxSplits; ++z) {
+    if (z >= n) break;
+    uint32_t there;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(a), "r"(z));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[z].x), "=f"(v[z].y), "=f"(v[z].z), "=f"(v[z].w) : "r"(there) : "memory");
+  }
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int z = 0; z < kUmmaMaxSplits; ++z) {
+    if (z >= n) break;
+    sum.x += v[z].x;
+    sum.y += v[z].y;
+    sum.z += v[z].z;
+    sum.w += v[z].w;
+  }
+  return sum;
+}
+__device__ __forceinline__ float4 times(float4 v, const float* s) { return make_float4(v.x * s[0], v.y * s[1], v.z * s[2], v.w * s[3]); }
+
 template <int KIND, int TERMS, bool DUAL = false>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ UmmaParams p) {
   extern __shared__ uint8_t smem_raw[];
   constexpr int TB = (KIND == I8_ROW) ? 2048 : (KIND == Q8_F32) ? 2304 : (KIND == Q4_F16) ? 1152 : 1280;
   constexpr bool kIs8 = KIND == I8_ROW || KIND == Q8_F32;
+  constexpr bool kExactSplit = KIND == Q4_F16 && TERMS == 2;
   constexpr int kTileLines = TB / 128;   // 128-byte lines of a tile: its weights, then its scales
   static_assert(KIND != I8_ROW || TERMS == 1, "int8 rows carry no scale into the operand: one exact term");
   // DUAL: the CTA covers two token tiles of p.ntok rows with one conversion of the weights: issuer warp 1 multiplies
@@ -34,6 +63,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   const uint32_t base_u32 = smem_u32(smem_raw);
   uint8_t* tiles_s = smem_raw + kUmmaHeader + ((1024 - ((base_u32 + kUmmaHeader) & 1023)) & 1023);  // 1024-aligned
   const size_t stage_bytes = umma_stage_bytes(p.ntok) * kTokTiles;
+  float* part_s = reinterpret_cast<float*>(tiles_s);            // K split: this CTA's partial sums, when the rings are done with
   uint8_t* raw_s = tiles_s + (size_t)p.stages * stage_bytes;   // [raw stages][8 tiles]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -64,19 +94,24 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   const int kc_len = min(p.kc_per_split, p.kc_total - kc_begin);
   const int n_kb = kc_len * 2;                                 // 64-k steps
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&x_full[s], 1);
-      mbar_init(&a_full[s], kUmmaGroupWarps);
-      mbar_init(&empty[s], DUAL ? 2 : 1);   // one commit per issuer that reads the stage
+  if (warp == 0) {
+    if (lane < S) {
+      mbar_init(&x_full[lane], 1);
+      mbar_init(&a_full[lane], kUmmaGroupWarps);
+      mbar_init(&empty[lane], DUAL ? 2 : 1);   // one commit per issuer that reads the stage
     }
-    for (int r = 0; r < RS; ++r) {
-      mbar_init(&raw_full[r], 1);
-      mbar_init(&raw_empty[r], kUmmaDqWarps);          // every group reads some tile of every ring slot
+    if (lane < RS) {
+      mbar_init(&raw_full[lane], 1);
+      mbar_init(&raw_empty[lane], kUmmaDqWarps);          // every group reads some tile of every ring slot
     }
-    mbar_init(acc_full, 2);
-    *failed = 0;
+    if (lane == 0) {
+      mbar_init(acc_full, 2);
+      *failed = 0;
+    }
     mbar_init_fence();
+  } else if (warp == 2 && lane == 0) {
+    prefetch_map(&x_map);
+    prefetch_map(&w_map);
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
@@ -84,7 +119,8 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
 
-  pdl_wait();
+  // (weights are not written by a kernel in flight: they stream and are converted before the wait for the activations, which
+  // the thread that copies them does; everything that is stored depends on these)
   pdl_launch_dependents();
 
   auto give_up = [&](int code) {
@@ -115,6 +151,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   } else if (warp == 2) {
     // ------------------------------------------------------------------ activation producer
     if (lane == 0) {
+      pdl_wait();
       int s = 0;
       uint32_t ph = 0;
       for (int kb = 0; kb < n_kb && !*failed; ++kb) {
@@ -247,7 +284,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS));
       uint32_t sh = 0, sl = 0;
       if constexpr (KIND != I8_ROW) {
-        // The scale as s_hi + s_lo, two bf16 numbers (exact for an f16 scale: 11 = 8 + 3 significant bits).
+        // Two terms of Q4 with f16 scales: s_hi = the scale rounded to five significant bits and s_lo = the rest, which has
+        // five too (of 11, rounded to nearest).  The integers have three (or are -8), so both products are exact in bf16, and
+        // so is 24 * s: each term is one fma over 24 + q, half the instructions of the general form below.
+        // General form: the scale as s_hi + s_lo, two bf16 numbers (exact for an f16 scale: 11 = 8 + 3 significant bits).
         // With t = q*s_lo (7 bits, exact in bf16), hi = fma(q, s_hi, t) is the exact product rounded once;
         // lo = t - fma(q, -s_hi, hi) = q*scale - hi, both steps exact, so hi + lo reproduces the product.
         // (f32 scales keep their first 16 significant bits this way, and with int8 values t itself is rounded to 8
@@ -256,10 +296,16 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         const int s_line = tile_line + (kIs8 ? 16 : 8) + (KIND == Q4_F16 ? 0 : h);
         if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(slot + s_line * 128 + (((4 * h + (g >> 1)) ^ (s_line & 7)) << 4) + 8 * (g & 1) + 4 * c));
         else f = *reinterpret_cast<const float2*>(slot + s_line * 128 + ((g ^ (s_line & 7)) << 4) + 8 * c);
+        if constexpr (kExactSplit) {
+          const uint32_t h0 = (__float_as_uint(f.x) + 0x40000u) & 0xFFF80000u, h1 = (__float_as_uint(f.y) + 0x40000u) & 0xFFF80000u;
+          sh = prmt(h0, h1, 0x7632u);
+          sl = prmt(__float_as_uint(f.x - __uint_as_float(h0)), __float_as_uint(f.y - __uint_as_float(h1)), 0x7632u);
+        } else {
         const __nv_bfloat162 shb = __floats2bfloat162_rn(f.x, f.y);
         sh = *reinterpret_cast<const uint32_t*>(&shb);
         const __nv_bfloat162 slb = __floats2bfloat162_rn(f.x - __uint_as_float(sh << 16), f.y - __uint_as_float(sh & 0xFFFF0000u));
         sl = *reinterpret_cast<const uint32_t*>(&slb);
+        }
       }
       uint32_t wq[4][4];                         // [k quarter][word]: Q4 uses words 0, 1 (blocks 2c, 2c+1)
 #pragma unroll
@@ -275,6 +321,20 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
 #pragma unroll
       for (int jj = 0; jj < 2; ++jj) {
         uint32_t hi[16], lo[16];
+        if constexpr (kExactSplit) {
+          const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u);
+          const uint32_t c_hi = bf16x2_mul(s_hi, 0xC1C0C1C0u), c_lo = bf16x2_mul(s_lo, 0xC1C0C1C0u);   // -24 s
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            uint32_t v[4];                         // 24 + q of (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t
+            dequant_q4_word_24(wq[t][jj], v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              hi[4 * t + e] = bf16x2_fma(v[e], s_hi, c_hi);
+              lo[4 * t + e] = bf16x2_fma(v[e], s_lo, c_lo);
+            }
+          }
+        } else {
         const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u), minus_s_hi = s_hi ^ 0x80008000u;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -291,6 +351,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
               if (TERMS == 2) lo[4 * t + e] = bf16x2_sub(tt, bf16x2_fma(q[e], minus_s_hi, hi[4 * t + e]));
             }
           }
+        }
         }
         if (kLateWait && jj == 0) {
           // the stage's columns were last read by MMAs whose commit is waited for here
@@ -341,13 +402,10 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
           }
         }
         if (p.splits > 1) {
-          // K is split over gridDim.z CTAs: park the f32 partial; the last CTA of the tile adds them up
-          float* part = p.partial + (size_t)blockIdx.z * p.m_total * p.n_rows;
+          // K is split over the CTAs of a cluster: the f32 partial sums go to shared memory (the rings are free: every MMA is done),
+          // [token][128 features]
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int m = mt + c0 + i;
-            if (m < m_end) __stcg(part + (size_t)m * p.n_rows + n, v[i]);
-          }
+          for (int i = 0; i < 16; ++i) part_s[(c0 + i) * kUmmaRows + 32 * q4 + lane] = v[i];
         } else if (p.swiglu) {
           // A gate row's up row sits eight lanes on (interleaved rows), or sixteen (halves: lanes 0..15 hold a gate block, 16..31 its
           // up block).  Of every two columns the gate lanes finish the first, the up lanes the second.
@@ -382,44 +440,45 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_d, 512);
   if (p.splits > 1) {
-    // Deterministic split-K meet: every CTA of the tile counts in after its partial is visible; the one
-    // that counts in last sums the partials in split order (so the result does not depend on which CTA
-    // that was), writes y and leaves the counter at zero for the next launch.
-    __shared__ int is_last;
-    __threadfence();
-    __syncthreads();
-    int* counter = p.counters + blockIdx.y * gridDim.x + blockIdx.x;
-    if (threadIdx.x == 0) {
-      const int seen = atomicAdd(counter, 1);
-      is_last = seen == p.splits - 1;
-      if (is_last) *counter = 0;
-    }
-    __syncthreads();
-    if (is_last) {
-      __threadfence();
-      const int m_hi = min(p.ntok, p.m_total - m0);
-      const size_t plane = (size_t)p.m_total * p.n_rows;
-      for (int idx = threadIdx.x; idx < m_hi * kUmmaRows; idx += blockDim.x) {
-        const int m = m0 + idx / kUmmaRows, n = blockIdx.x * kUmmaRows + idx % kUmmaRows;
-        const float* src = p.partial + (size_t)m * p.n_rows + n;
-        float sum = 0.f;
-        for (int z = 0; z < p.splits; ++z) sum += __ldcg(src + z * plane);
-        if constexpr (KIND == I8_ROW) sum *= row_scales[n];
-        if (p.swiglu) {
-          if (n & 8) continue;                                   // up rows are folded into their gate rows
-          float up = 0.f;
-          for (int z = 0; z < p.splits; ++z) up += __ldcg(src + 8 + z * plane);
-          if constexpr (KIND == I8_ROW) up *= row_scales[n + 8];
-          const float act = sum * (1.0f / (1.0f + expf(-sum))) * up;
-          const size_t o = (size_t)m * p.ldy + (n >> 4) * 8 + (n & 7);
-          if (p.y_bf16) reinterpret_cast<__nv_bfloat16*>(p.y)[o] = __float2bfloat16_rn(act);
-          else reinterpret_cast<float*>(p.y)[o] = act;
-          continue;
+    // Every CTA of the cluster adds up its share of the tokens over all of them, in split order (reproducible), and stores it.
+    cluster_sync();
+    const int m_hi = min(p.ntok, p.m_total - m0), share = (m_hi + p.splits - 1) / p.splits;
+    const int t_lo = (int)blockIdx.z * share, t_n = min(share, m_hi - t_lo);
+    for (int idx = threadIdx.x; idx < t_n * (kUmmaRows / 4); idx += kUmmaThreads) {
+      const int t = t_lo + idx / (kUmmaRows / 4), r = idx % (kUmmaRows / 4) * 4;
+      if (p.swiglu && (r & 8)) continue;                       // up rows are folded into their gate rows
+      float4 sum = cluster_sum(part_s + t * kUmmaRows + r, p.splits);
+      const int n = blockIdx.x * kUmmaRows + r;
+      int o_col = n;
+      if constexpr (KIND == I8_ROW) sum = times(sum, row_scales + n);
+      if (p.swiglu) {
+        float4 up = cluster_sum(part_s + t * kUmmaRows + r + 8, p.splits);
+        if constexpr (KIND == I8_ROW) up = times(up, row_scales + n + 8);
+        sum.x = sum.x * (1.0f / (1.0f + expf(-sum.x))) * up.x;
+        sum.y = sum.y * (1.0f / (1.0f + expf(-sum.y))) * up.y;
+        sum.z = sum.z * (1.0f / (1.0f + expf(-sum.z))) * up.z;
+        sum.w = sum.w * (1.0f / (1.0f + expf(-sum.w))) * up.w;
+        o_col = (n >> 4) * 8 + (n & 7);
+      }
+      const size_t o = (size_t)(m0 + t) * p.ldy + o_col;
+      const __nv_bfloat162 b0 = __floats2bfloat162_rn(sum.x, sum.y), b1 = __floats2bfloat162_rn(sum.z, sum.w);
+      if (p.y_bf16) {
+        __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(p.y) + o;
+        if (p.y_vec4) {
+          *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
+        } else {
+          y[0] = b0.x; y[1] = b0.y; y[2] = b1.x; y[3] = b1.y;
         }
-        if (p.y_bf16) reinterpret_cast<__nv_bfloat16*>(p.y)[(size_t)m * p.ldy + n] = __float2bfloat16_rn(sum);
-        else reinterpret_cast<float*>(p.y)[(size_t)m * p.ldy + n] = sum;
+      } else {
+        float* y = reinterpret_cast<float*>(p.y) + o;
+        if (p.y_vec4) {
+          *reinterpret_cast<float4*>(y) = sum;
+        } else {
+          y[0] = sum.x; y[1] = sum.y; y[2] = sum.z; y[3] = sum.w;
+        }
       }
     }
+    cluster_sync();                                            // nobody leaves while its partial sums are read
   }
 }
 
@@ -436,6 +495,31 @@ constexpr int kUmmaTwoTermTokens = 128;   // token tile of two-term products: wh
 // Whether two-term products of m rows run without a split of K.
 bool umma_fills_gpu(const tq_ctx* ctx, const tq_qweight* w, size_t m) {
   return !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)((m + kUmmaTwoTermTokens - 1) / kUmmaTwoTermTokens));
+}
+
+// How many clusters of `size` CTAs of this kernel the GPU holds at once (a CTA has an SM to itself, whatever its shared memory).
+static int umma_clusters(tq_ctx* ctx, int size) {
+  int& n = ctx->umma_clusters[size];
+  if (n == 0) {
+    auto kern = qgemm_umma_kernel<Q4_F16, 2>;
+    constexpr size_t kSmem = 200 * 1024;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(kUmmaThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = (unsigned)size;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = -1;
+    }
+  }
+  return n;
 }
 
 // y[m, rows] = x[m, cols] . W^T through the tcgen05 kernel.  x: bf16, 16-byte aligned rows.
@@ -487,10 +571,8 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   if (!grp && swiglu != 2 && umma_few_tiles(ctx, base_ctas)) {
     splits = ctx->sm_count / base_ctas;
     if (splits > w->n_kc / 4) splits = w->n_kc / 4;      // at least eight 64-k steps per CTA
-    if (splits > 16) splits = 16;
-    // the f32 partials are written and read once more: keep them below the bytes of the weights themselves
-    const size_t wbytes = (size_t)w->n_rb * w->n_kc * qk_tile_bytes(w->kind), pbytes = m * w->rows * 8;
-    if ((size_t)splits > wbytes / pbytes) splits = (int)(wbytes / pbytes);
+    if (splits > kUmmaMaxSplits) splits = kUmmaMaxSplits;
+    while (splits > 1 && umma_clusters(ctx, splits) < base_ctas) --splits;   // (all of them at once: one wave)
     if (splits < 1) splits = 1;
   }
   const int kc_per_split = (w->n_kc + splits - 1) / splits;
@@ -553,13 +635,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.err = ctx->dev_err;
   p.splits = splits;
   p.kc_per_split = kc_per_split;
-  p.partial = nullptr;
-  p.counters = ctx->dev_err + 1;
-  if (splits > 1) {
-    if (base_ctas > kTileCounters) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %d output tiles with split K", base_ctas);
-    if (int st = ensure_splitk(ctx, (size_t)splits * m * w->rows * sizeof(float))) return st;
-    p.partial = static_cast<float*>(ctx->splitk);
-  }
+  p.y_vec4 = ldy % 4 == 0 && ((uintptr_t)y & (p.y_bf16 ? 7 : 15)) == 0;
   p.stages = stages;
   p.raw_stages = raw_stages;
   p.kt = kt;
@@ -573,6 +649,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
+    if (splits > 1) return launch_k_cluster(ctx, kern, grid, dim3(kUmmaThreads), smem, dim3(1, 1, splits), map, w_map, p);
     return launch_k(ctx, kern, grid, dim3(kUmmaThreads), smem, map, w_map, p);
   };
   cudaError_t e;

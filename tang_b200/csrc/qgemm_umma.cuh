@@ -63,10 +63,9 @@ struct UmmaParams {
   int swiglu;             // 1: the weight is a gate/up projection in the interleaved row order (rows 0..7 of every 16 gate, rows
                           // 8..15 the matching up rows); 2: gate rows in the first half of the weight's (group's) rows, up rows in
                           // the second (no K split).  y [M][n_rows / 2] = silu(gate) * up, formed from the f32 sums
-  int splits;             // CTAs along K per output tile (gridDim.z)
+  int splits;             // CTAs along K per output tile (gridDim.z): a cluster
   int kc_per_split;       // 128-k tiles per split
-  float* partial;         // [splits][m_total][n_rows] f32, only when splits > 1
-  int* counters;          // one per output tile, zero between launches
+  int y_vec4;             // four values of a row of y are stored at once
   const int* g_counts;    // grouped launches (experts stacked by rows): rows of x / y per group, or null
   const int* g_offsets;   // first row of each group
   const int* g_active;    // optional list of group ids with rows (-1 = unused entry); blockIdx.z indexes it
@@ -85,7 +84,7 @@ struct UmmaGroups {
 };
 
 __host__ __device__ inline size_t umma_stage_bytes(int ntok) { return (size_t)ntok * 128; }   // an activation box
-constexpr int kUmmaMaxRawStages = 16, kUmmaMaxStages = 8;
+constexpr int kUmmaMaxRawStages = 16, kUmmaMaxStages = 8, kUmmaMaxSplits = 8;
 constexpr int kUmmaHeader = 1024;
 __host__ __device__ inline size_t umma_smem_bytes(int kind, int ntok, int stages, int raw_tiles) {
   return kUmmaHeader + 1024 /*alignment slack*/ + (size_t)stages * umma_stage_bytes(ntok) +
@@ -149,6 +148,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
 // D[tmem] (+)= A[tmem] * B[smem descriptor]: the A operand is read from tensor memory (lane = row, each 32-bit
 // column holds two consecutive k as bf16, eight columns per 16-k instruction).
