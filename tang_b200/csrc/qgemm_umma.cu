@@ -49,25 +49,26 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   // every stage with the first tile's activations, warp 3 with the second tile's, each into one accumulator
   static_assert(!DUAL || TERMS == 1, "two token tiles per CTA: single-term weights");
   constexpr int kTokTiles = DUAL ? 2 : 1;
-  constexpr int kMaxStages = kUmmaMaxStages;
   // ---- shared-memory carve-up (operand tiles need 1024-byte alignment for the 128-byte swizzle)
   uint8_t* smem = smem_raw;
-  uint64_t* x_full = reinterpret_cast<uint64_t*>(smem);       // [stages] activation box landed
-  uint64_t* a_full = x_full + kMaxStages;                      // [stages] A tiles written (one arrival per dequant warp)
-  uint64_t* empty = a_full + kMaxStages;                       // [stages] MMAs of the stage retired
-  uint64_t* raw_full = empty + kMaxStages;                     // [raw stages] packed tiles landed
+  uint64_t* x_full = reinterpret_cast<uint64_t*>(smem);       // [x slots] activation boxes landed
+  uint64_t* x_empty = x_full + kUmmaMaxXSlots;                 // [x slots] MMAs that read them retired (one commit per issuer that does)
+  uint64_t* a_full = x_empty + kUmmaMaxXSlots;                 // [stages] weights written (one arrival per dequant warp)
+  uint64_t* empty = a_full + kUmmaMaxStages;                   // [stages] MMAs of the stage retired (two token tiles: x_empty of its second box)
+  uint64_t* raw_full = empty + kUmmaMaxStages;                 // [raw stages] packed tiles landed
   uint64_t* raw_empty = raw_full + kUmmaMaxRawStages;             // [raw stages] packed tiles consumed (one arrival per dequant warp)
   uint64_t* acc_full = raw_empty + kUmmaMaxRawStages;             // accumulator complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t base_u32 = smem_u32(smem_raw);
   uint8_t* tiles_s = smem_raw + kUmmaHeader + ((1024 - ((base_u32 + kUmmaHeader) & 1023)) & 1023);  // 1024-aligned
-  const size_t stage_bytes = umma_stage_bytes(p.ntok) * kTokTiles;
+  const int KX = DUAL ? 1 : p.kx;                              // 64-k steps per activation slot
+  const size_t x_bytes = umma_box_bytes(p.ntok) * kTokTiles * KX;
   float* part_s = reinterpret_cast<float*>(tiles_s);            // K split: this CTA's partial sums, when the rings are done with
-  uint8_t* raw_s = tiles_s + (size_t)p.stages * stage_bytes;   // [raw stages][8 tiles]
+  uint8_t* raw_s = tiles_s + (size_t)p.x_slots * x_bytes;   // [raw stages][8 tiles]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int S = p.stages, RS = p.raw_stages, KT = p.kt;
+  const int S = p.stages, XS = p.x_slots, RS = p.raw_stages, KT = p.kt;
   // The eight 16-row blocks of this CTA come in two boxes of four: neighbours, or (swiglu 2) gate blocks and their up blocks
   int rb_first = (int)blockIdx.x * (p.swiglu == 2 ? 4 : 8);
   const int rb_away = p.swiglu == 2 ? p.n_rows / (2 * kTileRows) : 4;
@@ -92,13 +93,15 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   }
   const int kc_begin = p.g_counts ? 0 : blockIdx.z * p.kc_per_split;   // this CTA's slice of K, in 128-k tiles
   const int kc_len = min(p.kc_per_split, p.kc_total - kc_begin);
-  const int n_kb = kc_len * 2;                                 // 64-k steps
 
   if (warp == 0) {
-    if (lane < S) {
+    if (lane < XS) {
       mbar_init(&x_full[lane], 1);
+      mbar_init(&x_empty[lane], p.kx == 2 ? 1 : 2);
+    }
+    if (lane < S) {
       mbar_init(&a_full[lane], kUmmaGroupWarps);
-      mbar_init(&empty[lane], DUAL ? 2 : 1);   // one commit per issuer that reads the stage
+      mbar_init(&empty[lane], 1);
     }
     if (lane < RS) {
       mbar_init(&raw_full[lane], 1);
@@ -150,91 +153,104 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     }
   } else if (warp == 2) {
     // ------------------------------------------------------------------ activation producer
+    // Waiting for a slot, announcing the bytes and issuing one copy takes this thread 330 to 450 cycles, which is more than a step of
+    // few tokens: a copy brings KX boxes of 64 k.
     if (lane == 0) {
       pdl_wait();
       int s = 0;
-      uint32_t ph = 0;
-      for (int kb = 0; kb < n_kb && !*failed; ++kb) {
-        if (!mbar_wait_spin(&empty[s], ph ^ 1u)) { give_up(DERR_EMPTY_WAIT); break; }
-        mbar_arrive_expect_tx(&x_full[s], (uint32_t)(p.ntok * kTokTiles) * 128u);
-        tma_load_2d(tiles_s + (size_t)s * stage_bytes, &x_map,
-                    (kc_begin * 2 + kb) * kUmmaK, m0, &x_full[s]);
-        if constexpr (DUAL)     // (rows beyond the matrix read as zeros, a box entirely beyond it too)
-          tma_load_2d(tiles_s + (size_t)s * stage_bytes + (size_t)p.ntok * 128, &x_map, (kc_begin * 2 + kb) * kUmmaK,
-                      m0 + p.ntok, &x_full[s]);
-        if (++s == S) {
+      uint32_t ph = 0, tok = 1;
+      for (int kb = 0; kb < 2 * kc_len; kb += KX) {
+        if (!mbar_wait_token(&x_empty[s], ph ^ 1u, tok)) { give_up(DERR_EMPTY_WAIT); break; }
+        mbar_arrive_expect_tx(&x_full[s], (uint32_t)(p.ntok * kTokTiles * KX) * 128u);
+        uint8_t* slot = tiles_s + (size_t)s * x_bytes;
+        // (rows and k beyond the matrix read as zeros, a box entirely beyond it too)
+        tma_load_3d(slot, &x_map, 0, m0, kc_begin * 2 + kb, &x_full[s]);
+        if constexpr (DUAL) tma_load_3d(slot + (size_t)p.ntok * 128, &x_map, 0, m0 + p.ntok, kc_begin * 2 + kb, &x_full[s]);
+        if (++s == XS) {
           s = 0;
           ph ^= 1u;
+          if (*failed) break;
         }
+        tok = mbar_test(&x_empty[s], ph ^ 1u);
       }
     }
   } else if (warp == 1 || warp == 3) {
     // ------------------------------------------------------------------ MMA issuers
-    // Two of them: issuing one step's MMAs from a single thread (~55 cycles each, plus the waits and the
-    // commit) is what bounds the step time, so warp 1 takes the even steps into the even accumulators and warp 3
-    // the odd steps into the odd ones; the epilogue adds them all (a fixed order: reproducible).  With an
-    // even ring depth each issuer only ever returns to slots it consumed itself.
-    // The whole warp runs the loop (warp-uniform control flow keeps the descriptors in uniform
-    // registers); one elected lane issues.  The barriers of the NEXT step are looked at before this
-    // step's instructions are issued, so that the answer is there when the loop comes round.
+    // Two of them: a chunk of 128 k takes an issuer's thread its MMAs (~45 cycles each) and several hundred cycles for waits and
+    // commits, so warp 1 takes the even chunks into the even accumulators and warp 3 the odd chunks into the odd ones; the
+    // epilogue adds them all (a fixed order: reproducible).  With even rings an issuer returns to stages that it consumed itself.
+    // The whole warp runs the loop (warp-uniform control flow keeps the descriptors in uniform registers); one elected lane issues.
     const bool leader = elect_one();
     const uint32_t idesc = umma_idesc_bf16(p.ntok);
-    const uint64_t desc0 = umma_desc_sw128(tiles_s);
-    const uint32_t stage_u = (uint32_t)(stage_bytes >> 4);
-    bool ok = true;
     const int odd = warp == 3;
+    const uint32_t box_u = (uint32_t)((p.ntok * 128) >> 4), slot_u = (uint32_t)(x_bytes >> 4);
+    // slots of four boxes serve a chunk of either issuer, slots of two one chunk; with two token tiles (a box of each per slot) a
+    // chunk takes two slots and every issuer every chunk
+    const uint64_t desc0 = umma_desc_sw128(tiles_s) + (DUAL ? (uint32_t)odd * box_u : KX == 4 ? 2u * odd * box_u : 0u);
+    const uint32_t half_u = DUAL ? slot_u : box_u;
     // Each issuer rotates over n_acc / 2 accumulators: the tensor core truncates every f32 addition, an error that
     // grows with the number of additions one accumulator sees, so as many short sums as tensor memory holds
     // (512 columns) are kept and the epilogue adds them, in accumulator order.
     const int rot_mask = (p.n_acc >> 1) - 1;
-    int j = 0;                                  // this issuer's step count
-    constexpr int kStep = DUAL ? 1 : 2;         // (two token tiles: every issuer takes every step)
-    int s = DUAL ? 0 : odd;
-    uint32_t ph = 0;
-    uint32_t tok_x = mbar_test(&x_full[s], 0), tok_a = mbar_test(&a_full[s], 0);
-    const uint32_t tile_off_u = DUAL ? (uint32_t)odd * (uint32_t)((p.ntok * 128) >> 4) : 0u;
+    int j = 0;                                  // this issuer's 64-k steps
+    constexpr int kStep = DUAL ? 1 : 2;
+    const int x_step = KX == 4 ? 1 : 2;
+    int s = DUAL ? 0 : odd, xs = DUAL || KX == 4 ? 0 : odd;     // stage of weights; activation slot
+    uint32_t ph = 0, xph = 0, tok_a = 0;
 #pragma unroll 1
-    for (int kb = DUAL ? 0 : odd; kb < n_kb; kb += kStep) {
-      ok = !*failed && mbar_wait_token(&x_full[s], ph, tok_x) && mbar_wait_token(&a_full[s], ph, tok_a);
+    for (int ck = DUAL ? 0 : odd; ck < kc_len; ck += kStep) {
+      bool ok = mbar_wait_token(&a_full[s], ph, tok_a) && mbar_wait_spin(&x_full[xs], xph);
       if (!ok) { give_up(DERR_FULL_WAIT); break; }
       tc_fence_after();
-      const uint64_t ad = desc0 + (uint64_t)((uint32_t)s * stage_u);
-      const int s_cur = s;
+      const uint64_t xd = desc0 + (uint64_t)((uint32_t)xs * slot_u);
+      const uint32_t a_t0 = tmem_d + (uint32_t)(p.a_col0 + s * (64 * TERMS));
+#pragma unroll
+      for (int half = 0; half < 2; ++half, ++j) {
+        if (DUAL && half == 1) {
+          ok = mbar_wait_spin(&x_full[xs + 1], xph);
+          if (!ok) { give_up(DERR_FULL_WAIT); break; }
+        }
+        const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride);
+        const uint32_t fresh = (DUAL ? j == 0 : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
+        if (leader) {
+#pragma unroll
+          for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
+            const uint64_t bd = xd + half * half_u + 2 * k16;
+            // 32 columns (64 k) of the hi term, then 32 of the lo term
+            const uint32_t a_t = a_t0 + (uint32_t)(half * (32 * TERMS) + 8 * k16);
+            umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
+            if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
+          }
+          // (commits arrive when the MMAs so far have finished reading)
+          if (DUAL) umma_commit(&x_empty[xs + half]);
+        }
+      }
+      if (!ok) break;
+      if (!DUAL && leader) {
+        umma_commit(&empty[s]);
+        umma_commit(&x_empty[xs]);
+      }
+      __syncwarp();
+      xs += x_step;
+      if (xs >= XS) {
+        xs -= XS;
+        xph ^= 1u;
+      }
       s += kStep;
       if (s >= S) {
         s -= S;
         ph ^= 1u;
       }
-      const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride);
-      const uint32_t fresh = (DUAL ? j == 0 : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
-      ++j;
-      if (leader) {
-#pragma unroll
-        for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
-          const uint64_t bd = ad + tile_off_u + 2 * k16;
-          // the stage's weights sit in tensor memory: 32 columns (64 k) of the hi term, then 32 of the lo term
-          const uint32_t a_t = tmem_d + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS) + 8 * k16);
-          umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
-          if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
-        }
-      }
-      if (leader) umma_commit(&empty[s_cur]);   // arrives when the MMAs above have finished reading the stage
-      __syncwarp();
-      // Look at the next step's barriers only now: the answer takes ~70 cycles, during which an in-order
-      // thread issues nothing, and here the tensor core already has this step's work.
-      tok_x = mbar_test(&x_full[s], ph);
+      // Look at the next chunk's barrier only now: the answer takes ~70 cycles, during which an in-order
+      // thread issues nothing, and here the tensor core already has this chunk's work.
       tok_a = mbar_test(&a_full[s], ph);
     }
     if (leader) umma_commit(acc_full);           // arrives when every MMA issued so far has completed
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ dequant warps
-    // Everything that does not change from step to step (which words of the packed tiles this thread
-    // converts, where their scales sit, where the result goes in the swizzled A tile) is computed once.
-    // The dequant warps form kUmmaGroups groups; group g produces the stages kb = g, g + G, g + 2G, ...
-    // so that G stages are being converted at any time (one stage's chain of waits, loads, arithmetic,
-    // stores and fence is long; the groups overlap it).  G is even, so a group always reads the same
-    // half (c = g & 1) of its 128-k packed tiles.
+    // Two groups of eight warps convert every second chunk of 128 k, four warps of a group (one per lane quarter of tensor memory) its
+    // first 64 k, four the second: one chunk's chain of waits, loads, arithmetic, stores and fence is long, and the groups overlap it.
     const int group = (warp - kUmmaFirstDqWarp) / kUmmaGroupWarps;
     // This thread owns output row 32 * (warp % 4) + lane, i.e. that lane of tensor memory: row g + 8 h of tile rbi of the slot.  In
     // a tile the row's nibbles are 64 contiguous bytes (its four k quarters of 16 bytes, each holding one word per 32-block), its
@@ -243,31 +259,29 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     const int q4 = warp & 3;
     const int rbi = p.swiglu == 2 ? (lane >> 4) * 4 + q4 : 2 * q4 + (lane >> 4), h = (lane >> 3) & 1, g = lane & 7;
     bool ok = true;
-    const int c = group & 1;                                    // which 64-k half of the 128-k tile
-    int s = group, r = 0, within = group >> 1;                   // A/B slot; packed-tile slot and the tile inside it
+    const int c = ((warp - kUmmaFirstDqWarp) >> 2) & 1;          // which 64-k half of the chunk
+    int s = group, r = 0, within = group;                        // stage; packed-tile slot and the tile inside it (KT is 2 or 4)
     uint32_t ph = 0, rph = 0;
-    while (s >= S) {
-      s -= S;
-      ph ^= 1u;
-    }
-    uint32_t tok_raw = mbar_test(&raw_full[r], rph), tok_empty = mbar_test(&empty[s], ph ^ 1u);
+    uint64_t* const stage_empty = DUAL ? x_empty + 1 : empty;
+    constexpr int kEmptyStep = DUAL ? 2 : 1;
+    uint32_t tok_raw = 0, tok_empty = 1;                         // (what is free is free at first)
 #pragma unroll 1
-    for (int kb = group; kb < n_kb && ok; kb += kUmmaGroups) {
+    for (int ck = group; ck < kc_len; ck += kUmmaGroups) {
       // (with two terms the stage is only waited for when the first half of the row is converted:
       // the MMAs that last read it have that long to finish -- decode step at batch 64 8.27 -> 8.11 ms; with one term
       // the conversion is too short for that and the early wait measured 3 % better)
       constexpr bool kLateWait = TERMS == 2;
-      ok = !*failed && mbar_wait_token(&raw_full[r], rph, tok_raw) && (kLateWait || mbar_wait_token(&empty[s], ph ^ 1u, tok_empty));
+      ok = mbar_wait_token(&raw_full[r], rph, tok_raw) && (kLateWait || mbar_wait_token(&stage_empty[s * kEmptyStep], ph ^ 1u, tok_empty));
       if (!ok) { give_up(DERR_FULL_WAIT); break; }
       const int s_cur = s, r_cur = r, within_cur = within;
       const uint32_t ph_cur = ph;
       s += kUmmaGroups;
-      while (s >= S) {
+      if (s >= S) {
         s -= S;
         ph ^= 1u;
       }
-      within += kUmmaGroups / 2;                  // this group's next tile: two further on
-      const bool leaves = within >= KT;           // ... which lies in the next ring slot (KT is 2 or 4)
+      within += kUmmaGroups;
+      const bool leaves = within >= KT;           // this group's next tile lies in the next ring slot
       if (leaves) {
         within -= KT;
         if (++r == RS) {
@@ -281,7 +295,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       const int line = tile_line + (kIs8 ? 8 * h + 4 * c : 4 * h) + (g >> 1);
       const uint8_t* wrow = slot + line * 128 + (kIs8 ? 0 : 8 * c);
       const int chunk0 = ((g & 1) * 4) ^ (line & 7);
-      const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (32 * TERMS));
+      const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (64 * TERMS) + c * (32 * TERMS));
       uint32_t sh = 0, sl = 0;
       if constexpr (KIND != I8_ROW) {
         // Two terms of Q4 with f16 scales: s_hi = the scale rounded to five significant bits and s_lo = the rest, which has
@@ -355,7 +369,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         }
         if (kLateWait && jj == 0) {
           // the stage's columns were last read by MMAs whose commit is waited for here
-          ok = __all_sync(0xffffffffu, mbar_wait_token(&empty[s_cur], ph_cur ^ 1u, tok_empty));
+          ok = __all_sync(0xffffffffu, mbar_wait_token(&stage_empty[s_cur * kEmptyStep], ph_cur ^ 1u, tok_empty));
           tc_fence_after();
         }
         if (ok) {
@@ -371,9 +385,9 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         mbar_arrive(&a_full[s_cur]);
         if (leaves) mbar_arrive(&raw_empty[r_cur]);   // done with this ring slot (nobody waits for the final ones)
       }
-      if (kb + kUmmaGroups < n_kb) {                 // early look at what this group's next stage waits for
+      if (ck + kUmmaGroups < kc_len) {               // early look at what this group's next stage waits for
         tok_raw = leaves ? mbar_test(&raw_full[r], rph) : 1u;
-        tok_empty = mbar_test(&empty[s], ph ^ 1u);
+        tok_empty = mbar_test(&stage_empty[s * kEmptyStep], ph ^ 1u);
       }
     }
     // ---- epilogue: D[128 features x ntok tokens] -> y[token][feature]
@@ -388,8 +402,9 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         float v[16], v1[16];
         tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tile * p.acc_stride + c0), v);
         const int mt = m0 + tile * p.ntok;                // first token of the tile
-        const int used = DUAL ? 1 : min(p.n_acc, n_kb);   // step kb < n_acc is the first to touch accumulator kb
-        for (int a = 1; a < used; ++a) {
+        // (accumulator a: issuer a & 1's number a >> 1, which that issuer has reached if it had that many steps)
+        for (int a = 1; a < (DUAL ? 1 : p.n_acc); ++a) {
+          if ((a >> 1) >= 2 * ((kc_len + 1 - (a & 1)) >> 1)) continue;
           tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(a * p.acc_stride + c0), v1);
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] += v1[i];
@@ -490,11 +505,11 @@ bool umma_supported(const tq_qweight* w, size_t m) {
 
 // Fewer output tiles than this leave SMs idle, and K is split.
 static bool umma_few_tiles(const tq_ctx* ctx, long long ctas) { return ctas < (ctx->sm_count * 3) / 4; }
-constexpr int kUmmaTwoTermTokens = 128;   // token tile of two-term products: what tensor memory leaves beside the weights
+constexpr int kUmmaTokens = 128;   // token tile: what tensor memory leaves beside the weights
 
 // Whether two-term products of m rows run without a split of K.
 bool umma_fills_gpu(const tq_ctx* ctx, const tq_qweight* w, size_t m) {
-  return !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)((m + kUmmaTwoTermTokens - 1) / kUmmaTwoTermTokens));
+  return !umma_few_tiles(ctx, (long long)(w->rows / kUmmaRows) * (long long)((m + kUmmaTokens - 1) / kUmmaTokens));
 }
 
 // How many clusters of `size` CTAs of this kernel the GPU holds at once (a CTA has an SM to itself, whatever its shared memory).
@@ -531,22 +546,20 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   if (!encode_tiled()) return fail(ctx, TQ_EUNSUPPORTED, "cuTensorMapEncodeTiled is not available from this driver");
   TQ_REQUIRE(ctx, umma_supported(w, m), "tcgen05 GEMM: needs rows %% 128 == 0 and cols %% 128 == 0");
   TQ_REQUIRE(ctx, ((uintptr_t)x_bf16 & 15) == 0 && (ldx * 2) % 16 == 0, "tcgen05 GEMM: activation rows must be 16-byte aligned");
-  // Ring sizes.  Two rules come from the dequant groups running ahead of one another (a parity wait
-  // is only sound when the waiter is at most one phase ahead of the barrier): at least kUmmaGroups
-  // stages, and an even number of packed-tile slots whenever slots are reused.  Four stages of weights take 32
-  // columns of tensor memory per term each; the rest holds the accumulators, two at least (one per issuing warp): token
-  // tiles up to 128 with two terms, up to 192 with one, evened out over the tiles.
+  // The dequantised weights are an operand in tensor memory: per chunk of 128 k and term 64 columns, four stages with one
+  // term, two with two terms, i.e. 256 columns; the other 256 hold accumulators, two at least (one per issuing warp): token tiles
+  // up to 128, evened out over the tiles.
   const size_t kSmemMax = 227 * 1024, raw_tile = 8 * (size_t)qk_tile_bytes(w->kind);
   const size_t budget = kSmemMax - kUmmaHeader - 1024;
-  const int ntok_max = terms == 2 ? kUmmaTwoTermTokens : 192;
+  const int ntok_max = kUmmaTokens;
   // Many rows, one term: a CTA takes TWO token tiles (each MMA issuer multiplies every stage with its own tile's
   // activations), so the weights are converted once per 2 x <= 192 tokens; the accumulators are 2 x 192 columns, the
-  // weights 128.  Only where that still gives about a wave of CTAs (no K split in this form).
+  // weights (two stages) 128.  Only where that still gives about a wave of CTAs (no K split in this form).
   bool dual = false;
   int dual_ntok = 0;
   size_t n_pairs = 0;
-  if (terms == 1 && !grp && m > 192) {
-    int cap = (int)(((budget - 4 * raw_tile) / kUmmaGroups) / 256) / 16 * 16;   // two activation boxes per stage
+  if (terms == 1 && !grp && m > kUmmaTokens) {
+    int cap = (int)(((budget - 4 * raw_tile) / kUmmaMaxXSlots) / 256) / 16 * 16;   // two activation boxes per slot
     if (cap > 192) cap = 192;
     if (cap >= 64) {
       n_pairs = (m + 2 * (size_t)cap - 1) / (2 * (size_t)cap);
@@ -580,38 +593,25 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   int acc_stride = 32;
   while (acc_stride < ntok) acc_stride <<= 1;
   if (ntok > 128) acc_stride = 192;
-  const int acc_cols = 512 - 128 * terms;
+  const int a_col0 = dual ? 384 : 256, stages = terms == 2 || dual ? 2 : 4;
   int n_acc = 2;                       // a power of two, as many as tensor memory holds beside the weights
-  while (!dual && n_acc < 16 && 2 * n_acc * acc_stride <= acc_cols) n_acc <<= 1;
-  // Four A/B stages are what the dequant groups need; everything else goes to the packed-tile ring, because
-  // the bytes in flight from HBM (ring slots not being read) are what hides its latency.  A ring slot holds
-  // KT = 4 k-tiles of the eight row blocks (two copies of 18 KB) when three such slots fit, else KT = 2.
-  int stages = kUmmaGroups;
-  // Two terms and up to 32 tokens: four accumulators take 128 columns, which leaves room for SIX stages of weights, so
-  // that a converting group need not wait for the MMAs of its own previous stage (decode step at 20 / 32 rows:
-  // 5.16 -> 5.06 ms / 5.82 -> 5.71 ms).
-  int a_col0 = acc_cols;
-  if (terms == 2 && acc_stride == 32) {
-    stages = 6;
-    n_acc = 4;
-    a_col0 = 128;
-  }
-  // One term and up to 64 tokens: eight stages (28672 x 4096 at 64 rows 45.2 -> 42.0 us).
-  if (terms == 1 && acc_stride <= 64) {
-    stages = 8;
-    a_col0 = 256;
-  }
-  if ((budget - 4 * raw_tile) / umma_stage_bytes(ntok_stage) < (size_t)stages)
-    return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: token tile of %d does not fit", ntok);
-  const size_t avail = budget - (size_t)stages * umma_stage_bytes(ntok_stage);
-  int kt = avail / (4 * raw_tile) >= 3 ? 4 : 2;
+  while (!dual && n_acc < 16 && 2 * n_acc * acc_stride <= a_col0) n_acc <<= 1;
+  // Shared memory: slots of activations (KX boxes of 64 k by one copy; one box with two token tiles), the rest packed tiles, whose bytes
+  // in flight hide the latency of HBM: ring slots of KT = 4 k-tiles where two such fit, else 2.
+  const int kx = dual ? 1 : ntok <= 64 ? 4 : 2;
+  int x_slots = kx == 4 && ntok > 32 ? 3 : 4;
+  if (kx == 4 && x_slots > (kc_per_split + 1) / 2) x_slots = (kc_per_split + 1) / 2;
+  if (kx == 2 && (kc_per_split <= 2 || budget < (size_t)x_slots * kx * umma_box_bytes(ntok_stage) + 8 * raw_tile)) x_slots = 2;   // (even: a slot is always the same issuer's)
+  const size_t x_ring = (size_t)x_slots * kx * umma_box_bytes(ntok_stage);
+  if (x_ring + 4 * raw_tile > budget) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: token tile of %d does not fit", ntok);
+  const size_t avail = budget - x_ring;
+  const int kt = avail / (4 * raw_tile) >= 2 ? 4 : 2;
   int raw_stages = (int)(avail / ((size_t)kt * raw_tile));
   if (raw_stages > kUmmaMaxRawStages) raw_stages = kUmmaMaxRawStages;
   const int slots_needed = (kc_per_split + kt - 1) / kt;
   if (raw_stages > slots_needed) raw_stages = slots_needed;
-  if (stages < kUmmaGroups || raw_stages < 1) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: ring sizes %d/%d", stages, raw_stages);
   CUtensorMap map;
-  if (!encode_bf16_k64(&map, x_bf16, m, w->cols, ldx, (unsigned)ntok)) return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
+  if (!encode_bf16_k64_blocks(&map, x_bf16, m, w->cols, ldx, (unsigned)ntok, (unsigned)kx)) return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
   CUtensorMap w_map;   // the packed tiles as 128-byte lines, boxes of kt tiles of four row blocks
   if (!encode_lines128(&w_map, w->tiles, (size_t)w->n_kc * (qk_tile_bytes(w->kind) / 128), (size_t)w->n_rb, (unsigned)(kt * (qk_tile_bytes(w->kind) / 128)), 4))
     return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -637,9 +637,11 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.kc_per_split = kc_per_split;
   p.y_vec4 = ldy % 4 == 0 && ((uintptr_t)y & (p.y_bf16 ? 7 : 15)) == 0;
   p.stages = stages;
+  p.x_slots = x_slots;
+  p.kx = kx;
   p.raw_stages = raw_stages;
   p.kt = kt;
-  const size_t smem = umma_smem_bytes(w->kind, ntok_stage, stages, raw_stages * kt);
+  const size_t smem = umma_smem_bytes(w->kind, x_ring, raw_stages * kt);
   if (smem > kSmemMax) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
   dim3 grid((unsigned)(rows_g / kUmmaRows), (unsigned)((m + ntok_stage - 1) / ntok_stage), (unsigned)splits);
   if (grp) {

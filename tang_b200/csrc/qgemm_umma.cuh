@@ -6,26 +6,23 @@
 //
 // Operand roles are swapped so that any token count fits one instruction shape: the 128 output
 // features of a CTA are the UMMA M dimension (A operand, the dequantised weights), the tokens are
-// the UMMA N dimension (B operand, 16..256), and the f32 accumulator D[128 x tokens] lives in
-// tensor memory.  Per 64-k step:
-//   * warp 0 streams the packed fragment tiles (1-D bulk copies), warp 2 the activation boxes
-//     (cp.async.bulk.tensor, 128-byte swizzle, out-of-range token rows filled with zeros), each as
+// the UMMA N dimension (B operand, 16..192), and the f32 accumulators D[128 x tokens] live in
+// tensor memory.  Per chunk of 128 k:
+//   * warp 0 streams the packed fragment tiles (tensor copies of 128-byte lines, swizzled so that the row-per-thread reads below
+//     hit all banks), warp 2 the activations (boxes of 64 k, 128-byte swizzle, out-of-range token rows filled with zeros), each as
 //     far ahead as its own ring allows;
-//   * sixteen dequant warps, in four groups that each take every fourth step, turn nibbles into bf16 A tiles in shared memory in the K-major
-//     128-byte-swizzled layout UMMA reads.  The product q*scale (15 significant bits) is split into
-//     hi = bf16(q*scale) and lo = bf16(q*scale - hi); hi + lo equals q*scale EXACTLY, so two MMAs
-//     per k-step reproduce exact products with f32 accumulation (TERMS = 2).  TERMS = 1 keeps only
-//     hi (relative weight error at most 2^-8), for bf16 outputs;
-//   * one elected lane of warp 1 (even steps) and of warp 3 (odd steps) issues tcgen05.mma (kind::f16,
-//     bf16 x bf16 -> f32), each into an accumulator of its own, and commits each stage back to the
-//     producers;
-//   * the dequant warps finally read both accumulators with tcgen05.ld, add them and store y.
-// Tensor-memory operand (UmmaParams::ts, every launch whose token tile allows it): the A tiles do not go through
-// shared memory at all.  A dequant thread owns one output row = one tensor-memory lane (in a fragment tile the row's
-// nibbles are 64 contiguous bytes), converts the row's 64 k of the stage and writes them with tcgen05.st (32 columns
-// per term and stage); the MMA takes A from tensor memory and only the activation box from shared memory.  Writing
-// 32 KB of A tiles per step and reading them back was what bound the step time (14336 x 4096 at 64 rows, f32
-// results: the decode step at batch 64 went from 9.55 to 8.26 ms; 4096^2 Q8 blocks at 2048 rows 386 -> 130 us).
+//   * sixteen dequant warps, in two groups that each take every second chunk, turn the packed integers into bf16.  A thread owns one
+//     output row = one tensor-memory lane and 64 k (a row's nibbles are 64 contiguous bytes of a tile) and writes them with
+//     tcgen05.st.  The product q*scale (15 significant bits) is split into two bf16 numbers whose sum equals it EXACTLY, so two MMAs
+//     per k-step reproduce exact products with f32 accumulation (TERMS = 2).  TERMS = 1 keeps the product
+//     rounded to bf16 (relative weight error at most 2^-8), for bf16 outputs;
+//   * one elected lane of warp 1 (even chunks) and of warp 3 (odd chunks) issues tcgen05.mma (kind::f16,
+//     bf16 x bf16 -> f32; A from tensor memory), each into accumulators of its own, and commits each stage back to the producers;
+//   * the dequant warps finally read the accumulators with tcgen05.ld, add them and store y.
+// What bounds it, found with cycle counters: up to 64 rows first the threads that issue (a tensor copy 330 to 450 cycles with its wait and
+// its announcement; an MMA issuer's turn 700 beside the MMAs), hence copies of 256 k of activations and turns of 128 k; then the
+// conversion (1200 cycles of a group's 1640 per chunk, ALU and FMA pipes 60 % busy).  us per launch, chunks of 64 k -> as it is:
+// 28672 x 4096 at 64 rows 42.0 -> 34.7, 4096 x 14336 22.8 -> 20.4, int8 7168 x 16384 44.7 -> 35.7, 1024 x 4096 at 1024 rows 19.7 -> 16.3.
 // Every mbarrier wait is bounded; on failure the CTA records a code, skips ahead and still frees its
 // tensor memory.
 #pragma once
@@ -38,9 +35,9 @@
 namespace tq {
 
 constexpr int kUmmaRows = 128;        // output features per CTA
-constexpr int kUmmaK = 64;            // k per stage (one 128-byte swizzle span of bf16)
-constexpr int kUmmaGroups = 4;        // dequant groups, each converting every fourth 64-k stage (even)
-constexpr int kUmmaGroupWarps = 4;    // warps per group
+constexpr int kUmmaK = 64;            // k of an activation box (one 128-byte swizzle span of bf16)
+constexpr int kUmmaGroups = 2;        // dequant groups, each converting every second 128-k chunk
+constexpr int kUmmaGroupWarps = 8;    // warps per group
 constexpr int kUmmaDqWarps = kUmmaGroups * kUmmaGroupWarps;   // dequant / epilogue warps
 constexpr int kUmmaFirstDqWarp = 4;   // warps 0..3: weight producer, MMA issuer (even steps), activation producer, MMA issuer (odd steps)
 constexpr int kUmmaThreads = 32 * (kUmmaFirstDqWarp + kUmmaDqWarps);
@@ -54,9 +51,10 @@ struct UmmaParams {
   int kc_total;           // K / 128
   int ntok;               // tokens per CTA tile = UMMA N (multiple of 16, <= 256)
   int acc_stride;         // columns between accumulators
-  int a_col0;             // tensor-memory columns of the converted weights: stages x terms x 32 from here on
-  int n_acc;              // accumulators (2, 4, 8 or 16): step kb adds into number (kb & 1) + 2 * ((kb >> 1) % (n_acc / 2))
-  int stages;             // A/B ring depth
+  int a_col0;             // tensor-memory columns of the converted weights: stages x 2 x terms x 32 from here on
+  int n_acc;              // accumulators (2, 4 or 8): 64-k step j of issuer i adds into number i + 2 * (j % (n_acc / 2))
+  int stages;             // stages of converted weights in tensor memory (128 k each; even)
+  int x_slots, kx;        // slots of activations in shared memory, 64-k boxes per slot (4; more than 64 tokens 2, two token tiles 1)
   int raw_stages;         // packed-tile ring depth (slots of kt tiles of 128 k): what keeps the HBM stream in flight
   int kt;                 // k-tiles per ring slot (2 or 4)
   int y_bf16;
@@ -83,11 +81,11 @@ struct UmmaGroups {
   int expected_rows = 0;   // typical counts[e]: sets the token tile
 };
 
-__host__ __device__ inline size_t umma_stage_bytes(int ntok) { return (size_t)ntok * 128; }   // an activation box
-constexpr int kUmmaMaxRawStages = 16, kUmmaMaxStages = 8, kUmmaMaxSplits = 8;
+__host__ __device__ inline size_t umma_box_bytes(int ntok) { return (size_t)ntok * 128; }   // 64 k of a token tile's activations
+constexpr int kUmmaMaxRawStages = 16, kUmmaMaxStages = 4, kUmmaMaxXSlots = 4, kUmmaMaxSplits = 8;
 constexpr int kUmmaHeader = 1024;
-__host__ __device__ inline size_t umma_smem_bytes(int kind, int ntok, int stages, int raw_tiles) {
-  return kUmmaHeader + 1024 /*alignment slack*/ + (size_t)stages * umma_stage_bytes(ntok) +
+__host__ __device__ inline size_t umma_smem_bytes(int kind, size_t x_ring, int raw_tiles) {
+  return kUmmaHeader + 1024 /*alignment slack*/ + x_ring +
          (size_t)raw_tiles * 8 * qk_tile_bytes(kind);
 }
 
@@ -97,6 +95,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
           smem_u32(dst)),
       "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
       : "memory");
 }
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar, uint64_t policy) {

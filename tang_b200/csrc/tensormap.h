@@ -38,6 +38,19 @@ inline bool encode_bf16_k64(CUtensorMap* map, const void* base, size_t rows, siz
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same matrix, boxes of `box_blocks` neighbouring blocks of 64 columns, one behind the other in shared memory.  cols: a multiple of 64.
+inline bool encode_bf16_k64_blocks(CUtensorMap* map, const void* base, size_t rows, size_t cols, size_t ld, unsigned box_rows, unsigned box_blocks) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t gdim[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  const cuuint64_t gstride[2] = {(cuuint64_t)ld * 2, 128};
+  const cuuint32_t box[3] = {64, box_rows, box_blocks};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Bytes [blocks][lines][128], boxes of `box_lines` lines of `box_blocks` blocks in the 128-byte swizzle (16-byte chunk c of line l
 // of a 1024-byte aligned destination lands at chunk c ^ (l & 7)); lines behind a block's last read as zeros.
 inline bool encode_lines128(CUtensorMap* map, const void* base, size_t lines, size_t blocks, unsigned box_lines, unsigned box_blocks) {

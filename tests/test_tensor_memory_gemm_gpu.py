@@ -1,0 +1,72 @@
+"""Edges of the tcgen05 dequant-GEMM (tang_b200/csrc/qgemm_umma.cu) against f64 products of the oracle's dequantised weights: token tiles of
+one, two and four boxes, odd numbers of 128-k chunks, the split of K over clusters, rows of the result that are not 16-byte aligned.
+
+f32 results with f16 scales or a row scale are exact products, so the error is that of the f32 sums: the tensor core truncates, at most
+2^-23 of the sum of magnitudes per 16-k addition; K = 3200 in two accumulators has 200 additions, 2.4e-5 of the output's rms times the ratio
+of the sum of magnitudes to it, which grows with the root of K, about 50: 1.2e-3 at worst, and a twentieth of that (additions of random sign to
+partial sums that are smaller than the last) is what is asked for here.  f32 block scales keep 16 bits (2^-15 a product, 1e-4 after the sum)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from util import bf16_round, make_weight
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    import tang_b200
+
+    d = tang_b200.QuantComputeDevice(0)
+    yield d
+    d.close()
+
+
+def weights64(orc, kind, sc, pay, rows, cols):
+    if kind == 3:
+        return pay.astype(np.float64) * sc[:, None]
+    q = (orc.unpack_q4(pay) if kind < 2 else pay).reshape(rows, cols // 32, 32).astype(np.float64)
+    s = (sc.view(np.float16) if kind == 1 else sc).astype(np.float64)
+    return (q * s[:, :, None]).reshape(rows, cols)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(128, 128), (128, 640), (256, 3200), (1152, 1408), (2304, 1024), (6144, 1536)])
+@pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 127, 128, 129, 192, 193, 300])
+def test_token_tiles_chunks_and_splits(dev, orc, kind, rows, cols, m):
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(rows + cols + m + kind)
+    sc, pay = make_weight(rng, kind, rows, cols)
+    w = dev.upload_qarrays(kind, pay, sc, rows, cols)
+    xbits, xf = bf16_round(rng.standard_normal((m, cols)).astype(np.float32))
+    want = xf.astype(np.float64) @ weights64(orc, kind, sc, pay, rows, cols).T
+    rms = np.sqrt(np.mean(want * want))
+    y = dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.F32).to_vec().reshape(m, rows)
+    assert np.abs(y - want).max() < (1e-4 if kind in (0, 2) else 6e-5) * rms
+    yb = (dev.qlinear(dev.upload(xbits, tb.BF16), w, m, tb.BF16).to_vec().reshape(m, rows).astype(np.uint32) << 16).view(np.float32)
+    # the result rounded to bf16 (2^-9) and, but for row scales, every weight too (2^-9 each, of random sign: 2^-9 of the rms times six sigma)
+    assert (np.abs(yb - want) < 2.0 ** -8 * np.abs(want) + 6 * 2.0 ** -9 * rms).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("rows,cols,m,ld", [(512, 2048, 40, 515), (512, 2048, 40, 516), (128, 512, 20, 131), (14336, 256, 33, 14337)])
+def test_result_rows_of_any_stride(dev, orc, dtype, rows, cols, m, ld):
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(ld)
+    sc, pay = make_weight(rng, 1, rows, cols)
+    w = dev.upload_qarrays(1, pay, sc, rows, cols)
+    x = dev.upload(bf16_round(rng.standard_normal((m, cols)).astype(np.float32))[0], tb.BF16)
+    dt = tb.F32 if dtype == "f32" else tb.BF16
+    dense = dev.qlinear(x, w, m, dt).to_vec().reshape(m, rows)
+    fill = np.full(m * ld + 1, 7, np.float32 if dtype == "f32" else np.uint16)
+    out = dev.upload(fill, dt)
+    at = out.ptr + fill.itemsize              # one element in: no vector of four is aligned with ld 516 either
+    dev._check(dev._L.tq_qlinear(dev._ctx, C.c_void_p(w.handle), C.c_void_p(x.ptr), x.dtype, 0, m, C.c_void_p(at), dt, ld, C.c_void_p(0)))
+    got = out.to_vec()[1:].reshape(m, ld)
+    dev.sync()
+    assert np.array_equal(got[:, :rows], dense)
+    assert (got[:, rows:] == 7).all() and out.to_vec()[0] == 7
