@@ -32,8 +32,8 @@ constexpr int kMaxTopK = 16;
 int all_to_all_v(tq_ctx* ctx, tq_comm* comm, const void* send_dev, const size_t* send_off, const size_t* send_bytes, void* recv_dev,
                  const size_t* recv_off, const size_t* recv_bytes);
 int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, size_t m_total,
-                              const int* counts, const int* offsets, const int* active, int max_active, int max_rows,
-                              int expected_rows, void* y, int y_dtype, size_t ldy, int terms = 2, int swiglu = 0);
+                              const int* counts, const int* offsets, int max_active, int expected_rows, void* y, int y_dtype, size_t ldy,
+                              int terms = 2, int swiglu = 0);
 struct UmmaGroups;
 bool umma_supported(const tq_qweight* w, size_t m);
 bool umma_fills_gpu(const tq_ctx* ctx, const tq_qweight* w, size_t m);
@@ -607,14 +607,14 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   if (tensor_path) {
     // silu(gate) * up in the projection's epilogue, from the same f32 sums (two terms per weight although the result is bf16): the
     // f32 round trip of the 2 f wide projection and its kernel are gone
-    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, n, cnt, offs, active, max_active, (int)T, (int)(expected * 3 / 2),
+    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, n, cnt, offs, max_active, (int)(expected * 3 / 2),
                                       act, TQ_BF16, f, 2, 2));
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_gate_up, nl, xs, d, cap, cnt, offs, (int)T, 0, 0, gu, TQ_F32, 2 * f, active, max_active, n));
     TQ_STEP(tq_swiglu(ctx, gu, gu + f, TQ_F32, 2 * f, n, f, act, TQ_BF16));
   }
   if (tensor_path) {
-    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_down, nl, act, f, n, cnt, offs, active, max_active, (int)T, (int)(expected * 3 / 2), yo,
+    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_down, nl, act, f, n, cnt, offs, max_active, (int)(expected * 3 / 2), yo,
                                       TQ_F32, d));
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_down, nl, act, f, cap, cnt, offs, (int)T, 0, 0, yo, TQ_F32, d, active, max_active, n));
@@ -757,14 +757,14 @@ int tq_moe_ffn_dispatch(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, floa
   const size_t expected = (size_t)W * n / (size_t)c.n_experts;      // rows per local expert when routing is even
   const bool tensor_path = expected >= 24 && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
   if (tensor_path) {
-    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, Rr, cnt, offs, active, max_active, max_rows, (int)(expected * 3 / 2),
+    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, Rr, cnt, offs, max_active, (int)(expected * 3 / 2),
                                       gu, TQ_F32, 2 * f));
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_gate_up, nl, xs, d, chunk, cnt, offs, max_rows, 0, 0, gu, TQ_F32, 2 * f, active, max_active, Rr));
   }
   TQ_STEP(tq_swiglu(ctx, gu, gu + f, TQ_F32, 2 * f, Rr, f, act, TQ_BF16));
   if (tensor_path) {
-    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_down, nl, act, f, Rr, cnt, offs, active, max_active, max_rows, (int)(expected * 3 / 2), yo,
+    TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_down, nl, act, f, Rr, cnt, offs, max_active, (int)(expected * 3 / 2), yo,
                                       TQ_F32, d));
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_down, nl, act, f, chunk, cnt, offs, max_rows, 0, 0, yo, TQ_F32, d, active, max_active, Rr));

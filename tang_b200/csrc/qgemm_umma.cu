@@ -75,19 +75,46 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   int m0 = blockIdx.y * p.ntok * kTokTiles;                    // first token of this CTA
   int m_end = p.m_total;                                       // rows at or beyond this are not this CTA's to store
   const float* row_scales = p.row_scales;   // TQ_I8_ROW: per output row, applied to the accumulator
+  int ntok = p.ntok;                                           // tokens of this CTA's tile: the MMA's N
   if (p.g_counts) {
-    // grouped (experts): blockIdx.z picks the group, whose rows are g_offsets[e] .. +g_counts[e] of x and y and
-    // whose weights start g_tile_stride bytes further on; token tiles beyond the group's rows leave at once
+    // Grouped (experts): the token tiles of all groups are numbered one group after the other, and blockIdx.y is such a number (the grid
+    // has as many as there can be; a place per group and possible tile, most of them empty, cost 64 experts at 4096 tokens
+    // 40,000 CTAs that left at once).  Group e's rows are g_offsets[e] .. +g_counts[e] of x and y, evened out over its tiles, its weights
+    // n_rows further on.
     pdl_wait();
-    int e = blockIdx.z;
-    if (p.g_active) {
-      e = p.g_active[e];
-      if (e < 0) return;
+    __shared__ int mine[3];
+    if (warp == 0) {
+      int before = 0, e = -1, tile = 0, tiles = 1;
+      for (int g0 = 0; g0 < p.n_groups && e < 0; g0 += 32) {
+        const int n = g0 + lane < p.n_groups ? (p.g_counts[g0 + lane] + p.ntok - 1) / p.ntok : 0;
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += u;
+        }
+        const unsigned behind = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.y);
+        if (behind) {
+          const int l = __ffs(behind) - 1;
+          e = g0 + l;
+          tiles = __shfl_sync(0xffffffffu, n, l);
+          tile = (int)blockIdx.y - (before + __shfl_sync(0xffffffffu, upto, l) - tiles);
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+      }
+      if (lane == 0) {
+        mine[0] = e;
+        mine[1] = tile;
+        mine[2] = tiles;
+      }
     }
+    __syncthreads();
+    const int e = mine[0];
+    if (e < 0) return;
     const int cnt = p.g_counts[e];
-    if (m0 >= cnt) return;
+    ntok = ((cnt + mine[2] - 1) / mine[2] + 15) & ~15;
+    m0 = p.g_offsets[e] + mine[1] * ntok;
     m_end = p.g_offsets[e] + cnt;
-    m0 += p.g_offsets[e];
     rb_first += e * (p.n_rows / kTileRows);
     row_scales += (size_t)e * p.n_rows;
   }
@@ -181,7 +208,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     // epilogue adds them all (a fixed order: reproducible).  With even rings an issuer returns to stages that it consumed itself.
     // The whole warp runs the loop (warp-uniform control flow keeps the descriptors in uniform registers); one elected lane issues.
     const bool leader = elect_one();
-    const uint32_t idesc = umma_idesc_bf16(p.ntok);
+    const uint32_t idesc = umma_idesc_bf16(ntok);
     const int odd = warp == 3;
     const uint32_t box_u = (uint32_t)((p.ntok * 128) >> 4), slot_u = (uint32_t)(x_bytes >> 4);
     // slots of four boxes serve a chunk of either issuer, slots of two one chunk; with two token tiles (a box of each per slot) a
@@ -398,7 +425,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       const int n = blockIdx.x * kUmmaRows + 32 * q4 + lane;
       // two warps share a lane quarter and alternate over the 16-column chunks
       for (int tile = 0; tile < kTokTiles; ++tile)
-      for (int c0 = 16 * ((warp - kUmmaFirstDqWarp) >> 2); c0 < p.ntok; c0 += 16 * (kUmmaDqWarps / 4)) {
+      for (int c0 = 16 * ((warp - kUmmaFirstDqWarp) >> 2); c0 < ntok; c0 += 16 * (kUmmaDqWarps / 4)) {
         float v[16], v1[16];
         tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tile * p.acc_stride + c0), v);
         const int mt = m0 + tile * p.ntok;                // first token of the tile
@@ -623,7 +650,7 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.n_rows = (int)rows_g;
   p.g_counts = grp ? grp->counts : nullptr;
   p.g_offsets = grp ? grp->offsets : nullptr;
-  p.g_active = grp ? grp->active : nullptr;
+  p.n_groups = grp ? grp->n_groups : 1;
   p.kc_total = w->n_kc;
   p.ntok = ntok;
   p.acc_stride = acc_stride;
@@ -645,8 +672,8 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   if (smem > kSmemMax) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
   dim3 grid((unsigned)(rows_g / kUmmaRows), (unsigned)((m + ntok_stage - 1) / ntok_stage), (unsigned)splits);
   if (grp) {
-    grid.y = (unsigned)((grp->max_rows + ntok - 1) / ntok);
-    grid.z = (unsigned)((grp->active && grp->max_active < grp->n_groups) ? grp->max_active : grp->n_groups);
+    grid.y = (unsigned)(m / ntok + (size_t)(grp->max_active < grp->n_groups ? grp->max_active : grp->n_groups));   // (a last tile per group with rows)
+    grid.z = 1;
   }
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -671,15 +698,13 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
 
 // Grouped entry for the other translation units: experts stacked by rows, rows of x / y grouped by expert.
 int launch_qgemm_umma_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const void* x_bf16, size_t ldx, size_t m_total,
-                              const int* counts, const int* offsets, const int* active, int max_active, int max_rows,
-                              int expected_rows, void* y, int y_dtype, size_t ldy, int terms, int swiglu) {
+                              const int* counts, const int* offsets, int max_active, int expected_rows,
+                              void* y, int y_dtype, size_t ldy, int terms, int swiglu) {
   UmmaGroups g;
   g.n_groups = n_groups;
   g.counts = counts;
   g.offsets = offsets;
-  g.active = active;
   g.max_active = max_active;
-  g.max_rows = max_rows;
   g.expected_rows = expected_rows;
   return launch_qgemm_umma(ctx, w, x_bf16, ldx, m_total, y, y_dtype, ldy, terms, &g, swiglu);
 }

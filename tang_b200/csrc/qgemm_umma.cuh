@@ -66,7 +66,7 @@ struct UmmaParams {
   int y_vec4;             // four values of a row of y are stored at once
   const int* g_counts;    // grouped launches (experts stacked by rows): rows of x / y per group, or null
   const int* g_offsets;   // first row of each group
-  const int* g_active;    // optional list of group ids with rows (-1 = unused entry); blockIdx.z indexes it
+  int n_groups;
   int* err;
 };
 
@@ -75,9 +75,7 @@ struct UmmaGroups {
   int n_groups = 1;
   const int* counts = nullptr;
   const int* offsets = nullptr;
-  const int* active = nullptr;
-  int max_active = 0;      // upper bound of groups with rows (sizes gridDim.z)
-  int max_rows = 0;        // upper bound of counts[e] (sizes gridDim.y)
+  int max_active = 0;      // upper bound of groups with rows
   int expected_rows = 0;   // typical counts[e]: sets the token tile
 };
 
