@@ -82,7 +82,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     // 40,000 CTAs that left at once).  Group e's rows are g_offsets[e] .. +g_counts[e] of x and y, evened out over its tiles, its weights
     // n_rows further on.
     pdl_wait();
-    __shared__ int mine[3];
+    int* mine = reinterpret_cast<int*>(smem_raw + kUmmaHeader) - 3;   // (the header's end; a static array would not fit beside the rings)
     if (warp == 0) {
       int before = 0, e = -1, tile = 0, tiles = 1;
       for (int g0 = 0; g0 < p.n_groups && e < 0; g0 += 32) {
@@ -555,7 +555,7 @@ static int umma_clusters(tq_ctx* ctx, int size) {
     attr[0].val.clusterDim.z = (unsigned)size;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024)) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = -1;
