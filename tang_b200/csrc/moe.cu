@@ -292,6 +292,211 @@ __global__ void __launch_bounds__(256, 4) router_kernel(const __nv_bfloat16* h, 
   }
 }
 
+// The same logits, selection and weights with the sums on the f64 tensor cores.  What bounds router_kernel is the conversion of every
+// product to f64 (16 a cycle and SM against 64 additions); here every operand is converted, once per 8 partners, and the products
+// are mma.m8n8k4 of f64: exact, and in any order the reference's bits wherever the certificate holds.  The certificate needs two numbers
+// per (token, expert): sum |p| from a bf16 mma.sync of the magnitudes, and a lower bound of the products' ulp exponent from the smallest codes
+// of runs of eight k (a product of the run is a multiple of 2 to the sum of both minima); a pair that fails with that is looked at
+// product by product, and then summed in the reference order (of normal values 7 and 2 of 10,000).
+// A CTA takes 16 tokens and 8 experts, its warps every eighth block of 32 k; the CTA of a token block that finishes last selects.
+// 64 experts, d 2048, us (router_kernel -> this): 1 token 27.4 -> 18.9, 64 31.5 -> 23.4, 1000 117 -> 50, 4096 355 -> 127, 16384 1219 -> 438.
+constexpr int kRtTok = 16, kRtExp = 8;
+__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+__device__ __forceinline__ unsigned short run_ulp_code(const uint4& v) {   // the smallest code of eight values
+  unsigned m = __vminu2(bf16x2_ulp_code(v.x), bf16x2_ulp_code(v.y));
+  m = __vminu2(m, __vminu2(bf16x2_ulp_code(v.z), bf16x2_ulp_code(v.w)));
+  return (unsigned short)min(m & 0xFFFFu, m >> 16);
+}
+
+__global__ void __launch_bounds__(256) router_mma_kernel(const __nv_bfloat16* h, const __nv_bfloat16* wg, int T, int d, int E, int top_k,
+                                                         int renorm, int* idx_out, float* w_out, double* logits, int* counters) {
+  extern __shared__ __align__(16) uint8_t rt_smem[];
+  const int n_blk = (d + 31) / 32, runs = 4 * n_blk;         // blocks of 32 k, runs of 8
+  double* part = reinterpret_cast<double*>(rt_smem);          // [warp][token][expert]
+  float* mags = reinterpret_cast<float*>(part + 8 * kRtTok * kRtExp);
+  unsigned short* ch = reinterpret_cast<unsigned short*>(mags + 8 * kRtTok * kRtExp);   // [token][runs]
+  unsigned short* cw = ch + kRtTok * runs;                    // [expert][runs]
+  const int t0 = blockIdx.x * kRtTok, e0 = blockIdx.y * kRtExp, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, q4 = lane & 3;
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(h);
+  const unsigned short* wp = reinterpret_cast<const unsigned short*>(wg);
+  double acc0[2] = {0.0, 0.0}, acc1[2] = {0.0, 0.0};          // tokens g, g + 8; experts 2 q4, 2 q4 + 1
+  float mag[4] = {0.f, 0.f, 0.f, 0.f};
+  // lane (g, q4) has k = 8 q4 .. + 7 of a block for token g, token g + 8 and expert g: k 8 q4 + i is row q4 of step i's k on both sides
+#pragma unroll 4
+  for (int b = warp; b < n_blk; b += 8) {
+    const int k = 32 * b + 8 * q4;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const bool in = k < d;                                    // (d is a multiple of 8)
+    const uint4 a0 = in && t0 + g < T ? *reinterpret_cast<const uint4*>(hp + (size_t)(t0 + g) * d + k) : zero;
+    const uint4 a1 = in && t0 + g + 8 < T ? *reinterpret_cast<const uint4*>(hp + (size_t)(t0 + g + 8) * d + k) : zero;
+    const uint4 bw = in && e0 + g < E ? *reinterpret_cast<const uint4*>(wp + (size_t)(e0 + g) * d + k) : zero;
+    const int run = 4 * b + q4;
+    ch[g * runs + run] = run_ulp_code(a0);
+    ch[(g + 8) * runs + run] = run_ulp_code(a1);
+    cw[g * runs + run] = run_ulp_code(bw);
+    const unsigned x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w}, y[4] = {bw.x, bw.y, bw.z, bw.w};
+    constexpr unsigned kAbs = 0x7FFF7FFFu;
+    mma_bf16_16816(mag, x0[0] & kAbs, x1[0] & kAbs, x0[1] & kAbs, x1[1] & kAbs, y[0] & kAbs, y[1] & kAbs);
+    mma_bf16_16816(mag, x0[2] & kAbs, x1[2] & kAbs, x0[3] & kAbs, x1[3] & kAbs, y[2] & kAbs, y[3] & kAbs);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double b0 = (double)__uint_as_float(y[j] << 16), b1 = (double)__uint_as_float(y[j] & 0xFFFF0000u);
+      dmma_884(acc0, (double)__uint_as_float(x0[j] << 16), b0);
+      dmma_884(acc1, (double)__uint_as_float(x1[j] << 16), b0);
+      dmma_884(acc0, (double)__uint_as_float(x0[j] & 0xFFFF0000u), b1);
+      dmma_884(acc1, (double)__uint_as_float(x1[j] & 0xFFFF0000u), b1);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int at = warp * kRtTok * kRtExp + g * kRtExp + 2 * q4 + i;
+    part[at] = acc0[i];
+    part[at + 8 * kRtExp] = acc1[i];
+    mags[at] = mag[i];
+    mags[at + 8 * kRtExp] = mag[2 + i];
+  }
+  __syncthreads();
+  // two threads per (token, expert): half of the runs each
+  {
+    const int pair = threadIdx.x >> 1, half = threadIdx.x & 1, tk = pair >> 3, ex = pair & 7;
+    unsigned q2 = 0xFFFFFFFFu;
+    const uint2* ph = reinterpret_cast<const uint2*>(ch + tk * runs);     // (runs is a multiple of four)
+    const uint2* pw = reinterpret_cast<const uint2*>(cw + ex * runs);
+    for (int i = half; i < runs / 4; i += 2) {
+      const uint2 u = ph[i], v = pw[i];
+      q2 = __viaddmin_u16x2(u.x, v.x, q2);
+      q2 = __viaddmin_u16x2(u.y, v.y, q2);
+    }
+    unsigned q = min(q2 & 0xFFFFu, q2 >> 16);
+    q = min(q, __shfl_xor_sync(0xffffffffu, q, 1));
+    double sum = 0.0;
+    float sabs = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      sum += part[w * kRtTok * kRtExp + pair];
+      sabs += mags[w * kRtTok * kRtExp + pair];
+    }
+    // (as router_kernel: a factor of two for the rounding of sabs; products below the normal range of f32 are not certified)
+    auto certain = [&](unsigned code) { return code >= 0x2000u || (code >= 140u && (double)sabs < ldexp(1.0, 52 + (int)code - 268)); };
+    const bool live = t0 + tk < T && e0 + ex < E;
+    unsigned open = __ballot_sync(0xffffffffu, live && half == 0 && !certain(q));
+    while (open) {                                            // the whole warp looks at one pair after the other
+      const int src = __ffs(open) - 1, p = (threadIdx.x - lane + src) >> 1;
+      open &= open - 1;
+      const unsigned short *hr = hp + (size_t)(t0 + (p >> 3)) * d, *wr = wp + (size_t)(e0 + (p & 7)) * d;
+      unsigned m2 = 0xFFFFFFFFu;
+#pragma unroll 4
+      for (int k = 8 * lane; k < d; k += 256) {
+        const uint4 u = *reinterpret_cast<const uint4*>(hr + k), v = *reinterpret_cast<const uint4*>(wr + k);
+        m2 = __viaddmin_u16x2(bf16x2_ulp_code(u.x), bf16x2_ulp_code(v.x), m2);
+        m2 = __viaddmin_u16x2(bf16x2_ulp_code(u.y), bf16x2_ulp_code(v.y), m2);
+        m2 = __viaddmin_u16x2(bf16x2_ulp_code(u.z), bf16x2_ulp_code(v.z), m2);
+        m2 = __viaddmin_u16x2(bf16x2_ulp_code(u.w), bf16x2_ulp_code(v.w), m2);
+      }
+      unsigned m = min(m2 & 0xFFFFu, m2 >> 16);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (!__shfl_sync(0xffffffffu, (int)certain(m), src)) {
+        const double s = router_ordered_sum(hr, wr, d, lane);
+        if (lane == src) sum = s;
+      }
+    }
+    if (live && half == 0) logits[(size_t)(t0 + tk) * E + e0 + ex] = sum;
+  }
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(&counters[blockIdx.x], 1) == (int)gridDim.y - 1;
+    if (last) counters[blockIdx.x] = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // selection, a warp per token: the rule is "highest logit first, lowest index on ties, exactly top_k" (see router_kernel)
+  double* ex = reinterpret_cast<double*>(rt_smem) + warp * kMaxExperts;
+  __syncthreads();
+  for (int tk = warp; tk < kRtTok && t0 + tk < T; tk += 8) {
+    const int t = t0 + tk;
+    double v[kMaxExperts / 32];
+    double mx = __ldcg(logits + (size_t)t * E);
+    bool nan = false;
+#pragma unroll
+    for (int j = 0; j < kMaxExperts / 32; ++j) {
+      const int i = lane + 32 * j;
+      if (i >= E) break;
+      v[j] = __ldcg(logits + (size_t)t * E + i);
+      mx = fmax(mx, v[j]);
+      nan |= v[j] != v[j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    nan = __any_sync(0xffffffffu, nan);
+    int pick[kMaxTopK];
+    if (!nan) {
+      unsigned taken = 0;
+#pragma unroll
+      for (int s = 0; s < kMaxTopK; ++s) {
+        if (s >= top_k) break;
+        double bv = 0.0;
+        int bi = -1;
+#pragma unroll
+        for (int j = 0; j < kMaxExperts / 32; ++j)
+          if (lane + 32 * j < E && !((taken >> j) & 1u) && (bi < 0 || v[j] > bv)) {
+            bv = v[j];
+            bi = lane + 32 * j;
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) {
+            bv = ov;
+            bi = oi;
+          }
+        }
+        if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
+        pick[s] = bi;
+      }
+    } else {                                                  // a NaN has no order: the comparison loop as written (every lane alike)
+      unsigned long long taken[kMaxExperts / 64] = {0, 0, 0, 0};
+#pragma unroll
+      for (int s = 0; s < kMaxTopK; ++s) {
+        if (s >= top_k) break;
+        int best = -1;
+        for (int i = 0; i < E; ++i) {
+          if ((taken[i >> 6] >> (i & 63)) & 1ull) continue;
+          if (best < 0 || __ldcg(logits + (size_t)t * E + i) > __ldcg(logits + (size_t)t * E + best)) best = i;
+        }
+        taken[best >> 6] |= 1ull << (best & 63);
+        pick[s] = best;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kMaxExperts / 32; ++j)
+      if (lane + 32 * j < E) ex[lane + 32 * j] = exp(v[j] - mx);
+    __syncwarp();
+    double sum = 0.0;                                         // in index order, by every lane alike
+#pragma unroll 8
+    for (int i = 0; i < E; ++i) sum += ex[i];
+    int mine = 0;                                             // lane s has choice s
+#pragma unroll
+    for (int s = 0; s < kMaxTopK; ++s)
+      if (s < top_k && lane == s) mine = pick[s];
+    const double pw = lane < top_k ? ex[mine] / sum : 0.0;
+    double chosen = 0.0;
+    for (int s = 0; s < top_k; ++s) chosen += __shfl_sync(0xffffffffu, pw, s);
+    if (lane < top_k) {
+      idx_out[(size_t)t * top_k + lane] = mine;
+      w_out[(size_t)t * top_k + lane] = (float)(renorm ? pw / chosen : pw);
+    }
+    __syncwarp();
+  }
+}
+
 // counts[e] = rows routed to expert e (a single CTA; T*top_k entries).
 __global__ void moe_count_kernel(const int* idx, int n, int E, int* counts, int* offsets, int* cursor, int* active,
                                  int n_listed) {
@@ -422,9 +627,22 @@ static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf1
   TQ_REQUIRE(ctx, h_bf16_dev && wg_bf16_dev && idx_out_dev && weight_out_dev, "tq_moe_router: null pointer");
   TQ_REQUIRE(ctx, d_model <= 24576 && d_model % 8 == 0 && ((uintptr_t)h_bf16_dev & 15) == 0 && ((uintptr_t)wg_bf16_dev & 15) == 0,
              "tq_moe_router: d_model must be a multiple of 8 and at most 24576, arrays 16-byte aligned");
+  // the f64 tensor-core form where the logits have a place to meet and the token blocks a counter each
+  const size_t mma_smem = 8 * kRtTok * kRtExp * 12 + (size_t)(kRtTok + kRtExp) * ((d_model + 31) / 32 * 4) * 2;
+  const size_t blocks = (n_tokens + kRtTok - 1) / kRtTok;
+  if (logits_ws && blocks <= (size_t)kTileCounters && mma_smem <= 160 * 1024) {
+    const size_t smem = mma_smem > 8 * kMaxExperts * 8 ? mma_smem : 8 * kMaxExperts * 8;
+    if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(router_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    router_mma_kernel<<<dim3((unsigned)blocks, (unsigned)((n_experts + kRtExp - 1) / kRtExp)), 256, smem, ctx->stream>>>(
+        static_cast<const __nv_bfloat16*>(h_bf16_dev), static_cast<const __nv_bfloat16*>(wg_bf16_dev), (int)n_tokens, (int)d_model,
+        (int)n_experts, (int)top_k, renormalize, idx_out_dev, weight_out_dev, logits_ws, ctx->dev_err + 1);
+    ctx->launches++;
+    TQ_CUDA(ctx, cudaGetLastError());
+    return TQ_OK;
+  }
   unsigned gy = 1;
   if (logits_ws && n_tokens <= 64 && n_tokens <= (size_t)kTileCounters) gy = (unsigned)((n_experts + 7) / 8);
-  // four tokens per CTA once there are several waves of CTAs anyway (their activations and ulp codes: 16 d bytes;
+  // (without them) four tokens per CTA once there are several waves of CTAs anyway (their activations and ulp codes: 16 d bytes;
   // measured alone at 1000 / 2048 tokens: 154 / 209 us against 119 / 206 us with one token per CTA)
   const bool four = n_tokens >= 2048 && 16 * d_model <= 64 * 1024;
   const size_t smem = (four ? 4 : 1) * d_model * 2 * sizeof(unsigned short);

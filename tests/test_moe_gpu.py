@@ -229,3 +229,41 @@ def test_shared_expert_on_both_sides_of_its_rule(dev, d, f, T):
         want[rows] += top[rows, c][:, None] * expert(moe.experts[e], h[rows])
     d_ = torch.from_numpy(got).cuda().double() - want
     assert (d_.norm() / want.norm()).item() < 5e-4, (d_.norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("d", [8, 40, 264, 2048])
+@pytest.mark.parametrize("T,E,k", [(1, 2, 2), (15, 8, 3), (16, 9, 1), (17, 64, 6), (33, 61, 16), (130, 256, 8)])
+def test_router_blocks_of_tokens_and_experts(dev, orc, d, T, E, k):
+    """Edges of the blocks of 16 tokens, 8 experts and 32 k; subnormals, infinities and NaN in some rows."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(T * E + d)
+    h = rng.standard_normal((T, d)).astype(np.float32)
+    wg = (rng.standard_normal((E, d)) * 0.05).astype(np.float32)
+    h[T // 2, d // 2] = 1e-39
+    wg[E // 2, 0] = 2e-30
+    if T > 16:
+        h[3, 1] = np.inf
+        h[16, d - 1] = np.nan
+    hb, hf = bf16_round(h)
+    wb, wf = bf16_round(wg)
+    if T > 16:
+        hb[16, d - 1] = 0x7FC0
+        hf[16, d - 1] = np.nan
+    idx, w, lg = tb.moe_router(dev, dev.upload(hb, tb.BF16), dev.upload(wb, tb.BF16), T, d, E, k)
+    for t in range(T):
+        oi, ow, ol = orc.router_f64(hf[t].astype(np.float64), wf.astype(np.float64), E, k)
+        assert np.array_equal(lg[t], ol, equal_nan=True), t
+        if not np.isnan(ol).any() and np.isfinite(ol).all():
+            assert list(idx[t]) == list(oi), t
+            assert np.abs(w[t] - ow).max() < 1e-6
+
+
+@pytest.mark.parametrize("E,T", [(40, 300), (70, 600)])
+def test_token_tiles_of_uneven_experts(dev, orc, E, T):
+    """The grouped tcgen05 GEMM with groups beyond one warp's scan: a few experts get most of the tokens."""
+    host = HostMoe(np.random.default_rng(E), d=256, ffn=128, n_experts=E, top_k=4, n_shared=0)
+    scale = np.full((E, 1), 0.05)
+    scale[1::E // 3] = 40.0
+    host.wg_bits, host.wg = bf16_round((host.wg * scale).astype(np.float32))
+    check(dev, orc, host, T, seed=E)
