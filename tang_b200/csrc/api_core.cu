@@ -125,6 +125,9 @@ int tq_ctx_create(int device, void* stream, tq_ctx** out) {
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(TQ_ECUDA);
     ctx->owns_stream = true;
   }
+  if (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&ctx->side_begin, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->side_done, cudaEventDisableTiming) != cudaSuccess)
+    return bail(TQ_ECUDA);
   if (cudaMalloc(&ctx->dev_err, (1 + kTileCounters) * sizeof(int)) != cudaSuccess) return bail(TQ_ECUDA);
   if (cudaMemsetAsync(ctx->dev_err, 0, (1 + kTileCounters) * sizeof(int), ctx->stream) != cudaSuccess) return bail(TQ_ECUDA);
   const size_t ws_bytes = (size_t)kGemvSets * kGemvMaxGrid * 2 * 128 * sizeof(unsigned long long);
@@ -158,6 +161,9 @@ int tq_ctx_destroy(tq_ctx* ctx) {
   if (ctx->hostx_tags) cudaFree(ctx->hostx_tags);   // (the epoch word sits behind the tags)
   if (ctx->bounce) cudaFreeHost(ctx->bounce);
   if (ctx->host_err) cudaFreeHost(ctx->host_err);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
+  if (ctx->side_begin) cudaEventDestroy(ctx->side_begin);
+  if (ctx->side_done) cudaEventDestroy(ctx->side_done);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return TQ_OK;

@@ -803,6 +803,33 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   ctx->launches++;      \
   TQ_CUDA(ctx, cudaGetLastError());
 
+  auto shared_experts = [&]() -> int {
+    for (size_t i = 0; i < m->sh_gate_up.size() && Ts > 0; ++i) {
+      // The same epilogue where K would not be split anyway (d 2048: f 1408 at 641 tokens 37.5 -> 33.1 us a shared expert, at 1000 60.1 ->
+      // 52.6; f 4096 at 512 76.1 -> 66.6; 4096 x 14336 at 256 207 -> 181), and for many tokens of a narrow expert, where the f32
+      // partials cost more than the idle SMs (1061 tokens, f 384 31.0 -> 28.4; 2048 45.5 -> 40.7; f 128 38.2 -> 36.0).
+      const tq_qweight* gate_up = m->sh_gate_up[i];
+      const bool sized = gate_up->rows == 2 * f && gate_up->cols == d;      // (any other size is for tq_qlinear to refuse)
+      const bool many = Ts >= 1024 || (Ts >= (size_t)umma_min_m(TQ_F32) && umma_fills_gpu(ctx, gate_up, Ts));
+      if (sized && many && gate_up->kind != TQ_I8_ROW && umma_supported(gate_up, Ts)) {
+        TQ_STEP(launch_qgemm_umma(ctx, gate_up, h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
+      } else {
+        TQ_STEP(tq_qlinear(ctx, gate_up, h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
+        TQ_STEP(tq_swiglu(ctx, shgu, shgu + f, TQ_F32, 2 * f, Ts, f, shact, TQ_BF16));
+      }
+      TQ_STEP(tq_qlinear(ctx, m->sh_down[i], shact, TQ_BF16, f, Ts, sh + i * Ts * d, TQ_F32, d, nullptr));
+    }
+    return TQ_OK;
+  };
+  // Routing needs few SMs and the shared experts do not need it: where their projections are the tcgen05 kernel's, which uses none of
+  // the context's workspaces, they run on a stream beside it, from what is in order here to the combination (layer with two shared
+  // experts: 64 tokens 227.7 -> 198.6 us, 4096 1563 -> 1541).
+  bool beside = Ts >= (size_t)umma_min_m(TQ_F32) && !m->sh_gate_up.empty();
+  for (size_t i = 0; i < m->sh_gate_up.size(); ++i) {
+    const tq_qweight *gu_w = m->sh_gate_up[i], *dn_w = m->sh_down[i];
+    beside = beside && gu_w->rows == 2 * f && gu_w->cols == d && dn_w->rows == d && dn_w->cols == f && umma_supported(gu_w, Ts) && umma_supported(dn_w, Ts);
+  }
+  if (beside) TQ_CUDA(ctx, cudaEventRecord(ctx->side_begin, ctx->stream));
   TQ_STEP(launch_router(ctx, h, m->wg, T, d, c.n_experts, k, c.renormalize, idx, w, reinterpret_cast<double*>(s + o_lg)));
   moe_localize_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(idx, (int)n, m->expert_lo, nl, idl);
   TQ_LAUNCHED();
@@ -812,6 +839,28 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   TQ_LAUNCHED();
   moe_gather_kernel<<<(unsigned)n, 128, 0, ctx->stream>>>(h, slot, (int)n, (int)k, (int)d, xs);
   TQ_LAUNCHED();
+  struct Join {   // whichever way the call returns: nothing is left running, or open in a capture, beside the caller's stream
+    tq_ctx* ctx = nullptr;
+    int now() {
+      tq_ctx* c = ctx;
+      ctx = nullptr;
+      if (c) TQ_CUDA(c, cudaStreamWaitEvent(c->stream, c->side_done, 0));
+      return TQ_OK;
+    }
+    ~Join() { now(); }
+  } join;
+  if (beside) {
+    cudaStream_t main = ctx->stream;
+    TQ_CUDA(ctx, cudaStreamWaitEvent(ctx->side, ctx->side_begin, 0));
+    ctx->stream = ctx->side;
+    st = shared_experts();
+    ctx->stream = main;
+    ctx->inflight_unknown = true;
+    ctx->n_inflight = 0;
+    TQ_CUDA(ctx, cudaEventRecord(ctx->side_done, ctx->side));
+    join.ctx = ctx;
+    if (st != TQ_OK) return st;
+  }
   // a token picks an expert at most once (counts[e] <= T); the chunk of rows one CTA takes follows the
   // expected rows per expert (T k / E), so that small batches do not pay for 64-row tiles
   size_t want = 2 * n / (size_t)c.n_experts + 1;
@@ -837,21 +886,8 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   } else {
     TQ_STEP(launch_qgemm_grouped(ctx, m->w_down, nl, act, f, cap, cnt, offs, (int)T, 0, 0, yo, TQ_F32, d, active, max_active, n));
   }
-  for (size_t i = 0; i < m->sh_gate_up.size() && Ts > 0; ++i) {
-    // The same epilogue where K would not be split anyway (d 2048: f 1408 at 641 tokens 37.5 -> 33.1 us a shared expert, at 1000 60.1 ->
-    // 52.6; f 4096 at 512 76.1 -> 66.6; 4096 x 14336 at 256 207 -> 181), and for many tokens of a narrow expert, where the f32
-    // partials cost more than the idle SMs (1061 tokens, f 384 31.0 -> 28.4; 2048 45.5 -> 40.7; f 128 38.2 -> 36.0).
-    const tq_qweight* gate_up = m->sh_gate_up[i];
-    const bool sized = gate_up->rows == 2 * f && gate_up->cols == d;      // (any other size is for tq_qlinear to refuse)
-    const bool many = Ts >= 1024 || (Ts >= (size_t)umma_min_m(TQ_F32) && umma_fills_gpu(ctx, gate_up, Ts));
-    if (sized && many && gate_up->kind != TQ_I8_ROW && umma_supported(gate_up, Ts)) {
-      TQ_STEP(launch_qgemm_umma(ctx, gate_up, h + sh_lo * d, d, Ts, shact, TQ_BF16, f, 2, nullptr, 2));
-    } else {
-      TQ_STEP(tq_qlinear(ctx, gate_up, h + sh_lo * d, TQ_BF16, d, Ts, shgu, TQ_F32, 2 * f, nullptr));
-      TQ_STEP(tq_swiglu(ctx, shgu, shgu + f, TQ_F32, 2 * f, Ts, f, shact, TQ_BF16));
-    }
-    TQ_STEP(tq_qlinear(ctx, m->sh_down[i], shact, TQ_BF16, f, Ts, sh + i * Ts * d, TQ_F32, d, nullptr));
-  }
+  st = beside ? join.now() : shared_experts();
+  if (st != TQ_OK) return st;
   moe_combine_local_kernel<<<dim3((unsigned)T, (unsigned)((d + 1023) / 1024)), 256, 0, ctx->stream>>>(yo, slot, idl, w, (c.n_shared && Ts) ? sh : nullptr, (int)c.n_shared,
                                                                  Ts * d, (int)sh_lo, (int)sh_hi, (int)k, (int)d, nl, out_dev);
   TQ_LAUNCHED();
