@@ -22,6 +22,12 @@
 
 namespace tq {
 
+// gqa_prefill_umma.cu
+bool gqa_prefill_umma_supported(const void* q, const void* k, const void* v, const void* out, size_t seq_stride);
+int launch_gqa_prefill_umma(tq_ctx* ctx, const void* q, const void* k, const void* v, const int* cache_start, size_t batch, size_t q_len,
+                            size_t n_heads, size_t n_kv, size_t seq_stride, float scale, void* out, int out_f32);
+
+
 constexpr int kHD = 128;              // head dimension of the MMA kernel
 constexpr int kTileKeys = 64;         // positions per smem tile
 constexpr int kRowBytes = kHD * 2 + 16;  // padded smem row: 272 B keeps ldmatrix / 4-byte reads conflict-free
@@ -297,7 +303,7 @@ __global__ void __launch_bounds__(kHD) gqa_combine_kernel(const float* part_o, c
 // Causal GQA attention for a chunk of q_len new positions per sequence (prefill, q_len > 1 of
 // ComputeDevice::kv_attention, crates/tang-compute/src/device.rs:161-180; cpu.rs:257-315): query i of sequence b
 // attends cache positions 0 .. cache_start[b] + i.  bf16 q / K / V, f32 online softmax, bf16 probabilities into
-// the tensor core (mma.sync m16n8k16).  A CTA owns 64 (position, head-of-the-group) rows of one KV head -- so the
+// the tensor core (mma.sync m16n8k16; many rows: gqa_prefill_umma.cu).  A CTA owns 64 (position, head-of-the-group) rows of one KV head -- so the
 // K/V tiles it streams (cp.async, double-buffered, 64 keys each) serve every query head of the group -- and each
 // of its four warps 16 of those rows against all 64 keys of a tile.
 // ---------------------------------------------------------------------------------------------
@@ -617,6 +623,12 @@ int tq_gqa_prefill(tq_ctx* ctx, const void* q_dev, const void* k_cache_dev, cons
   TQ_REQUIRE(ctx, n_kv_heads > 0 && n_heads % n_kv_heads == 0 && (group == 1 || group == 2 || group == 4 || group == 8),
              "tq_gqa_prefill: n_heads/n_kv_heads must be 1, 2, 4 or 8");
   TQ_REQUIRE(ctx, out_dtype == TQ_BF16 || out_dtype == TQ_F32, "tq_gqa_prefill: out must be bf16 or f32");
+  // The tcgen05 kernel from 1024 rows (position, head of a KV head's group) per sequence on: its CTAs take 256 rows, and below that too few of
+  // them are busy unless many positions are cached, which only the device knows.  32 heads, 8 KV heads, us (mma.sync, tcgen05): 256 positions
+  // 15.1, 12.8; 128 positions 7.5, 9.6; 64 positions 6.5, 9.3, behind 1000 cached ones 39.6, 33.9.
+  if (q_len * group >= 1024 && gqa_prefill_umma_supported(q_dev, k_cache_dev, v_cache_dev, out_dev, seq_stride))
+    return launch_gqa_prefill_umma(ctx, q_dev, k_cache_dev, v_cache_dev, cache_start_dev, batch, q_len, n_heads, n_kv_heads, seq_stride,
+                                   1.0f / sqrtf((float)head_dim), out_dev, out_dtype == TQ_F32);
   PrefillParams p;
   p.q = static_cast<const __nv_bfloat16*>(q_dev);
   p.k_cache = static_cast<const __nv_bfloat16*>(k_cache_dev);
