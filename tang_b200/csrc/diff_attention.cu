@@ -12,6 +12,7 @@
 // Key tiles of 64 rows arrive by cp.async, two in flight.  Only tiles with visible keys are visited: those of the kept
 // first tokens, then those of the window.
 //
+// diff_attention_umma.cu is the first form on tcgen05, for one pair of head sizes and many rows.
 // diff_attention_simt_kernel is the exact f32 form (and takes bf16 heads of any size).
 #include "diff_attention.cuh"
 
@@ -537,6 +538,11 @@ static int launch_mma(tq_ctx* ctx, DiffParams& p, bool split, size_t smem, dim3 
   return split ? go(diff_attention_kernel<DVT, true>, 128) : go(diff_attention_kernel<DVT, false>, 256);
 }
 
+// diff_attention_umma.cu
+bool diff_attention_umma_supported(const DiffAttn& a, const RaggedBatch& b, const void* q, size_t ldq, const void* k, const void* v, const void* out, size_t ldo);
+int launch_diff_attention_umma(tq_ctx* ctx, const DiffAttn& a, const RaggedBatch& b, const void* q, size_t ldq, const void* k, const void* v, void* out,
+                               size_t ldo);
+
 int launch_diff_attention(tq_ctx* ctx, const DiffAttn& a, const RaggedBatch& b, int dtype, const void* q, size_t ldq, const void* k_cache,
                           const void* v_cache, void* out, size_t ldo) {
   TQ_REQUIRE(ctx, a.heads > 0 && a.kv_heads > 0 && a.heads % a.kv_heads == 0, "differential attention: heads must be a multiple of kv_heads");
@@ -546,6 +552,11 @@ int launch_diff_attention(tq_ctx* ctx, const DiffAttn& a, const RaggedBatch& b, 
   if (b.rows == 0 || b.n_seqs == 0) return TQ_OK;
   if (dtype == TQ_F32) return launch_simt<float>(ctx, a, b, q, ldq, k_cache, v_cache, out, ldo);
   if (a.dim > 256 || a.vdim > 256) return launch_simt<__nv_bfloat16>(ctx, a, b, q, ldq, k_cache, v_cache, out, ldo);
+  // The tcgen05 kernel from 1024 rows (query, head of a KV head's group) of the longest sequence on: a CTA takes 128 rows in both maps, and below
+  // that too few are busy.  Four layers of the 1b shape, us (mma.sync, tcgen05): one prompt of 64 tokens 414, 442, of 128 481, 472, of 256 554, 518,
+  // of 1024 1025, 807; eight of 128 with a window of 128 555, 565.
+  if (b.max_q > 1 && (long long)b.max_q * (a.heads / a.kv_heads) >= 1024 && diff_attention_umma_supported(a, b, q, ldq, k_cache, v_cache, out, ldo))
+    return launch_diff_attention_umma(ctx, a, b, q, ldq, k_cache, v_cache, out, ldo);
   DiffParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
   p.k = static_cast<const __nv_bfloat16*>(k_cache);

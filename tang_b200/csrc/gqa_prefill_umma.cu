@@ -16,14 +16,12 @@
 
 #include <cuda_bf16.h>
 
+#include "attn_umma.cuh"
 #include "internal.h"
-#include "qgemm_umma.cuh"
-#include "tensormap.h"
 
 namespace tq {
 
-constexpr int kPfThreads = 384, kPfTile = 128, kPfHd = 128;
-constexpr int kPfBox = kPfTile * 128;                 // 128 rows of 64 bf16
+constexpr int kPfThreads = 384, kPfHd = 128;
 constexpr int kPfStage = 4 * kPfBox;                  // K, V: two boxes each
 constexpr int kPfStages = 2;
 constexpr size_t kPfSmem = 1024 + 1024 + 4 * (size_t)kPfBox + kPfStages * (size_t)kPfStage;
@@ -36,27 +34,6 @@ struct PrefillUmmaParams {
   int out_f32;
   int* err;
 };
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void pf_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-               "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\ttcgen05.wait::ld.sync.aligned;"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-                 "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                 "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]) : "r"(taddr) : "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-// Operand whose rows are k and whose 64-element columns are contiguous (see mla_umma.cu)
-__device__ __forceinline__ uint64_t pf_desc_mn(const void* smem_ptr) {
-  return (uint64_t)((smem_u32(smem_ptr) >> 4) & 0x3FFF) | (uint64_t)(kPfBox >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
 
 __global__ void __launch_bounds__(kPfThreads, 1)
 gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
@@ -309,15 +286,6 @@ gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
   if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-static bool encode_3d(CUtensorMap* map, const void* base, size_t d0, size_t d1, size_t d2, size_t stride1, size_t stride2, unsigned b1, unsigned b2) {
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return false;
-  const cuuint64_t gdim[3] = {d0, d1, d2}, gstride[2] = {stride1, stride2};
-  const cuuint32_t box[3] = {64, b1, b2}, estr[3] = {1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 bool gqa_prefill_umma_supported(const void* q, const void* k, const void* v, const void* out, size_t seq_stride) {
   return encode_tiled() && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) == 0 && seq_stride % 8 == 0;
 }
@@ -337,8 +305,8 @@ int launch_gqa_prefill_umma(tq_ctx* ctx, const void* q, const void* k, const voi
   p.out_f32 = out_f32;
   p.err = ctx->dev_err;
   CUtensorMap qm, km, vm;
-  if (!encode_3d(&qm, q, kPfHd, n_heads, batch * q_len, kPfHd * 2, n_heads * kPfHd * 2, (unsigned)group, (unsigned)(kPfTile / group)) ||
-      !encode_3d(&km, k, row, rows_max, batch, row * 2, seq_stride * 2, kPfTile, 1) || !encode_3d(&vm, v, row, rows_max, batch, row * 2, seq_stride * 2, kPfTile, 1))
+  if (!encode_bf16_boxes(&qm, q, kPfHd, n_heads, batch * q_len, kPfHd * 2, n_heads * kPfHd * 2, (unsigned)group, (unsigned)(kPfTile / group)) ||
+      !encode_bf16_boxes(&km, k, row, rows_max, batch, row * 2, seq_stride * 2, kPfTile, 1) || !encode_bf16_boxes(&vm, v, row, rows_max, batch, row * 2, seq_stride * 2, kPfTile, 1))
     return fail(ctx, TQ_ECUDA, "cuTensorMapEncodeTiled failed");
   TQ_CUDA(ctx, cudaFuncSetAttribute(gqa_prefill_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPfSmem));
   TQ_CUDA(ctx, launch_k(ctx, gqa_prefill_umma_kernel, dim3((unsigned)((q_len + per_cta - 1) / per_cta), (unsigned)n_kv, (unsigned)batch), dim3(kPfThreads),
