@@ -26,6 +26,9 @@ int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const v
                          void* y, int y_dtype, size_t ldy, const int* active = nullptr,
                          int max_active = 0, size_t total_rows = 0);
 
+// Rows per expert, when routing is even, from which the experts' products are the tcgen05 kernel's (the other kernel reads an expert's weights
+// once per eight rows).  64 experts, 6 chosen, d 2048, f 1408, two shared experts, us (qgemm_skg, tcgen05): 96 tokens 202, 253, 128 294, 253, 192 406, 273.
+constexpr size_t kTensorRows = 12;
 constexpr int kMaxExperts = 256;
 constexpr int kMaxTopK = 16;
 
@@ -868,9 +871,9 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
   while (cap < 64 && (size_t)cap < want) cap <<= 1;
   if ((size_t)cap > T) cap = (int)T;
   const int max_active = (int)(n < (size_t)nl ? n : (size_t)nl);   // at most one expert per (token, choice)
-  // from about 24 rows per expert on, the expert GEMMs run on the tcgen05 kernel (one launch over all experts)
+  // many rows per expert: the expert GEMMs run on the tcgen05 kernel (one launch over all experts)
   const size_t expected = n / (size_t)c.n_experts;
-  const bool tensor_path = expected >= 24 && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
+  const bool tensor_path = expected >= kTensorRows && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
   if (tensor_path) {
     // silu(gate) * up in the projection's epilogue, from the same f32 sums (two terms per weight although the result is bf16): the
     // f32 round trip of the 2 f wide projection and its kernel are gone
@@ -1009,7 +1012,7 @@ int tq_moe_ffn_dispatch(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, floa
   const int max_rows = (int)((size_t)W * T < R ? (size_t)W * T : R);   // an expert gets a token at most once
   const int max_active = (int)(R < (size_t)nl ? R : (size_t)nl);
   const size_t expected = (size_t)W * n / (size_t)c.n_experts;      // rows per local expert when routing is even
-  const bool tensor_path = expected >= 24 && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
+  const bool tensor_path = expected >= kTensorRows && umma_grouped_supported(m->w_gate_up, nl) && umma_grouped_supported(m->w_down, nl);
   if (tensor_path) {
     TQ_STEP(launch_qgemm_umma_grouped(ctx, m->w_gate_up, nl, xs, d, Rr, cnt, offs, max_active, (int)(expected * 3 / 2),
                                       gu, TQ_F32, 2 * f));
