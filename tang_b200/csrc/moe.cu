@@ -302,8 +302,11 @@ __global__ void __launch_bounds__(256, 4) router_kernel(const __nv_bfloat16* h, 
 // of runs of eight k (a product of the run is a multiple of 2 to the sum of both minima); a pair that fails with that is looked at
 // product by product, and then summed in the reference order (of normal values 7 and 2 of 10,000).
 // A CTA takes 16 tokens and 8 experts, its warps every eighth block of 32 k; the CTA of a token block that finishes last selects.
-// 64 experts, d 2048, us (router_kernel -> this): 1 token 27.4 -> 18.9, 64 31.5 -> 23.4, 1000 117 -> 50, 4096 355 -> 127, 16384 1219 -> 438.
+// 64 experts, d 2048, us (router_kernel -> this): 1 token 27.4 -> 17, 64 31.7 -> 21, 1000 117 -> 44, 4096 355 -> 104, 16384 1219 -> 343.
 constexpr int kRtTok = 16, kRtExp = 8;
+// Rows of codes lie 16 bytes apart in the banks, since eight experts' rows are read at once: without, 88 % of the wavefronts of shared
+// memory were conflicts (4096 tokens 127 us against 104).
+__host__ __device__ constexpr int router_code_ld(int runs) { return (runs + 63) / 64 * 64 + 8; }
 __device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
@@ -316,11 +319,11 @@ __device__ __forceinline__ unsigned short run_ulp_code(const uint4& v) {   // th
 __global__ void __launch_bounds__(256) router_mma_kernel(const __nv_bfloat16* h, const __nv_bfloat16* wg, int T, int d, int E, int top_k,
                                                          int renorm, int* idx_out, float* w_out, double* logits, int* counters) {
   extern __shared__ __align__(16) uint8_t rt_smem[];
-  const int n_blk = (d + 31) / 32, runs = 4 * n_blk;         // blocks of 32 k, runs of 8
+  const int n_blk = (d + 31) / 32, runs = 4 * n_blk, ld = router_code_ld(runs);   // blocks of 32 k, runs of 8
   double* part = reinterpret_cast<double*>(rt_smem);          // [warp][token][expert]
   float* mags = reinterpret_cast<float*>(part + 8 * kRtTok * kRtExp);
-  unsigned short* ch = reinterpret_cast<unsigned short*>(mags + 8 * kRtTok * kRtExp);   // [token][runs]
-  unsigned short* cw = ch + kRtTok * runs;                    // [expert][runs]
+  unsigned short* ch = reinterpret_cast<unsigned short*>(mags + 8 * kRtTok * kRtExp);   // [token][ld]
+  unsigned short* cw = ch + kRtTok * ld;                      // [expert][ld]
   const int t0 = blockIdx.x * kRtTok, e0 = blockIdx.y * kRtExp, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, q4 = lane & 3;
   const unsigned short* hp = reinterpret_cast<const unsigned short*>(h);
@@ -337,9 +340,9 @@ __global__ void __launch_bounds__(256) router_mma_kernel(const __nv_bfloat16* h,
     const uint4 a1 = in && t0 + g + 8 < T ? *reinterpret_cast<const uint4*>(hp + (size_t)(t0 + g + 8) * d + k) : zero;
     const uint4 bw = in && e0 + g < E ? *reinterpret_cast<const uint4*>(wp + (size_t)(e0 + g) * d + k) : zero;
     const int run = 4 * b + q4;
-    ch[g * runs + run] = run_ulp_code(a0);
-    ch[(g + 8) * runs + run] = run_ulp_code(a1);
-    cw[g * runs + run] = run_ulp_code(bw);
+    ch[g * ld + run] = run_ulp_code(a0);
+    ch[(g + 8) * ld + run] = run_ulp_code(a1);
+    cw[g * ld + run] = run_ulp_code(bw);
     const unsigned x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w}, y[4] = {bw.x, bw.y, bw.z, bw.w};
     constexpr unsigned kAbs = 0x7FFF7FFFu;
     mma_bf16_16816(mag, x0[0] & kAbs, x1[0] & kAbs, x0[1] & kAbs, x1[1] & kAbs, y[0] & kAbs, y[1] & kAbs);
@@ -366,8 +369,8 @@ __global__ void __launch_bounds__(256) router_mma_kernel(const __nv_bfloat16* h,
   {
     const int pair = threadIdx.x >> 1, half = threadIdx.x & 1, tk = pair >> 3, ex = pair & 7;
     unsigned q2 = 0xFFFFFFFFu;
-    const uint2* ph = reinterpret_cast<const uint2*>(ch + tk * runs);     // (runs is a multiple of four)
-    const uint2* pw = reinterpret_cast<const uint2*>(cw + ex * runs);
+    const uint2* ph = reinterpret_cast<const uint2*>(ch + tk * ld);     // (ld is a multiple of four)
+    const uint2* pw = reinterpret_cast<const uint2*>(cw + ex * ld);
     for (int i = half; i < runs / 4; i += 2) {
       const uint2 u = ph[i], v = pw[i];
       q2 = __viaddmin_u16x2(u.x, v.x, q2);
@@ -675,7 +678,7 @@ static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf1
   TQ_REQUIRE(ctx, d_model <= 24576 && d_model % 8 == 0 && ((uintptr_t)h_bf16_dev & 15) == 0 && ((uintptr_t)wg_bf16_dev & 15) == 0,
              "tq_moe_router: d_model must be a multiple of 8 and at most 24576, arrays 16-byte aligned");
   // the f64 tensor-core form where the logits have a place to meet and the token blocks a counter each
-  const size_t mma_smem = 8 * kRtTok * kRtExp * 12 + (size_t)(kRtTok + kRtExp) * ((d_model + 31) / 32 * 4) * 2;
+  const size_t mma_smem = 8 * kRtTok * kRtExp * 12 + (size_t)(kRtTok + kRtExp) * router_code_ld(((int)d_model + 31) / 32 * 4) * 2;
   const size_t blocks = (n_tokens + kRtTok - 1) / kRtTok;
   if (logits_ws && blocks <= (size_t)kTileCounters && mma_smem <= 160 * 1024) {
     const size_t smem = mma_smem > 8 * kMaxExperts * 8 ? mma_smem : 8 * kMaxExperts * 8;
