@@ -45,6 +45,7 @@ diff_attention_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
   uint64_t* p_full = s_full + 2;
   uint64_t* o_done = p_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);   // a map's softmax gave up
   uint8_t* q_s = smem_raw + 1024 + ((1024 - ((smem_u32(smem_raw) + 1024) & 1023)) & 1023);
   uint8_t* kv_s = q_s + 2 * kPfBox;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -81,6 +82,7 @@ diff_attention_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
         mbar_init(&p_full[x], 4);
         mbar_init(&o_done[x], 1);
       }
+      *failed = 0;
       mbar_init_fence();
     }
   } else if (warp == 1) {
@@ -252,9 +254,16 @@ diff_attention_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[x]);
     }
-    // ---- both maps' outputs, a2 through shared memory (the stages are free when both maps' products are done)
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_spin(&o_done[0], (n - 1) & 1) && mbar_wait_spin(&o_done[1], (n - 1) & 1));
-    if (!ok) give_up(DERR_TMEM);
+    // ---- both maps' outputs, a2 through shared memory.  The stages are free when both maps' products are done.  Each map's group looks at its
+    // own map's barrier, since a wait for a parity is only sound for a thread that knows the phase before to be over (the scores of tile n - 1
+    // stand behind this map's products of tile n - 2; the other map may be tiles behind), and the groups then meet.
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait_spin(&o_done[x], (n - 1) & 1));
+    if (!ok) {
+      give_up(DERR_TMEM);
+      *failed = 1;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    ok = *failed == 0;
     tc_fence_after();
     float* a2 = reinterpret_cast<float*>(kv_s) + r;   // [column][row]
     if (ok && x == 1) {

@@ -66,3 +66,19 @@ def test_one_key_decides(dev, window, keep):
         case = Aligned(rng, 4, 1, 64, 128, window, keep, seqs=[(120, 264)], max_seq=384)
         D._stand_out(case, 0, pos - 120, j, 12.0, n % 4, n % 2)
         D.check(dev, case, rows=[pos - 120])
+
+
+@pytest.mark.parametrize("grows", [0, 1])
+@pytest.mark.parametrize("tiles", [2, 4, 5, 7])
+def test_one_map_behind_the_other(dev, tiles, grows):
+    """The row maxima of one map grow with every tile, so that its outputs are rescaled each time, and the other map's hardly do: the maps run apart
+    by whole tiles, and the exchange of the second map's outputs has to wait for the first's last products."""
+    rng = np.random.default_rng(tiles)
+    case = Aligned(rng, 8, 1, 64, 128, 2000, 0, seqs=[(128 * (tiles - 1), 128), (128 * (tiles - 1) + 5, 123)], max_seq=128 * tiles)
+    for b in range(2):
+        u = case.q[b][0, 0, grows].copy()
+        case.q[b][:, :, grows] = bf16_round(u * rng.uniform(0.8, 1.2, case.q[b].shape[:2] + (1,)).astype(np.float32))[1]
+        n = case.k[b].shape[0]
+        case.k[b][:, 0, grows] = bf16_round((u / np.dot(u, u) / case.scale * (np.arange(n) / 32)[:, None]).astype(np.float32))[1]
+        case.k[b][:, 0, 1 - grows] = bf16_round(case.k[b][:, 0, 1 - grows] * 0.05)[1]
+    D.check(dev, case, rows=[0, 1, 64, 122])
