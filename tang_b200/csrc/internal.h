@@ -52,8 +52,9 @@ struct tq_ctx {
   int sm_count = 148;
   int umma_clusters[9] = {};     // clusters of that many CTAs of the tcgen05 GEMM that run at once (0: not asked yet, -1: none)
   // Kernels that may still be running when the next kernel launched with the programmatic-launch attribute
-  // starts: either exactly the previous one, with unknown outputs (`inflight_unknown`; every kernel but the
-  // persistent GEMV waits for its predecessor before it lets its successor be scheduled), or a run of
+  // starts: either the previous one and what that one waits for, with unknown outputs (`inflight_unknown`; most kernels
+  // wait for their predecessor before they let their successor be scheduled, the tcgen05 dequant-GEMM after, but none
+  // completes before its predecessor has), or a run of
   // persistent GEMVs whose inputs and outputs are the byte ranges listed here.  A GEMV whose activations
   // overlap none of the outputs reads them without waiting and lets its own successor be scheduled at once; if
   // its output and residual are clear of everything listed as well, it does not wait at all.
@@ -160,8 +161,10 @@ int ensure_splitk(tq_ctx* ctx, size_t bytes);
 
 // Launches `kern` on the context's stream.  With programmatic dependent launch enabled (default;
 // TQ_PDL=0 turns it off) the launch carries the programmatic-stream-serialization attribute, so the
-// kernel may start while its predecessor drains; every kernel launched this way executes
-// `griddepcontrol.wait` before it touches memory another kernel wrote or still reads.
+// kernel may start while its predecessor drains.  A kernel launched this way executes `griddepcontrol.wait` before it
+// touches memory another kernel wrote or still reads, with two exceptions: the GEMVs' inputs and outputs that the list of
+// kernels in flight clears, and quantised weights, which the products copy before they wait.  For these the constructors end with
+// a kernel launched without the attribute (qlinear.cu) or with a synchronisation.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(tq_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
   cudaLaunchConfig_t cfg = {};

@@ -149,8 +149,8 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
 
-  // (weights are not written by a kernel in flight: they stream and are converted before the wait for the activations, which
-  // the thread that copies them does; everything that is stored depends on these)
+  // (weights are not written by a kernel in flight -- their constructors end with a launch or a wait that sees to it --: they stream and are
+  // converted before the wait for the activations, which the thread that copies them does; everything that is stored depends on these)
   pdl_launch_dependents();
 
   auto give_up = [&](int code) {

@@ -811,6 +811,16 @@ static void plain_strides(int kind, size_t cols, size_t* ld_pay, size_t* ld_sc) 
   *ld_sc = kind == TQ_I8_ROW ? 0 : bpr * scale_elem(kind);
 }
 
+// The last launch of a constructor that returns with its kernels queued.  Products copy their weights before griddepcontrol.wait, and a kernel
+// launched with the programmatic attribute may start when its predecessor's CTAs have left, before their stores are guaranteed visible.
+// This one is launched without it, so it starts behind all that was written, and a product behind it behind that.
+__global__ void weights_written_kernel() {}
+static cudaError_t launch_weights_written(tq_ctx* ctx) {
+  weights_written_kernel<<<1, 1, 0, ctx->stream>>>();
+  ctx->launches++;
+  return cudaGetLastError();
+}
+
 // Repacks plain device arrays into w->tiles.
 static int repack_from_device(tq_ctx* ctx, tq_qweight* w, const uint8_t* pay, const uint8_t* sc) {
   size_t ld_pay, ld_sc;
@@ -822,6 +832,7 @@ static int repack_from_device(tq_ctx* ctx, tq_qweight* w, const uint8_t* pay, co
   TQ_CUDA(ctx, cudaGetLastError());
   if (w->kind == TQ_I8_ROW)
     TQ_CUDA(ctx, cudaMemcpyAsync(w->row_scales, sc, w->rows * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+  TQ_CUDA(ctx, launch_weights_written(ctx));
   return TQ_OK;
 }
 
@@ -1356,6 +1367,7 @@ extern "C" int tq_qweight_interleave_gate_up(tq_ctx* ctx, const tq_qweight* w_ga
         e = cudaMemcpyAsync(w->row_scales + 16 * (size_t)b + 8, w_gate_up->row_scales + f + 8 * (size_t)b, 8 * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
     }
   }
+  if (e == cudaSuccess) e = launch_weights_written(ctx);
   if (e != cudaSuccess) {
     tq_qweight_free(ctx, w);
     return tq::fail(ctx, TQ_ECUDA, "tq_qweight_interleave_gate_up: %s", cudaGetErrorString(e));

@@ -70,3 +70,29 @@ def test_result_rows_of_any_stride(dev, orc, dtype, rows, cols, m, ld):
     dev.sync()
     assert np.array_equal(got[:, :rows], dense)
     assert (got[:, rows:] == 7).all() and out.to_vec()[0] == 7
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(256, 512), (14336, 1024)])
+@pytest.mark.parametrize("m", [1, 4, 12, 17, 64, 300])
+def test_product_right_behind_its_weight(dev, kind, rows, cols, m):
+    """Both constructors that return before their kernels have run, and a product with the weight at once: the products copy their weights
+    before they wait for the kernel in front.  Every product is of a weight of its own."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(rows + m)
+    sc, pay = make_weight(rng, kind, rows, cols)
+    pay_d, sc_d = dev.upload(pay.view(np.uint8), tb.U8), dev.upload(np.ascontiguousarray(sc).view(np.uint8), tb.U8)
+    x = dev.upload(bf16_round(rng.standard_normal((m, cols)).astype(np.float32))[0], tb.BF16)
+    dev.sync()
+    ws, ys = [], []
+    for i in range(4):
+        ws.append(dev.qweight_from_device(kind, pay_d.ptr, sc_d.ptr, rows, cols))
+        if i & 1:
+            ws.append(dev.interleave_gate_up(ws[-1], free_source=False))
+        ys.append(dev.qlinear(x, ws[-1], m, tb.F32))
+    dev.sync()
+    plain, mixed = dev.qlinear(x, ws[0], m, tb.F32).to_vec(), dev.qlinear(x, ws[2], m, tb.F32).to_vec()
+    for i, y in enumerate(ys):
+        # (a row block's pieces may meet in another order: f32 roundings, 1e-5 of the rms; stale weights are off by all of it)
+        assert np.abs(y.to_vec() - (mixed if i & 1 else plain)).max() < 1e-5 * np.sqrt(np.mean(plain.astype(np.float64) ** 2)), i
