@@ -36,7 +36,7 @@ __device__ __forceinline__ float4 cluster_sum(const float* mine, int n) {
 }
 __device__ __forceinline__ float4 times(float4 v, const float* s) { return make_float4(v.x * s[0], v.y * s[1], v.z * s[2], v.w * s[3]); }
 
-template <int KIND, int TERMS, bool DUAL = false>
+template <int KIND, int TERMS, int DUAL = 0>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ UmmaParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -46,7 +46,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   constexpr int kTileLines = TB / 128;   // 128-byte lines of a tile: its weights, then its scales
   static_assert(KIND != I8_ROW || TERMS == 1, "int8 rows carry no scale into the operand: one exact term");
   // DUAL: the CTA covers two token tiles of p.ntok rows with one conversion of the weights: issuer warp 1 multiplies
-  // every stage with the first tile's activations, warp 3 with the second tile's, each into one accumulator
+  // every stage with the first tile's activations, warp 3 with the second tile's, each into DUAL accumulators
   static_assert(!DUAL || TERMS == 1, "two token tiles per CTA: single-term weights");
   constexpr int kTokTiles = DUAL ? 2 : 1;
   // ---- shared-memory carve-up (operand tiles need 1024-byte alignment for the 128-byte swizzle)
@@ -237,8 +237,8 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
           ok = mbar_wait_spin(&x_full[xs + 1], xph);
           if (!ok) { give_up(DERR_FULL_WAIT); break; }
         }
-        const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride);
-        const uint32_t fresh = (DUAL ? j == 0 : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
+        const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride) + (DUAL == 2 ? (uint32_t)(half * kUmmaDualAcc) : 0u);
+        const uint32_t fresh = (DUAL ? j < DUAL : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
         if (leader) {
 #pragma unroll
           for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
@@ -430,9 +430,9 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tile * p.acc_stride + c0), v);
         const int mt = m0 + tile * p.ntok;                // first token of the tile
         // (accumulator a: issuer a & 1's number a >> 1, which that issuer has reached if it had that many steps)
-        for (int a = 1; a < (DUAL ? 1 : p.n_acc); ++a) {
-          if ((a >> 1) >= 2 * ((kc_len + 1 - (a & 1)) >> 1)) continue;
-          tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(a * p.acc_stride + c0), v1);
+        for (int a = 1; a < (DUAL ? DUAL : p.n_acc); ++a) {
+          if (!DUAL && (a >> 1) >= 2 * ((kc_len + 1 - (a & 1)) >> 1)) continue;
+          tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)((DUAL ? tile * p.acc_stride + a * kUmmaDualAcc : a * p.acc_stride) + c0), v1);
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] += v1[i];
         }
@@ -623,6 +623,10 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   const int a_col0 = dual ? 384 : 256, stages = terms == 2 || dual ? 2 : 4;
   int n_acc = 2;                       // a power of two, as many as tensor memory holds beside the weights
   while (!dual && n_acc < 16 && 2 * n_acc * acc_stride <= a_col0) n_acc <<= 1;
+  // Two accumulators for each of two token tiles, where they fit and the sums' error shows: int8 rows with f32 results.  14336 x 4096 at 144 rows:
+  // error 1.05e-6 with one, 4.3e-7 with two, as with a token tile per CTA; 26 us either way.  (A kernel that can do both costs 2048 rows 2.5 %.)
+  const bool two_acc = dual && ntok <= kUmmaDualAcc && w->kind == TQ_I8_ROW && y_dtype == TQ_F32;
+  if (two_acc) acc_stride = 2 * kUmmaDualAcc;
   // Shared memory: slots of activations (KX boxes of 64 k by one copy; one box with two token tiles), the rest packed tiles, whose bytes
   // in flight hide the latency of HBM: ring slots of KT = 4 k-tiles where two such fit, else 2.
   const int kx = dual ? 1 : ntok <= 64 ? 4 : 2;
@@ -684,10 +688,10 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   cudaError_t e;
   if (dual) {
     if (splits != 1) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: two token tiles per CTA with K split");
-    if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1, true>);
-    else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 1, true>);
-    else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 1, true>);
-    else e = go(qgemm_umma_kernel<Q4_F32, 1, true>);
+    if (w->kind == TQ_I8_ROW) e = two_acc ? go(qgemm_umma_kernel<I8_ROW, 1, 2>) : go(qgemm_umma_kernel<I8_ROW, 1, 1>);
+    else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 1, 1>);
+    else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 1, 1>);
+    else e = go(qgemm_umma_kernel<Q4_F32, 1, 1>);
   } else if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1>);
   else if (w->kind == TQ_Q4_F16) e = terms == 2 ? go(qgemm_umma_kernel<Q4_F16, 2>) : go(qgemm_umma_kernel<Q4_F16, 1>);
   else if (w->kind == TQ_Q8_F32) e = terms == 2 ? go(qgemm_umma_kernel<Q8_F32, 2>) : go(qgemm_umma_kernel<Q8_F32, 1>);

@@ -40,6 +40,7 @@ constexpr int kUmmaGroups = 2;        // dequant groups, each converting every s
 constexpr int kUmmaGroupWarps = 8;    // warps per group
 constexpr int kUmmaDqWarps = kUmmaGroups * kUmmaGroupWarps;   // dequant / epilogue warps
 constexpr int kUmmaFirstDqWarp = 4;   // warps 0..3: weight producer, MMA issuer (even steps), activation producer, MMA issuer (odd steps)
+constexpr int kUmmaDualAcc = 96;      // two token tiles per CTA: columns between a tile's accumulators, where it has two
 constexpr int kUmmaThreads = 32 * (kUmmaFirstDqWarp + kUmmaDqWarps);
 
 struct UmmaParams {
@@ -49,10 +50,10 @@ struct UmmaParams {
   int m_total;            // activation rows
   int n_rows;             // output features (multiple of 128)
   int kc_total;           // K / 128
-  int ntok;               // tokens per CTA tile = UMMA N (multiple of 16, <= 256)
-  int acc_stride;         // columns between accumulators
+  int ntok;               // tokens per CTA tile = UMMA N (multiple of 16, <= 192)
+  int acc_stride;         // columns between accumulators (two token tiles: between the tiles')
   int a_col0;             // tensor-memory columns of the converted weights: stages x 2 x terms x 32 from here on
-  int n_acc;              // accumulators (2, 4 or 8): 64-k step j of issuer i adds into number i + 2 * (j % (n_acc / 2))
+  int n_acc;              // accumulators (2, 4 or 8): 64-k step j of issuer i adds into number i + 2 * (j % (n_acc / 2)) (two token tiles: see the kernel)
   int stages;             // stages of converted weights in tensor memory (128 k each; even)
   int x_slots, kx;        // slots of activations in shared memory, 64-k boxes per slot (4; more than 64 tokens 2, two token tiles 1)
   int raw_stages;         // packed-tile ring depth (slots of kt tiles of 128 k): what keeps the HBM stream in flight

@@ -96,3 +96,44 @@ def test_product_right_behind_its_weight(dev, kind, rows, cols, m):
     for i, y in enumerate(ys):
         # (a row block's pieces may meet in another order: f32 roundings, 1e-5 of the rms; stale weights are off by all of it)
         assert np.abs(y.to_vec() - (mixed if i & 1 else plain)).max() < 1e-5 * np.sqrt(np.mean(plain.astype(np.float64) ** 2)), i
+
+
+def sum_error(dev, kind, rows, cols, m):
+    """Relative error (2-norm) of f32 results against f64, normal weights and activations."""
+    import tang_b200 as tb
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(rows + cols + m)
+    w = torch.randn((rows, cols), device="cuda", generator=g) * cols ** -0.5
+    if kind == 3:
+        sc = w.abs().amax(1) / 127
+        q = torch.round(w / sc[:, None]).clamp(-127, 127)
+        pay, w64 = q.to(torch.int8), q.double() * sc.double()[:, None]
+    else:
+        b = w.view(rows, cols // 32, 32)
+        sc = (b.abs().amax(2) / 7).half()
+        q = torch.round(b / sc.float()[..., None]).clamp(-8, 7)
+        u = (q + 8).to(torch.uint8)
+        pay, w64 = u[..., 0::2] | (u[..., 1::2] << 4), (q.double() * sc.double()[..., None]).view(rows, cols)
+    pay, sc = pay.contiguous(), sc.contiguous()
+    x = torch.randn((m, cols), device="cuda", generator=g).bfloat16()
+    torch.cuda.synchronize()
+    wq = dev.qweight_from_device(kind, pay.data_ptr(), sc.data_ptr(), rows, cols)
+    y = torch.empty((m, rows), device="cuda")
+    dev._check(dev._L.tq_qlinear(dev._ctx, C.c_void_p(wq.handle), C.c_void_p(x.data_ptr()), tb.BF16, cols, m, C.c_void_p(y.data_ptr()), tb.F32, rows, C.c_void_p(0)))
+    dev.sync()
+    want = x.double() @ w64.T
+    return ((y.double() - want).norm() / want.norm()).item()
+
+
+# The tensor core truncates every addition of 16 k: 3.4e-9 of the result per addition that an accumulator sees with int8 rows, 1.2e-8 with the
+# two terms of int4 weights (measured, 48 to 512 additions), beside the f32 roundings outside.
+def allowed(kind, additions):
+    return 4e-9 * additions + 6e-8 if kind == 3 else 1.4e-8 * additions + 1e-7
+
+
+@pytest.mark.parametrize("rows,cols", [(14336, 4096), (16384, 2048), (24576, 1536)])
+@pytest.mark.parametrize("m", [129, 144, 160, 192, 193, 384])
+def test_sums_of_two_token_tiles_per_cta(dev, rows, cols, m):
+    """Two accumulators per tile where tensor memory holds them (up to 192 rows), one beyond."""
+    assert sum_error(dev, 3, rows, cols, m) < allowed(3, cols // 16 // (2 if m <= 192 else 1))
