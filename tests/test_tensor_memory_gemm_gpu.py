@@ -137,3 +137,10 @@ def allowed(kind, additions):
 def test_sums_of_two_token_tiles_per_cta(dev, rows, cols, m):
     """Two accumulators per tile where tensor memory holds them (up to 192 rows), one beyond."""
     assert sum_error(dev, 3, rows, cols, m) < allowed(3, cols // 16 // (2 if m <= 192 else 1))
+
+
+@pytest.mark.parametrize("rows", [128, 2304])
+@pytest.mark.parametrize("m", [65, 96, 128, 144, 400])
+def test_sums_of_an_odd_chunk(dev, rows, m):
+    """K = 128, one chunk for two issuers with an accumulator each: half of it for either (1.9e-7 with the chunk in one, 1.2e-7 so)."""
+    assert sum_error(dev, 1, rows, 128, m) < 1.5e-7
