@@ -36,7 +36,20 @@ __device__ __forceinline__ float4 cluster_sum(const float* mine, int n) {
 }
 __device__ __forceinline__ float4 times(float4 v, const float* s) { return make_float4(v.x * s[0], v.y * s[1], v.z * s[2], v.w * s[3]); }
 
-template <int KIND, int TERMS, int DUAL = 0>
+// Adds the accumulators' columns c0 .. c0 + 15 of this warp's lanes up, in their order: number a is issuer a & 1's, which has reached it if it had
+// more than a >> 1 steps (steps0, steps1).
+__device__ __forceinline__ void sum_accumulators(uint32_t tmem_lanes, const UmmaParams& p, int c0, int steps0, int steps1, float (&v)[16]) {
+  float u[16];
+  tmem_ld16(tmem_lanes + (uint32_t)c0, v);
+  for (int a = 1; a < p.n_acc; ++a) {
+    if ((a >> 1) >= ((a & 1) ? steps1 : steps0)) continue;
+    tmem_ld16(tmem_lanes + (uint32_t)(a * p.acc_stride + c0), u);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += u[i];
+  }
+}
+
+template <int KIND, int TERMS, int DUAL = 0, bool RUNS = false>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ UmmaParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -48,6 +61,9 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   // DUAL: the CTA covers two token tiles of p.ntok rows with one conversion of the weights: issuer warp 1 multiplies
   // every stage with the first tile's activations, warp 3 with the second tile's, each into DUAL accumulators
   static_assert(!DUAL || TERMS == 1, "two token tiles per CTA: single-term weights");
+  // RUNS: the sums are cut every p.run_kc chunks: the epilogue's warps add the accumulators up in f32, in shared memory of their own (registers
+  // held over the conversion cost it a tenth), and the issuers start them anew.
+  static_assert(!DUAL || !RUNS, "cut sums: one token tile per CTA");
   constexpr int kTokTiles = DUAL ? 2 : 1;
   // ---- shared-memory carve-up (operand tiles need 1024-byte alignment for the 128-byte swizzle)
   uint8_t* smem = smem_raw;
@@ -58,7 +74,8 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   uint64_t* raw_full = empty + kUmmaMaxStages;                 // [raw stages] packed tiles landed
   uint64_t* raw_empty = raw_full + kUmmaMaxRawStages;             // [raw stages] packed tiles consumed (one arrival per dequant warp)
   uint64_t* acc_full = raw_empty + kUmmaMaxRawStages;             // accumulator complete
-  uint64_t* x_tail = acc_full + 1;                             // a last chunk that both issuers share: its activations landed,
+  uint64_t* acc_free = acc_full + 1;                           // accumulators of a run read (RUNS)
+  uint64_t* x_tail = acc_free + 1;                             // a last chunk that both issuers share: its activations landed,
   uint64_t* a_tail = x_tail + 1;                               // its weights written
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_tail + 1);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -143,6 +160,7 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     }
     if (lane == 0) {
       mbar_init(acc_full, 2);
+      if (RUNS) mbar_init(acc_free, kUmmaDqWarps);
       if (kTail) {
         mbar_init(x_tail, 1);
         mbar_init(a_tail, kUmmaGroupWarps);
@@ -244,8 +262,13 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     int s = DUAL ? 0 : odd, xs = DUAL || KX == 4 ? 0 : odd;     // stage of weights; activation slot
     uint32_t ph = 0, xph = 0, tok_a = 0;
     bool ok = true;
+    int ck = DUAL ? 0 : odd, run = 0;
+    // (run_kc is even: every run but the last has as many chunks for either issuer)
+    for (int run_end = RUNS ? min(p.run_kc, kc_len) : kc_len;; run_end = min(run_end + p.run_kc, kc_len), ++run) {
+    const int ck_end = run_end == kc_len ? kc_len - shared_tail : run_end;
+    j = 0;
 #pragma unroll 1
-    for (int ck = DUAL ? 0 : odd; ck < kc_len - shared_tail; ck += kStep) {
+    for (; ck < ck_end; ck += kStep) {
       ok = mbar_wait_token(&a_full[s], ph, tok_a) && mbar_wait_spin(&x_full[xs], xph);
       if (!ok) { give_up(DERR_FULL_WAIT); break; }
       tc_fence_after();
@@ -292,6 +315,17 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       // thread issues nothing, and here the tensor core already has this chunk's work.
       tok_a = mbar_test(&a_full[s], ph);
     }
+    if (!RUNS || run_end == kc_len || !ok) break;
+    // the run's sums are complete when its products are, and the accumulators the next run's when they have been read
+    if (leader) umma_commit(acc_full);
+    __syncwarp();
+    ok = mbar_wait_spin(acc_free, run & 1);
+    if (!ok) {
+      give_up(DERR_TMEM);
+      break;
+    }
+    tc_fence_after();
+    }
     if (shared_tail && ok) {                     // (slots of two boxes: a chunk each)
       ok = mbar_wait_spin(a_tail, 0) && mbar_wait_spin(x_tail, 0);
       if (!ok) give_up(DERR_FULL_WAIT);
@@ -328,8 +362,18 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     uint64_t* const stage_empty = DUAL ? x_empty + 1 : empty;
     constexpr int kEmptyStep = DUAL ? 2 : 1;
     uint32_t tok_raw = 0, tok_empty = 1;                         // (what is free is free at first)
+    const uint32_t tmem_lanes = tmem_d + ((uint32_t)(32 * q4) << 16);
+    const int col0 = 16 * ((warp - kUmmaFirstDqWarp) >> 2);      // four warps share a lane quarter and alternate over the 16-column chunks
+    constexpr int kColStep = 16 * (kUmmaDqWarps / 4);
+    float* const sums = reinterpret_cast<float*>(raw_s + (size_t)RS * 8 * KT * TB) + 32 * q4 + lane;   // RUNS: the runs so far, [token][128 features]
+    int run = 0;
+    int ck = group;
+    // RUNS: the first group takes a run behind its first chunk of the next one, while the run's last products go on, the second, which converted the
+    // run's last chunk, at once
+    for (int stop = RUNS ? min(p.run_kc + (group ? 0 : kUmmaGroups), kc_len) : kc_len;; stop = min(stop + p.run_kc, kc_len)) {
+    const int from = ck;
 #pragma unroll 1
-    for (int ck = group; ck < kc_len; ck += kUmmaGroups) {
+    for (; ck < stop; ck += kUmmaGroups) {
       // (with two terms the stage is only waited for when the first half of the row is converted:
       // the MMAs that last read it have that long to finish -- decode step at batch 64 8.27 -> 8.11 ms; with one term
       // the conversion is too short for that and the early wait measured 3 % better)
@@ -453,25 +497,49 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         tok_empty = mbar_test(&stage_empty[s * kEmptyStep], ph ^ 1u);
       }
     }
-    if (shared_tail && group == 0 && lane == 0) mbar_arrive(a_tail);   // (the last chunk was this group's)
+    if (shared_tail && stop == kc_len && from < kc_len && group == 0 && lane == 0) mbar_arrive(a_tail);   // (the last chunk was this group's)
+    if (!RUNS || !ok || (run + 1) * p.run_kc >= kc_len) break;
+    ok = __all_sync(0xffffffffu, mbar_wait_spin(acc_full, run & 1));
+    if (!ok) break;
+    tc_fence_after();
+    for (int c0 = col0; c0 < ntok; c0 += kColStep) {
+      float v[16];
+      sum_accumulators(tmem_lanes, p, c0, p.run_kc, p.run_kc, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sums[(c0 + i) * kUmmaRows] = run ? sums[(c0 + i) * kUmmaRows] + v[i] : v[i];
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(acc_free);
+    ++run;
+    }
     // ---- epilogue: D[128 features x ntok tokens] -> y[token][feature]
-    if (ok && !*failed) ok = mbar_wait_spin(acc_full, 0);
+    if (ok && !*failed) ok = mbar_wait_spin(acc_full, run & 1);
     if (!ok) give_up(DERR_TMEM);
     tc_fence_after();
     if (ok) {
       const int n = blockIdx.x * kUmmaRows + 32 * q4 + lane;
-      // two warps share a lane quarter and alternate over the 16-column chunks
+      const int kc_run = RUNS ? kc_len - run * p.run_kc : kc_len;
       for (int tile = 0; tile < kTokTiles; ++tile)
-      for (int c0 = 16 * ((warp - kUmmaFirstDqWarp) >> 2); c0 < ntok; c0 += 16 * (kUmmaDqWarps / 4)) {
-        float v[16], v1[16];
-        tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(tile * p.acc_stride + c0), v);
+      for (int c0 = col0; c0 < ntok; c0 += kColStep) {
+        float v[16];
         const int mt = m0 + tile * p.ntok;                // first token of the tile
-        // (accumulator a: issuer a & 1's number a >> 1, which that issuer has reached if it had that many steps)
-        for (int a = 1; a < (DUAL ? DUAL : p.n_acc); ++a) {
-          if (!DUAL && !shared_tail && (a >> 1) >= 2 * ((kc_len + 1 - (a & 1)) >> 1)) continue;
-          tmem_ld16(tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)((DUAL ? tile * p.acc_stride + a * kUmmaDualAcc : a * p.acc_stride) + c0), v1);
+        if constexpr (DUAL) {
+          float v1[16];
+          tmem_ld16(tmem_lanes + (uint32_t)(tile * p.acc_stride + c0), v);
+          if (DUAL == 2) {
+            tmem_ld16(tmem_lanes + (uint32_t)(tile * p.acc_stride + kUmmaDualAcc + c0), v1);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] += v1[i];
+            for (int i = 0; i < 16; ++i) v[i] += v1[i];
+          }
+        } else {
+          sum_accumulators(tmem_lanes, p, c0, shared_tail ? 2 : 2 * ((kc_run + 1) >> 1), shared_tail ? 2 : 2 * (kc_run >> 1), v);
+        }
+        if constexpr (RUNS) {
+          if (run) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += sums[(c0 + i) * kUmmaRows];
+          }
         }
         if constexpr (KIND == I8_ROW) {
           if (p.splits == 1) {   // (with K split, the scale multiplies the sum of the partials instead)
@@ -664,15 +732,38 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   // error 1.05e-6 with one, 4.3e-7 with two, as with a token tile per CTA; 26 us either way.  (A kernel that can do both costs 2048 rows 2.5 %.)
   const bool two_acc = dual && ntok <= kUmmaDualAcc && w->kind == TQ_I8_ROW && y_dtype == TQ_F32;
   if (two_acc) acc_stride = 2 * kUmmaDualAcc;
+  // Clusters take fewer CTAs along K than there are idle SMs (eight at most, as many as run at once), and token tiles of 128 leave fewer idle than
+  // wider ones would.  f32 results of exact products keep sums as short as an even spread of K over the idle SMs gives (limited where its
+  // partial sums would outweigh the weights): after a run of that many chunks the accumulators are added up in shared memory and start anew.  Not
+  // bf16 results, nor weights rounded to bf16: that rounding is a thousand times the sums' error.
+  // Error, us, uncut -> cut: int4 6144 x 4096 at 64 rows 6.9e-7 -> 3.9e-7, 13.1 -> 14.7; 1024 x 14336 at 48 rows 6.1e-7 -> 2.7e-7, 11.6 -> 13.9;
+  // int8 5120 x 7168 at 144 rows 8.6e-7 -> 2.2e-7, 27.6 -> 32.6.  A cut costs 1 us: the products of the next run wait for it.
+  int run_kc = 0;
+  if (!grp && !dual && y_dtype == TQ_F32 && (terms == 2 || w->kind == TQ_I8_ROW)) {
+    const size_t wide = terms == 2 ? kUmmaTokens : 192;
+    const long long tiles = (long long)(w->rows / kUmmaRows) * (long long)((m + wide - 1) / wide);
+    if (umma_few_tiles(ctx, tiles)) {
+      long long spread = ctx->sm_count / tiles;
+      const long long limit = (long long)(w->tile_bytes / (m * w->rows * 8));
+      if (spread > w->n_kc / 4) spread = w->n_kc / 4;
+      if (spread > 16) spread = 16;
+      if (spread > limit) spread = limit;
+      if (spread < 1) spread = 1;
+      // (two terms and up to 32 rows: four accumulators were enough; eight are there, for twice the chunks)
+      const int kc = (int)((w->n_kc + spread - 1) / spread) * (terms == 2 && n_acc == 8 ? 2 : 1);
+      if (kc < kc_per_split) run_kc = kc < 2 ? 2 : kc & ~1;
+    }
+  }
+  const size_t sum_bytes = run_kc ? (size_t)ntok * kUmmaRows * 4 : 0, ring_budget = budget - sum_bytes;
   // Shared memory: slots of activations (KX boxes of 64 k by one copy; one box with two token tiles), the rest packed tiles, whose bytes
   // in flight hide the latency of HBM: ring slots of KT = 4 k-tiles where two such fit, else 2.
   const int kx = dual ? 1 : ntok <= 64 ? 4 : 2;
   int x_slots = kx == 4 && ntok > 32 ? 3 : 4;
   if (kx == 4 && x_slots > (kc_per_split + 1) / 2) x_slots = (kc_per_split + 1) / 2;
-  if (kx == 2 && (kc_per_split <= 2 || budget < (size_t)x_slots * kx * umma_box_bytes(ntok_stage) + 8 * raw_tile)) x_slots = 2;   // (even: a slot is always the same issuer's)
+  if (kx == 2 && (kc_per_split <= 2 || ring_budget < (size_t)x_slots * kx * umma_box_bytes(ntok_stage) + 8 * raw_tile)) x_slots = 2;   // (even: a slot is always the same issuer's)
   const size_t x_ring = (size_t)x_slots * kx * umma_box_bytes(ntok_stage);
-  if (x_ring + 4 * raw_tile > budget) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: token tile of %d does not fit", ntok);
-  const size_t avail = budget - x_ring;
+  if (x_ring + 4 * raw_tile > ring_budget) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: token tile of %d does not fit", ntok);
+  const size_t avail = ring_budget - x_ring;
   const int kt = avail / (4 * raw_tile) >= 2 ? 4 : 2;
   int raw_stages = (int)(avail / ((size_t)kt * raw_tile));
   if (raw_stages > kUmmaMaxRawStages) raw_stages = kUmmaMaxRawStages;
@@ -703,13 +794,14 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.err = ctx->dev_err;
   p.splits = splits;
   p.kc_per_split = kc_per_split;
+  p.run_kc = run_kc;
   p.y_vec4 = ldy % 4 == 0 && ((uintptr_t)y & (p.y_bf16 ? 7 : 15)) == 0;
   p.stages = stages;
   p.x_slots = x_slots;
   p.kx = kx;
   p.raw_stages = raw_stages;
   p.kt = kt;
-  const size_t smem = umma_smem_bytes(w->kind, x_ring, raw_stages * kt);
+  const size_t smem = umma_smem_bytes(w->kind, x_ring, raw_stages * kt) + sum_bytes;
   if (smem > kSmemMax) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
   dim3 grid((unsigned)(rows_g / kUmmaRows), (unsigned)((m + ntok_stage - 1) / ntok_stage), (unsigned)splits);
   if (grp) {
@@ -729,6 +821,11 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
     else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 1, 1>);
     else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 1, 1>);
     else e = go(qgemm_umma_kernel<Q4_F32, 1, 1>);
+  } else if (run_kc) {
+    if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1, 0, true>);
+    else if (w->kind == TQ_Q4_F16) e = go(qgemm_umma_kernel<Q4_F16, 2, 0, true>);
+    else if (w->kind == TQ_Q8_F32) e = go(qgemm_umma_kernel<Q8_F32, 2, 0, true>);
+    else e = go(qgemm_umma_kernel<Q4_F32, 2, 0, true>);
   } else if (w->kind == TQ_I8_ROW) e = go(qgemm_umma_kernel<I8_ROW, 1>);
   else if (w->kind == TQ_Q4_F16) e = terms == 2 ? go(qgemm_umma_kernel<Q4_F16, 2>) : go(qgemm_umma_kernel<Q4_F16, 1>);
   else if (w->kind == TQ_Q8_F32) e = terms == 2 ? go(qgemm_umma_kernel<Q8_F32, 2>) : go(qgemm_umma_kernel<Q8_F32, 1>);

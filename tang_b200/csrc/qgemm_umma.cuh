@@ -64,6 +64,7 @@ struct UmmaParams {
                           // the second (no K split).  y [M][n_rows / 2] = silu(gate) * up, formed from the f32 sums
   int splits;             // CTAs along K per output tile (gridDim.z): a cluster
   int kc_per_split;       // 128-k tiles per split
+  int run_kc;             // chunks that the accumulators sum before they are added up and start anew (even; 0: all)
   int y_vec4;             // four values of a row of y are stored at once
   const int* g_counts;    // grouped launches (experts stacked by rows): rows of x / y per group, or null
   const int* g_offsets;   // first row of each group

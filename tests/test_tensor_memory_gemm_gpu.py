@@ -127,9 +127,10 @@ def sum_error(dev, kind, rows, cols, m):
 
 
 # The tensor core truncates every addition of 16 k: 3.4e-9 of the result per addition that an accumulator sees with int8 rows, 1.2e-8 with the
-# two terms of int4 weights (measured, 48 to 512 additions), beside the f32 roundings outside.
+# two terms of int4 weights (measured, 48 to 512 additions).  Outside it every f32 addition rounds, 2^-24 / sqrt(3) = 3.4e-8 rms of a partial sum:
+# eight accumulators and eight splits are sixteen such additions, to sums of half the result's variance on average, 3.4e-8 * sqrt(8) = 1e-7.
 def allowed(kind, additions):
-    return 4e-9 * additions + 6e-8 if kind == 3 else 1.4e-8 * additions + 1e-7
+    return (4e-9 if kind == 3 else 1.4e-8) * additions + 1e-7
 
 
 @pytest.mark.parametrize("rows,cols", [(14336, 4096), (16384, 2048), (24576, 1536)])
@@ -144,3 +145,31 @@ def test_sums_of_two_token_tiles_per_cta(dev, rows, cols, m):
 def test_sums_of_an_odd_chunk(dev, rows, m):
     """K = 128, one chunk for two issuers with an accumulator each: half of it for either (1.9e-7 with the chunk in one, 1.2e-7 so)."""
     assert sum_error(dev, 1, rows, 128, m) < 1.5e-7
+
+
+@pytest.mark.parametrize("kind,rows,cols,m,chunks,accumulators", [
+    (1, 6144, 4096, 64, 11, 4), (1, 6144, 4096, 33, 11, 4), (1, 6144, 4096, 96, 11, 2), (1, 2048, 8192, 48, 8, 4), (1, 1024, 14336, 40, 7, 4),
+    (1, 512, 14336, 64, 7, 4), (3, 512, 14336, 20, 7, 8), (3, 1024, 14336, 100, 8, 2), (3, 5120, 7168, 129, 19, 2), (3, 6144, 4096, 192, 16, 2),
+    (3, 7168, 16384, 160, 64, 2), (3, 3072, 7168, 300, 19, 2), (3, 4096, 14336, 320, 56, 2)])
+def test_sums_are_cut_where_clusters_do_not_spread_k(dev, kind, rows, cols, m, chunks, accumulators):
+    """As short as an even spread of K over the idle SMs gives: `chunks` of 128 k into that many accumulators."""
+    assert sum_error(dev, kind, rows, cols, m) < allowed(kind, chunks * 8 * (1 if kind == 3 else 2) // accumulators)
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,cols", [(512, 7168), (640, 9216), (2304, 6272)])
+@pytest.mark.parametrize("m", [17, 40, 70, 130, 200])
+def test_cut_sums(dev, orc, kind, rows, cols, m):
+    """Runs of four to twelve chunks, last runs of one chunk (without one for an issuer, or shared by both), splits that need no cut beside some that do."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(rows + cols + m + kind)
+    sc, pay = make_weight(rng, kind, rows, cols)
+    w = dev.upload_qarrays(kind, pay, sc, rows, cols)
+    xbits, xf = bf16_round(rng.standard_normal((m, cols)).astype(np.float32))
+    want = xf.astype(np.float64) @ weights64(orc, kind, sc, pay, rows, cols).T
+    rms = np.sqrt(np.mean(want * want))
+    x = dev.upload(xbits, tb.BF16)
+    got = [dev.qlinear(x, w, m, tb.F32).to_vec().reshape(m, rows) for _ in range(3)]
+    assert np.abs(got[0] - want).max() < (1e-4 if kind in (0, 2) else 6e-5) * rms
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
