@@ -307,6 +307,14 @@ constexpr int kRtTok = 16, kRtExp = 8;
 // Rows of codes lie 16 bytes apart in the banks, since eight experts' rows are read at once: without, 88 % of the wavefronts of shared
 // memory were conflicts (4096 tokens 127 us against 104).
 __host__ __device__ constexpr int router_code_ld(int runs) { return (runs + 63) / 64 * 64 + 8; }
+constexpr int kRtMaxWidth = 24576;                            // largest d_model
+constexpr size_t router_mma_smem(size_t d) {                  // (the selection's exponentials lie over it)
+  const size_t n = 8 * kRtTok * kRtExp * 12 + (size_t)(kRtTok + kRtExp) * router_code_ld((int)(d + 31) / 32 * 4) * 2, sel = 8 * kMaxExperts * 8;
+  return n > sel ? n : sel;
+}
+// The limit of a kernel's shared memory belongs to the kernel, not to a context: every host thread sets the largest width's.
+constexpr size_t kRtMaxSmem = router_mma_smem(kRtMaxWidth);
+static_assert(kRtMaxSmem <= 227 * 1024, "the widest router does not fit");
 __device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
@@ -675,14 +683,13 @@ static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf1
              "tq_moe_router: need 1 <= top_k <= n_experts <= %d and top_k <= %d", kMaxExperts, kMaxTopK);
   if (n_tokens == 0) return TQ_OK;
   TQ_REQUIRE(ctx, h_bf16_dev && wg_bf16_dev && idx_out_dev && weight_out_dev, "tq_moe_router: null pointer");
-  TQ_REQUIRE(ctx, d_model <= 24576 && d_model % 8 == 0 && ((uintptr_t)h_bf16_dev & 15) == 0 && ((uintptr_t)wg_bf16_dev & 15) == 0,
-             "tq_moe_router: d_model must be a multiple of 8 and at most 24576, arrays 16-byte aligned");
+  TQ_REQUIRE(ctx, d_model <= (size_t)kRtMaxWidth && d_model % 8 == 0 && ((uintptr_t)h_bf16_dev & 15) == 0 && ((uintptr_t)wg_bf16_dev & 15) == 0,
+             "tq_moe_router: d_model must be a multiple of 8 and at most %d, arrays 16-byte aligned", kRtMaxWidth);
   // the f64 tensor-core form where the logits have a place to meet and the token blocks a counter each
-  const size_t mma_smem = 8 * kRtTok * kRtExp * 12 + (size_t)(kRtTok + kRtExp) * router_code_ld(((int)d_model + 31) / 32 * 4) * 2;
   const size_t blocks = (n_tokens + kRtTok - 1) / kRtTok;
-  if (logits_ws && blocks <= (size_t)kTileCounters && mma_smem <= 160 * 1024) {
-    const size_t smem = mma_smem > 8 * kMaxExperts * 8 ? mma_smem : 8 * kMaxExperts * 8;
-    if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(router_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (logits_ws && blocks <= (size_t)kTileCounters) {
+    const size_t smem = router_mma_smem(d_model);
+    if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(router_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRtMaxSmem));
     router_mma_kernel<<<dim3((unsigned)blocks, (unsigned)((n_experts + kRtExp - 1) / kRtExp)), 256, smem, ctx->stream>>>(
         static_cast<const __nv_bfloat16*>(h_bf16_dev), static_cast<const __nv_bfloat16*>(wg_bf16_dev), (int)n_tokens, (int)d_model,
         (int)n_experts, (int)top_k, renormalize, idx_out_dev, weight_out_dev, logits_ws, ctx->dev_err + 1);
@@ -697,7 +704,7 @@ static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf1
   const bool four = n_tokens >= 2048 && 16 * d_model <= 64 * 1024;
   const size_t smem = (four ? 4 : 1) * d_model * 2 * sizeof(unsigned short);
   auto kern = four ? router_kernel<4> : router_kernel<1>;
-  if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, four ? 64 * 1024 : kRtMaxWidth * 4));
   kern<<<dim3((unsigned)((n_tokens + (four ? 3 : 0)) / (four ? 4 : 1)), gy), 256, smem, ctx->stream>>>(
       static_cast<const __nv_bfloat16*>(h_bf16_dev), static_cast<const __nv_bfloat16*>(wg_bf16_dev), (int)n_tokens,
       (int)d_model, (int)n_experts, (int)top_k, renormalize, idx_out_dev, weight_out_dev, logits_ws, ctx->dev_err + 1);

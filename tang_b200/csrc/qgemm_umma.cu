@@ -637,6 +637,8 @@ bool umma_supported(const tq_qweight* w, size_t m) {
 
 // Fewer output tiles than this leave SMs idle, and K is split.
 static bool umma_few_tiles(const tq_ctx* ctx, long long ctas) { return ctas < (ctx->sm_count * 3) / 4; }
+// The limit of a kernel's shared memory belongs to the kernel, not to a context: every host thread sets the same value.
+constexpr int kUmmaMaxSmem = 227 * 1024;
 constexpr int kUmmaTokens = 128;   // token tile: what tensor memory leaves beside the weights
 
 // Whether two-term products of m rows run without a split of K.
@@ -649,18 +651,17 @@ static int umma_clusters(tq_ctx* ctx, int size) {
   int& n = ctx->umma_clusters[size];
   if (n == 0) {
     auto kern = qgemm_umma_kernel<Q4_F16, 2>;
-    constexpr size_t kSmem = 200 * 1024;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, size);
     cfg.blockDim = dim3(kUmmaThreads);
-    cfg.dynamicSmemBytes = kSmem;
+    cfg.dynamicSmemBytes = 200 * 1024;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = (unsigned)size;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaMaxSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = -1;
@@ -681,8 +682,8 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   // The dequantised weights are an operand in tensor memory: per chunk of 128 k and term 64 columns, four stages with one
   // term, two with two terms, i.e. 256 columns; the other 256 hold accumulators, two at least (one per issuing warp): token tiles
   // up to 128, evened out over the tiles.
-  const size_t kSmemMax = 227 * 1024, raw_tile = 8 * (size_t)qk_tile_bytes(w->kind);
-  const size_t budget = kSmemMax - kUmmaHeader - 1024;
+  const size_t raw_tile = 8 * (size_t)qk_tile_bytes(w->kind);
+  const size_t budget = kUmmaMaxSmem - kUmmaHeader - 1024;
   const int ntok_max = kUmmaTokens;
   // Many rows, one term: a CTA takes TWO token tiles (each MMA issuer multiplies every stage with its own tile's
   // activations), so the weights are converted once per 2 x <= 192 tokens; the accumulators are 2 x 192 columns, the
@@ -802,14 +803,14 @@ int launch_qgemm_umma(tq_ctx* ctx, const tq_qweight* w, const void* x_bf16, size
   p.raw_stages = raw_stages;
   p.kt = kt;
   const size_t smem = umma_smem_bytes(w->kind, x_ring, raw_stages * kt) + sum_bytes;
-  if (smem > kSmemMax) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
+  if (smem > kUmmaMaxSmem) return fail(ctx, TQ_EUNSUPPORTED, "tcgen05 GEMM: %zu bytes of shared memory needed", smem);
   dim3 grid((unsigned)(rows_g / kUmmaRows), (unsigned)((m + ntok_stage - 1) / ntok_stage), (unsigned)splits);
   if (grp) {
     grid.y = (unsigned)(m / ntok + (size_t)(grp->max_active < grp->n_groups ? grp->max_active : grp->n_groups));   // (a last tile per group with rows)
     grid.z = 1;
   }
   auto go = [&](auto kern) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kUmmaMaxSmem);
     if (e != cudaSuccess) return e;
     if (splits > 1) return launch_k_cluster(ctx, kern, grid, dim3(kUmmaThreads), smem, dim3(1, 1, splits), map, w_map, p);
     return launch_k(ctx, kern, grid, dim3(kUmmaThreads), smem, map, w_map, p);

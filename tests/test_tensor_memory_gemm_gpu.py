@@ -173,3 +173,47 @@ def test_cut_sums(dev, orc, kind, rows, cols, m):
     got = [dev.qlinear(x, w, m, tb.F32).to_vec().reshape(m, rows) for _ in range(3)]
     assert np.abs(got[0] - want).max() < (1e-4 if kind in (0, 2) else 6e-5) * rms
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+def test_two_threads_with_a_context_each(orc):
+    """The shared-memory limit is the kernel's, not the context's: a thread's launches of large sizes and another's of small ones, with
+    the query for clusters that a context's first narrow product makes, keep out of each other's way.  The router too."""
+    import threading
+
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(5)
+    sc, pay = make_weight(rng, 1, 1024, 2048)
+    sizes = [(1024, 2048, 17), (1024, 2048, 120)]
+    routers = [(64, 512, 8), (64, 24576, 8)]
+    xs = [bf16_round(rng.standard_normal((m, c)).astype(np.float32))[0] for _, c, m in sizes]
+    hs = [bf16_round(rng.standard_normal((t, d)).astype(np.float32))[0] for t, d, _ in routers]
+    wgs = [bf16_round((rng.standard_normal((e, d)) * 0.05).astype(np.float32))[0] for _, d, e in routers]
+    out, errors = [[], []], []
+
+    def work(i, times):
+        try:
+            for _ in range(times):
+                dev = tb.QuantComputeDevice(0)                # (a new context asks for the clusters again)
+                w = dev.upload_qarrays(1, pay, sc, 1024, 2048)
+                x, h, wg = dev.upload(xs[i], tb.BF16), dev.upload(hs[i], tb.BF16), dev.upload(wgs[i], tb.BF16)
+                for _ in range(20):
+                    y = dev.qlinear(x, w, sizes[i][2], tb.F32)
+                    r = tb.moe_router(dev, h, wg, routers[i][0], routers[i][1], routers[i][2], 2)
+                dev.sync()
+                out[i].append((y.to_vec(), r[2]))
+                dev.close()
+        except Exception as e:                                # noqa: BLE001
+            errors.append(e)
+
+    for i in (0, 1):
+        work(i, 1)
+    threads = [threading.Thread(target=work, args=(i, 5)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for o in out:
+        for y, logits in o[1:]:
+            assert np.array_equal(y, o[0][0]) and np.array_equal(logits, o[0][1])
