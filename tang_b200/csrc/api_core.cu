@@ -125,9 +125,6 @@ int tq_ctx_create(int device, void* stream, tq_ctx** out) {
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(TQ_ECUDA);
     ctx->owns_stream = true;
   }
-  if (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&ctx->side_begin, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->side_done, cudaEventDisableTiming) != cudaSuccess)
-    return bail(TQ_ECUDA);
   if (cudaMalloc(&ctx->dev_err, (1 + kTileCounters) * sizeof(int)) != cudaSuccess) return bail(TQ_ECUDA);
   if (cudaMemsetAsync(ctx->dev_err, 0, (1 + kTileCounters) * sizeof(int), ctx->stream) != cudaSuccess) return bail(TQ_ECUDA);
   const size_t ws_bytes = (size_t)kGemvSets * kGemvMaxGrid * 2 * 128 * sizeof(unsigned long long);

@@ -23,7 +23,8 @@ struct tq_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool owns_stream = false;
-  cudaStream_t side = nullptr;   // work that a call runs beside `stream`: begun behind an event of it, joined before the call's last kernel
+  cudaStream_t side = nullptr;   // work that a call runs beside `stream`: begun behind an event of it, joined before the call's last kernel;
+                                 // made with the first layer that has such work
   cudaEvent_t side_begin = nullptr, side_done = nullptr;
   int* dev_err = nullptr;        // device status word written by kernels that give up a bounded wait,
                                  // followed by kTileCounters zeroed tile counters (split-K meets of the dense

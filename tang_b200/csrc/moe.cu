@@ -721,6 +721,20 @@ int tq_moe_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf16_dev, 
                        weight_out_dev, logits_out_dev);
 }
 
+// Whether the context has its side stream; made here unless a capture is open, in which streams are not made.
+static bool side_stream(tq_ctx* ctx) {
+  if (ctx->side) return true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+  if ((ctx->side_begin || cudaEventCreateWithFlags(&ctx->side_begin, cudaEventDisableTiming) == cudaSuccess) &&
+      (ctx->side_done || cudaEventCreateWithFlags(&ctx->side_done, cudaEventDisableTiming) == cudaSuccess) &&
+      cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  ctx->side = nullptr;
+  return false;
+}
+
 int tq_moe_create(tq_ctx* ctx, const tq_moe_config* cfg, const void* wg_bf16_dev, const tq_qweight* w_gate_up_stacked,
                   const tq_qweight* w_down_stacked, const tq_qweight* const* shared_gate_up,
                   const tq_qweight* const* shared_down, tq_moe** out) {
@@ -754,6 +768,7 @@ int tq_moe_create(tq_ctx* ctx, const tq_moe_config* cfg, const void* wg_bf16_dev
     m->sh_gate_up.push_back(shared_gate_up[i]);
     m->sh_down.push_back(shared_down[i]);
   }
+  if (cfg->n_shared) side_stream(ctx);
   *out = m;
   return TQ_OK;
 }
@@ -886,6 +901,7 @@ int tq_moe_ffn(tq_moe* m, const void* h_bf16_dev, size_t n_tokens, float* out_de
     const tq_qweight *gu_w = m->sh_gate_up[i], *dn_w = m->sh_down[i];
     beside = beside && gu_w->rows == 2 * f && gu_w->cols == d && dn_w->rows == d && dn_w->cols == f && umma_supported(gu_w, Ts) && umma_supported(dn_w, Ts);
   }
+  beside = beside && side_stream(ctx);
   if (beside) TQ_CUDA(ctx, cudaEventRecord(ctx->side_begin, ctx->stream));
   TQ_STEP(launch_router(ctx, h, m->wg, T, d, c.n_experts, k, c.renormalize, idx, w, reinterpret_cast<double*>(s + o_lg)));
   if (n <= kPlanPairs) {

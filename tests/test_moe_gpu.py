@@ -267,3 +267,31 @@ def test_token_tiles_of_uneven_experts(dev, orc, E, T):
     scale[1::E // 3] = 40.0
     host.wg_bits, host.wg = bf16_round((host.wg * scale).astype(np.float32))
     check(dev, orc, host, T, seed=E)
+
+
+@pytest.mark.parametrize("T", [5, 40, 300])
+def test_recorded_layer_replays(dev, T):
+    """A layer recorded into a graph, shared experts on the context's side stream among it (40 and 300 tokens), against the same call outside:
+    twice, with other activations in between, and beside a call that is not recorded."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(T)
+    layer = HostMoe(rng, 256, 384, 16, 4, 2).to_device(dev)
+    xs = [dev.upload(bf16_round(rng.standard_normal((T, 256)).astype(np.float32))[0], tb.BF16) for _ in range(2)]
+    want = [layer.forward(x, T).to_vec() for x in xs]
+    x, out = dev.alloc(T * 256, tb.BF16), dev.alloc(T * 256, tb.F32)
+    dev.upload_into(x, xs[0].to_vec())
+    layer.forward(x, T, out=out)
+    dev.sync()
+    dev.begin_capture()
+    layer.forward(x, T, out=out)
+    graph = dev.end_capture()
+    for i in (1, 0, 1):
+        dev.upload_into(x, xs[i].to_vec())
+        graph.launch()
+        if i == 0:
+            assert np.array_equal(layer.forward(xs[1], T).to_vec(), want[1])
+        dev.sync()
+        assert np.array_equal(out.to_vec(), want[i]), i
+    graph.free()
+    layer.destroy()
