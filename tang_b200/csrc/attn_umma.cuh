@@ -31,6 +31,31 @@ __device__ __forceinline__ uint64_t pf_desc_mn(const void* smem_ptr) {
   return (uint64_t)((smem_u32(smem_ptr) >> 4) & 0x3FFF) | (uint64_t)(kPfBox >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
 
+// One row's softmax attention over keys first .. end - 1, key by key in a warp: lane i has values KD i .. of the query and the keys, and 4 i .. of
+// the 128 values' sums.  For the rows of a tile that met, with probability zero, an infinity or a NaN in the values of a key that they do not see: zero
+// times that is NaN.  (Stops when every sum is NaN, as in a row that sees nothing else.)
+template <int KD>
+__device__ __forceinline__ void attend_row(const __nv_bfloat16* k, size_t k_ld, const __nv_bfloat16* v, size_t v_ld, int first, int end, const float (&q)[KD],
+                                           float scale_log2, int lane, float& m, float& l, float (&acc)[4]) {
+#pragma unroll 1
+  for (int key = first; key < end; ++key) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < KD; ++i) s = fmaf(q[i], __bfloat162float(k[(size_t)key * k_ld + KD * lane + i]), s);
+    s = warp_sum(s) * scale_log2;
+    const float mn = fmaxf(m, s), f = ex2(m - mn), w = ex2(s - mn);
+    m = mn;
+    l = l * f + w;
+    bool nan = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[i] = acc[i] * f + w * __bfloat162float(v[(size_t)key * v_ld + 4 * lane + i]);
+      nan = nan && acc[i] != acc[i];
+    }
+    if (__all_sync(0xffffffffu, nan)) break;
+  }
+}
+
 // bf16 [d2][d1][d0] with byte strides, boxes of 64 x b1 x b2 in the 128-byte swizzle; what lies outside reads as zeros.
 inline bool encode_bf16_boxes(CUtensorMap* map, const void* base, size_t d0, size_t d1, size_t d2, size_t stride1, size_t stride2, unsigned b1, unsigned b2) {
   EncodeTiledFn enc = encode_tiled();

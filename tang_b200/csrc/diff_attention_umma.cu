@@ -5,7 +5,8 @@
 // of its rows in tensor memory and finishes the difference and the head norm itself.
 //   warp 0        copies Q once, then K (a box per map) and V tiles of 128 keys
 //   warps 1, 2    issue a map's MMAs: S = Q K^T, then O += (P_hi + P_lo) V
-//   warp 3        zeroes the V rows behind the last key
+//   warp 3        zeroes the V rows behind the last key (where the values of a key that a row of the tiles does not see are not finite, that row is
+//                 formed once more, over its own keys)
 //   warps 4..7, 8..11   softmax of a map, a thread per row, the scores of a tile in registers: the two terms (64 columns each) take their place
 // Only tiles with visible keys are visited: those of the kept first tokens, then those of the window.
 // What bounds it: 2 x (4 + 16) MMAs of 128 x 128 x 16 a tile (about 3100 cycles) against 2 x 128 exponentials a thread (2050).  Prompts of 1024, 820,
@@ -27,8 +28,9 @@ struct DiffUmmaParams {
   DiffAttn a;
   RaggedBatch b;
   int group;
+  const __nv_bfloat16 *q, *k, *v;
   __nv_bfloat16* out;
-  long long ldo;
+  long long ldq, ldo;
   int* err;
 };
 
@@ -304,6 +306,32 @@ diff_attention_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
           y[j] = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
+      unsigned rows = __ballot_sync(0xffffffffu, live && !(fabsf(sqs) <= FLT_MAX));
+      const size_t ke = (size_t)p.a.kv_heads * 128, ve = (size_t)p.a.kv_heads * kDuaV;
+      while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const int at = row0 + __shfl_sync(0xffffffffu, qi, src), pos = __shfl_sync(0xffffffffu, qpos, src), h = __shfl_sync(0xffffffffu, head, src);
+        const int lo = max(0, pos - p.a.window + 1), kept = min(p.a.keep_first, lo);
+        const __nv_bfloat16* vb = p.v + (size_t)seq0 * ve + (size_t)kvh * kDuaV;
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f;
+#pragma unroll 1
+        for (int mp = 0; mp < 2; ++mp) {
+          const __nv_bfloat16* kb = p.k + (size_t)seq0 * ke + (size_t)kvh * 128 + 64 * mp;
+          float qr[2], rm = -FLT_MAX, rl = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 2; ++i) qr[i] = __bfloat162float(p.q[(size_t)at * p.ldq + (size_t)h * 128 + 64 * mp + 2 * lane + i]);
+          attend_row(kb, ke, vb, ve, 0, kept, qr, sl2, lane, rm, rl, acc);
+          attend_row(kb, ke, vb, ve, lo, pos + 1, qr, sl2, lane, rm, rl, acc);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sum[i] = mp ? sum[i] - acc[i] * (p.a.lambda / rl) : acc[i] * (1.0f / rl);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq += sum[i] * sum[i];
+        const float rinv = p.a.out_scale / sqrtf(warp_sum(sq) / (float)kDuaV + p.a.eps);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p.out[(size_t)at * p.ldo + (size_t)h * kDuaV + 4 * lane + i] = __float2bfloat16_rn(sum[i] * rinv);
+      }
     }
   }
   tc_fence_before();
@@ -324,6 +352,10 @@ int launch_diff_attention_umma(tq_ctx* ctx, const DiffAttn& a, const RaggedBatch
   p.a = a;
   p.b = b;
   p.group = a.heads / a.kv_heads;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.ldq = (long long)ldq;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.ldo = (long long)ldo;
   p.err = ctx->dev_err;

@@ -4,7 +4,8 @@
 // A CTA takes two query tiles of 128 rows (128 / group positions x the group's heads of one KV head) over the same key tiles of 128:
 //   warp 0        copies Q once, then K and V tiles (two stages)
 //   warps 1, 2    issue a query tile's MMAs: S = Q K^T (both from shared memory), then O += P V (P from tensor memory, V N-major)
-//   warp 3        zeroes the V rows behind the last key (whatever the cache holds there must not meet a probability of zero)
+//   warp 3        zeroes the V rows behind the last key (whatever the cache holds there must not meet a probability of zero; where the values of a
+//                 later key of the chunk are not finite, the rows before it are formed once more, over their own keys)
 //   warps 4..7, 8..11   softmax of a query tile, a thread per row: maximum, probabilities over the scores' columns, and, only where a
 //                 row's maximum grew, a rescaling of O (a reference that may lag behind the maximum would save a tenth of the time, but
 //                 then the largest probability is no longer 1, which bf16 holds exactly: errors against 64 bits 1.50e-3 -> 1.65e-3)
@@ -30,6 +31,8 @@ struct PrefillUmmaParams {
   const int* cache_start;
   int q_len, n_heads, n_kv, group, rows_max;          // rows_max: positions that a sequence's cache holds
   float scale_log2;
+  const __nv_bfloat16 *q, *k, *v;
+  size_t seq_stride;
   void* out;
   int out_f32;
   int* err;
@@ -256,11 +259,14 @@ gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
     if (ok && n) {
       const float inv = l > 0.f ? 1.0f / l : 0.f;
       const size_t at = (((size_t)b * p.q_len + (live ? pos : 0)) * p.n_heads + head) * kPfHd;
+      float zero = 0.f;                               // NaN if some sum is not finite
 #pragma unroll 1
       for (int c = 0; c < kPfHd; c += 32) {
         float o[32];
         pf_ld32(o_t + (uint32_t)c, o);
         if (!live) continue;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) zero = fmaf(o[j], 0.f, zero);
         if (p.out_f32) {
           float4* y = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at + c);
 #pragma unroll
@@ -276,6 +282,33 @@ gqa_prefill_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_
               w[e] = *reinterpret_cast<const uint32_t*>(&h);
             }
             y[j] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+      unsigned rows = __ballot_sync(0xffffffffu, live && zero != zero);
+      if (rows) {
+        // Keys that rows of this CTA do not see and their tiles hold: from its first position on.
+        const size_t ld = (size_t)p.n_kv * kPfHd;
+        const __nv_bfloat16 *kb = p.k + (size_t)b * p.seq_stride + (size_t)kvh * kPfHd, *vb = p.v + (size_t)b * p.seq_stride + (size_t)kvh * kPfHd;
+        float z = 0.f;
+        for (int key = start + pos0 + 1; key < k_end; ++key)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) z = fmaf(__bfloat162float(vb[(size_t)key * ld + 4 * lane + i]), 0.f, z);
+        if (!__any_sync(0xffffffffu, z != z)) rows = 0u;
+        while (rows) {
+          const int src = __ffs(rows) - 1;
+          rows &= rows - 1;
+          const int row_limit = __shfl_sync(0xffffffffu, limit, src);
+          const size_t row_at = __shfl_sync(0xffffffffu, (unsigned long long)at, src) + 4 * lane;
+          float qr[4], rm = -FLT_MAX, rl = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) qr[i] = __bfloat162float(p.q[row_at + i]);
+          attend_row(kb, ld, vb, ld, 0, row_limit + 1, qr, p.scale_log2, lane, rm, rl, acc);
+          const float rinv = rl > 0.f ? 1.0f / rl : 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (p.out_f32) static_cast<float*>(p.out)[row_at + i] = acc[i] * rinv;
+            else static_cast<__nv_bfloat16*>(p.out)[row_at + i] = __float2bfloat16_rn(acc[i] * rinv);
           }
         }
       }
@@ -301,6 +334,10 @@ int launch_gqa_prefill_umma(tq_ctx* ctx, const void* q, const void* k, const voi
   p.group = (int)group;
   p.rows_max = (int)rows_max;
   p.scale_log2 = scale * 1.44269504088896340736f;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.seq_stride = seq_stride;
   p.out = out;
   p.out_f32 = out_f32;
   p.err = ctx->dev_err;

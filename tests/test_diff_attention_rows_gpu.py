@@ -15,7 +15,8 @@ dev = D.dev
 class Aligned(D.Case):
     """As Case, with result rows that are 16-byte aligned."""
 
-    def run(self, dev, dtype, poison=True):
+    def run(self, dev, dtype, poison=True, bits_of=0x7FC0):
+        """bits_of: what stands for a NaN in bf16."""
         import tang_b200 as tb
 
         n_slots = len(self.seqs) + 2
@@ -29,7 +30,7 @@ class Aligned(D.Case):
             cache_row += range(s * self.max_seq + start, s * self.max_seq + start + n)
         counts = [n for _, n in self.seqs]
         q = np.concatenate([x.reshape(x.shape[0], -1) for x in self.q])
-        bits = lambda a: np.where(np.isnan(a), np.uint16(0x7FC0), bf16_round(np.nan_to_num(a))[0])
+        bits = lambda a: np.where(np.isnan(a), np.uint16(bits_of), bf16_round(np.nan_to_num(a))[0])
         up = (lambda a: dev.upload(bits(np.ascontiguousarray(a)), tb.BF16)) if dtype == tb.BF16 else dev.upload
         qb, kb, vb = up(q), up(kc), up(vc)
         i32 = lambda a: dev.upload(np.asarray(a, np.int32), tb.I32)
@@ -82,3 +83,24 @@ def test_one_map_behind_the_other(dev, tiles, grows):
         case.k[b][:, 0, grows] = bf16_round((u / np.dot(u, u) / case.scale * (np.arange(n) / 32)[:, None]).astype(np.float32))[1]
         case.k[b][:, 0, 1 - grows] = bf16_round(case.k[b][:, 0, 1 - grows] * 0.05)[1]
     D.check(dev, case, rows=[0, 1, 64, 122])
+
+
+@pytest.mark.parametrize("window,keep,start", [(100, 3, 0), (64, 0, 200), (2000, 0, 0), (130, 140, 150)])
+@pytest.mark.parametrize("bits", [0x7F80, 0x7FC0])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(dev, window, keep, start, bits):
+    """One key whose values hold an infinity or a NaN: the queries before it, and those behind its window, share tiles with it and do not see it."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(window)
+    case = Aligned(rng, 8, 1, 64, 128, window, keep, seqs=[(start, 260)], max_seq=start + 260)
+    bad = start + 141
+    case.v[0][bad, 0, 17] = np.nan
+    got = case.run(dev, tb.BF16, bits_of=bits)[0]
+    pos = start + np.arange(260)
+    sees = (pos >= bad) & ((pos - bad < window) | (bad < keep))
+    assert np.array_equal(np.isnan(got).any(axis=(1, 2)), sees)
+    case.v[0][bad, 0, 17] = 0
+    rows = [i for i in (0, 127, 128, 140, 141 + window, 200 + window, 259) if i < 260 and not sees[i]]
+    want = case.want(0, rows)
+    rms = np.sqrt(np.mean(want ** 2))
+    assert np.abs(got[rows] - want).max() < 6e-3 * max(rms, np.abs(want).max())

@@ -57,3 +57,36 @@ def test_a_chunk_beyond_the_cache_is_reported(dev):
     with pytest.raises(tb.TangqError):
         dev.sync()
     dev.sync()
+
+
+@pytest.mark.parametrize("nh,nkv,q_len,start", [(8, 2, 320, 0), (8, 8, 1024, 3), (8, 1, 200, 100)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them(dev, orc, nh, nkv, q_len, start, f32):
+    """An infinity and a NaN in the values of two keys of the chunk: the positions before each do not see it, though they share tiles with it."""
+    import tang_b200 as tb
+
+    hd, per = 128, 256 // (nh // nkv)
+    rng = np.random.default_rng(q_len)
+    n = start + q_len
+    qb, qf = bf16_round(rng.standard_normal((q_len, nh * hd)).astype(np.float32))
+    kb, kf = bf16_round(rng.standard_normal((n, nkv * hd)).astype(np.float32))
+    vb, vf = bf16_round(rng.standard_normal((n, nkv * hd)).astype(np.float32))
+    at_inf, at_nan = start + per - 2, start + per + per // 2
+    vb[at_inf, 5::hd], vf[at_inf, 5::hd] = 0x7F80, np.inf
+    vb[at_nan, 9::hd], vf[at_nan, 9::hd] = 0x7FC0, np.nan
+    got = dev.gqa_prefill(dev.upload(qb, tb.BF16), dev.upload(kb, tb.BF16), dev.upload(vb, tb.BF16), np.array([start], np.int32), 1, q_len, nh, nkv, hd,
+                          n * nkv * hd, out_dtype=tb.F32 if f32 else tb.BF16).to_vec().reshape(q_len, nh, hd)
+    dev.sync()
+    if not f32:
+        got = (got.astype(np.uint32) << 16).view(np.float32)
+    pos = start + np.arange(q_len)
+    sees = np.zeros((q_len, hd), bool)
+    sees[pos >= at_inf, 5] = True
+    sees[pos >= at_nan, 9] = True
+    assert np.array_equal(~np.isfinite(got), np.broadcast_to(sees[:, None], got.shape))
+    assert (got[pos >= at_inf, :, 5] == np.inf).all() and np.isnan(got[pos >= at_nan, :, 9]).all()
+    vf[at_inf, 5::hd] = vf[at_nan, 9::hd] = 0
+    for i in sorted({0, per - 3, per - 2, per - 1, per, at_nan - start - 1, at_nan - start, q_len - 1}):
+        want = orc.attention_decode_f64(qf[i], kf[:start + i + 1], vf[:start + i + 1], start + i + 1, nh, nkv, hd).reshape(nh, hd)
+        g = np.where(sees[i], want, got[i])
+        assert rel_err(g, want, floor_frac=1.0) < 1e-2, i
