@@ -129,7 +129,7 @@ __device__ __noinline__ double router_ordered_sum(const unsigned short* hrow_s, 
 // TT tokens per CTA share every load of a gate row (many tokens: the rows then come from L2 once per TT tokens).
 template <int TT>
 __global__ void __launch_bounds__(256, 4) router_kernel(const __nv_bfloat16* h, const __nv_bfloat16* wg, int T, int d, int E,
-                                                     int top_k, int renorm, int* idx_out, float* w_out, double* logits_out, int* counters) {
+                                                     int top_k, int renorm, int* idx_out, float* w_out, double* logits_out) {
   extern __shared__ __align__(16) unsigned short hs[];   // [TT][d] activations (bf16 bits), then [TT][d] their ulp codes
   __shared__ double lg[TT][kMaxExperts];
   unsigned short* he = hs + (size_t)TT * d;
@@ -141,9 +141,7 @@ __global__ void __launch_bounds__(256, 4) router_kernel(const __nv_bfloat16* h, 
     *reinterpret_cast<unsigned*>(he + i) = bf16x2_ulp_code(pair);
   }
   __syncthreads();
-  // gridDim.y CTAs share a token's experts (few tokens would otherwise occupy few SMs); the CTA that
-  // finishes last (counter) reads all logits back and makes the selection
-  for (int e = blockIdx.y * 8 + warp; e < E; e += 8 * gridDim.y) {
+  for (int e = warp; e < E; e += 8) {
     const unsigned short* wrow = reinterpret_cast<const unsigned short*>(wg) + (size_t)e * d;
     double acc[TT];
     float sabs[TT];
@@ -202,20 +200,6 @@ __global__ void __launch_bounds__(256, 4) router_kernel(const __nv_bfloat16* h, 
         if (logits_out) logits_out[(size_t)(t0 + tt) * E + e] = acc[tt];
       }
     }
-  }
-  if (gridDim.y > 1) {
-    __shared__ int last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      last = atomicAdd(&counters[blockIdx.x], 1) == (int)gridDim.y - 1;
-      if (last) counters[blockIdx.x] = 0;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int i = threadIdx.x; i < TT * E; i += blockDim.x)
-      if (t0 + i / E < T) lg[i / E][i % E] = __ldcg(logits_out + (size_t)t0 * E + i);
   }
   __syncthreads();
   for (int tt = 0; tt < TT && t0 + tt < T; ++tt) {
@@ -674,8 +658,7 @@ using namespace tq;
 
 extern "C" {
 
-// logits_ws: [n_tokens][n_experts] f64 that the kernel may use to share logits between the CTAs of a token
-// (null: one CTA per token).
+// logits_ws: [n_tokens][n_experts] f64, where the logits go and the CTAs of a token block meet (null: one CTA has a token's experts).
 static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf16_dev, size_t n_tokens, size_t d_model,
                          size_t n_experts, size_t top_k, int renormalize, int* idx_out_dev, float* weight_out_dev,
                          double* logits_ws) {
@@ -697,17 +680,15 @@ static int launch_router(tq_ctx* ctx, const void* h_bf16_dev, const void* wg_bf1
     TQ_CUDA(ctx, cudaGetLastError());
     return TQ_OK;
   }
-  unsigned gy = 1;
-  if (logits_ws && n_tokens <= 64 && n_tokens <= (size_t)kTileCounters) gy = (unsigned)((n_experts + 7) / 8);
-  // (without them) four tokens per CTA once there are several waves of CTAs anyway (their activations and ulp codes: 16 d bytes;
-  // measured alone at 1000 / 2048 tokens: 154 / 209 us against 119 / 206 us with one token per CTA)
+  // Without them, or with more token blocks than counters: a CTA has all experts of its tokens, four tokens once there are several waves of CTAs
+  // anyway (their activations and ulp codes: 16 d bytes; measured alone at 1000 / 2048 tokens: 154 / 209 us against 119 / 206 us with one)
   const bool four = n_tokens >= 2048 && 16 * d_model <= 64 * 1024;
   const size_t smem = (four ? 4 : 1) * d_model * 2 * sizeof(unsigned short);
   auto kern = four ? router_kernel<4> : router_kernel<1>;
   if (smem > 48 * 1024) TQ_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, four ? 64 * 1024 : kRtMaxWidth * 4));
-  kern<<<dim3((unsigned)((n_tokens + (four ? 3 : 0)) / (four ? 4 : 1)), gy), 256, smem, ctx->stream>>>(
+  kern<<<(unsigned)((n_tokens + (four ? 3 : 0)) / (four ? 4 : 1)), 256, smem, ctx->stream>>>(
       static_cast<const __nv_bfloat16*>(h_bf16_dev), static_cast<const __nv_bfloat16*>(wg_bf16_dev), (int)n_tokens,
-      (int)d_model, (int)n_experts, (int)top_k, renormalize, idx_out_dev, weight_out_dev, logits_ws, ctx->dev_err + 1);
+      (int)d_model, (int)n_experts, (int)top_k, renormalize, idx_out_dev, weight_out_dev, logits_ws);
   ctx->launches++;
   TQ_CUDA(ctx, cudaGetLastError());
   return TQ_OK;

@@ -295,3 +295,61 @@ def test_recorded_layer_replays(dev, T):
         assert np.array_equal(out.to_vec(), want[i]), i
     graph.free()
     layer.destroy()
+
+
+def _router_without_logits(dev, h, wg, T, d, E, k, renorm=0):
+    """The form for callers that give no room for the logits."""
+    import ctypes as C
+
+    import tang_b200 as tb
+
+    idx, w = dev.alloc(T * k, tb.I32), dev.alloc(T * k, tb.F32)
+    dev._check(dev._L.tq_moe_router(dev._ctx, C.c_void_p(h.ptr), C.c_void_p(wg.ptr), T, d, E, k, renorm, C.c_void_p(idx.ptr), C.c_void_p(w.ptr), C.c_void_p(0)))
+    dev.sync()
+    return idx.to_vec().reshape(T, k), w.to_vec().reshape(T, k)
+
+
+@pytest.mark.parametrize("T,d,E,k,renorm", [(1, 40, 2, 2, 0), (70, 2048, 64, 6, 1), (2049, 264, 61, 16, 0), (2100, 4104, 9, 1, 0)])
+def test_router_without_logits_makes_the_same_choices(dev, T, d, E, k, renorm):
+    """One and four tokens per CTA; rows that round, an infinity and a NaN among them."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(T + d)
+    h = rng.standard_normal((T, d)).astype(np.float32)
+    h[T // 2, d // 2] = 1e-30
+    bits = bf16_round(h)[0]
+    if T > 1:
+        bits[3, 1], bits[T - 1, d - 1] = 0x7F80, 0x7FC0
+    hb, wb = dev.upload(bits, tb.BF16), dev.upload(bf16_round((rng.standard_normal((E, d)) * 0.05).astype(np.float32))[0], tb.BF16)
+    want_i, want_w, _ = tb.moe_router(dev, hb, wb, T, d, E, k, bool(renorm))
+    idx, w = _router_without_logits(dev, hb, wb, T, d, E, k, renorm)
+    assert np.array_equal(idx, want_i) and np.array_equal(w, want_w, equal_nan=True)
+
+
+def test_router_of_more_tokens_than_counters(dev):
+    """More than 16 x 1024 tokens take the other router, with the logits written too."""
+    import tang_b200 as tb
+
+    T, d, E, k = 16400, 64, 5, 2
+    rng = np.random.default_rng(4)
+    bits = bf16_round(rng.standard_normal((T, d)).astype(np.float32))[0]
+    wb = dev.upload(bf16_round((rng.standard_normal((E, d)) * 0.05).astype(np.float32))[0], tb.BF16)
+    whole = tb.moe_router(dev, dev.upload(bits, tb.BF16), wb, T, d, E, k)
+    parts = [tb.moe_router(dev, dev.upload(bits[t:t + 8200], tb.BF16), wb, 8200, d, E, k) for t in (0, 8200)]
+    for a, b in zip(whole, zip(*parts)):
+        assert np.array_equal(a, np.concatenate(b))
+
+
+def test_plan_of_more_pairs_than_one_cta_takes(dev):
+    """More than 32768 (token, choice) pairs: local ids, counts and slots in kernels of their own; the same tokens in two halves take one."""
+    import tang_b200 as tb
+
+    rng = np.random.default_rng(9)
+    layer = HostMoe(rng, 128, 128, 8, 4, 1).to_device(dev)
+    T = 8200
+    bits, _ = bf16_round(rng.standard_normal((T, 128)).astype(np.float32))
+    whole = layer.forward(dev.upload(bits, tb.BF16), T).to_vec().reshape(T, 128)
+    parts = np.concatenate([layer.forward(dev.upload(bits[t:t + 4100], tb.BF16), 4100).to_vec().reshape(-1, 128) for t in (0, 4100)])
+    worst, share = rel_err_profile(whole, parts)
+    assert worst < 1e-2 and share < 5e-3, (worst, share)
+    layer.destroy()
