@@ -217,3 +217,32 @@ def test_two_threads_with_a_context_each(orc):
     for o in out:
         for y, logits in o[1:]:
             assert np.array_equal(y, o[0][0]) and np.array_equal(logits, o[0][1])
+
+
+def test_first_products_of_a_process_from_four_threads():
+    """Each thread's first call asks for what the process looks up once; no thread may find the answer missing.  (A process of its own: here the
+    question has been asked.)"""
+    import subprocess
+    import sys
+
+    code = """
+import threading, numpy as np, tang_b200 as tb
+errors, gate = [], threading.Barrier(4)
+def work():
+    try:
+        dev = tb.QuantComputeDevice(0)
+        w = dev.upload_qarrays(1, np.zeros((128, 128), np.uint8), np.zeros((128, 8), np.uint16), 128, 256)
+        x = dev.upload(np.zeros((64, 256), np.uint16), tb.BF16)
+        dev.sync()
+        gate.wait()
+        dev.qlinear(x, w, 64, tb.F32)
+        dev.sync()
+    except Exception as e:
+        errors.append(e)
+        gate.abort()
+ts = [threading.Thread(target=work) for _ in range(4)]
+[t.start() for t in ts]; [t.join() for t in ts]
+assert not errors, errors
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
