@@ -27,7 +27,8 @@ int launch_qgemm_grouped(tq_ctx* ctx, const tq_qweight* w, int n_groups, const v
                          int max_active = 0, size_t total_rows = 0);
 
 // Rows per expert, when routing is even, from which the experts' products are the tcgen05 kernel's (the other kernel reads an expert's weights
-// once per eight rows).  64 experts, 6 chosen, d 2048, f 1408, two shared experts, us (qgemm_skg, tcgen05): 96 tokens 202, 253, 128 294, 253, 192 406, 273.
+// once per eight rows).  64 experts, 6 chosen, d 2048, f 1408, two shared experts, us (qgemm_skg, tcgen05): 96 tokens 202, 253, 128 294, 253, 192 406, 273;
+// the dispatching form, whose gate and up do not meet in the epilogue: 128 tokens 367, 329, 192 477, 343, 224 486, 356.
 constexpr size_t kTensorRows = 12;
 constexpr int kMaxExperts = 256;
 constexpr int kMaxTopK = 16;
@@ -519,7 +520,8 @@ __global__ void moe_count_kernel(const int* idx, int n, int E, int* counts, int*
 }
 
 // Few (token, choice) pairs: local ids, counts, offsets, the list of groups with rows and the slots in one CTA (three launches of 2 to 3 us each
-// otherwise; up to 32768 pairs its two passes are no longer than theirs: under ncu 384 pairs 10.8 -> 3.8 us, 24576 28 -> 17).
+// otherwise; up to 32768 pairs its two passes are no longer than theirs: under ncu 384 pairs 10.8 -> 3.8 us, 24576 28 -> 17.  With experts over eight
+// ranks, where seven of eight pairs fall into one bucket, the layer takes, three launches -> one: 384 pairs 123 -> 116 us, 12288 231 -> 223, 32766 505 -> 484).
 constexpr size_t kPlanPairs = 32768;
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* idx, int n, int lo, int n_local, int* idx_local, int* counts, int* offsets, int* active,
                                                         int* slot) {
