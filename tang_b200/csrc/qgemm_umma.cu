@@ -265,66 +265,66 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     int ck = DUAL ? 0 : odd, run = 0;
     // (run_kc is even: every run but the last has as many chunks for either issuer)
     for (int run_end = RUNS ? min(p.run_kc, kc_len) : kc_len;; run_end = min(run_end + p.run_kc, kc_len), ++run) {
-    const int ck_end = run_end == kc_len ? kc_len - shared_tail : run_end;
-    j = 0;
+      const int ck_end = run_end == kc_len ? kc_len - shared_tail : run_end;
+      j = 0;
 #pragma unroll 1
-    for (; ck < ck_end; ck += kStep) {
-      ok = mbar_wait_token(&a_full[s], ph, tok_a) && mbar_wait_spin(&x_full[xs], xph);
-      if (!ok) { give_up(DERR_FULL_WAIT); break; }
-      tc_fence_after();
-      const uint64_t xd = desc0 + (uint64_t)((uint32_t)xs * slot_u);
-      const uint32_t a_t0 = tmem_d + (uint32_t)(p.a_col0 + s * (64 * TERMS));
+      for (; ck < ck_end; ck += kStep) {
+        ok = mbar_wait_token(&a_full[s], ph, tok_a) && mbar_wait_spin(&x_full[xs], xph);
+        if (!ok) { give_up(DERR_FULL_WAIT); break; }
+        tc_fence_after();
+        const uint64_t xd = desc0 + (uint64_t)((uint32_t)xs * slot_u);
+        const uint32_t a_t0 = tmem_d + (uint32_t)(p.a_col0 + s * (64 * TERMS));
 #pragma unroll
-      for (int half = 0; half < 2; ++half, ++j) {
-        if (DUAL && half == 1) {
-          ok = mbar_wait_spin(&x_full[xs + 1], xph);
-          if (!ok) { give_up(DERR_FULL_WAIT); break; }
-        }
-        const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride) + (DUAL == 2 ? (uint32_t)(half * kUmmaDualAcc) : 0u);
-        const uint32_t fresh = (DUAL ? j < DUAL : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
-        if (leader) {
-#pragma unroll
-          for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
-            const uint64_t bd = xd + half * half_u + 2 * k16;
-            // 32 columns (64 k) of the hi term, then 32 of the lo term
-            const uint32_t a_t = a_t0 + (uint32_t)(half * (32 * TERMS) + 8 * k16);
-            umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
-            if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
+        for (int half = 0; half < 2; ++half, ++j) {
+          if (DUAL && half == 1) {
+            ok = mbar_wait_spin(&x_full[xs + 1], xph);
+            if (!ok) { give_up(DERR_FULL_WAIT); break; }
           }
-          // (commits arrive when the MMAs so far have finished reading)
-          if (DUAL) umma_commit(&x_empty[xs + half]);
+          const uint32_t acc = tmem_d + (uint32_t)((DUAL ? odd : odd + 2 * (j & rot_mask)) * p.acc_stride) + (DUAL == 2 ? (uint32_t)(half * kUmmaDualAcc) : 0u);
+          const uint32_t fresh = (DUAL ? j < DUAL : j <= rot_mask) ? 0u : 1u;   // the accumulator's first step overwrites it
+          if (leader) {
+#pragma unroll
+            for (int k16 = 0; k16 < kUmmaK / 16; ++k16) {
+              const uint64_t bd = xd + half * half_u + 2 * k16;
+              // 32 columns (64 k) of the hi term, then 32 of the lo term
+              const uint32_t a_t = a_t0 + (uint32_t)(half * (32 * TERMS) + 8 * k16);
+              umma_f16_ts(acc, a_t, bd, idesc, fresh | (k16 != 0));
+              if (TERMS == 2) umma_f16_ts(acc, a_t + 32u, bd, idesc, 1u);
+            }
+            // (commits arrive when the MMAs so far have finished reading)
+            if (DUAL) umma_commit(&x_empty[xs + half]);
+          }
         }
+        if (!ok) break;
+        if (!DUAL && leader) {
+          umma_commit(&empty[s]);
+          umma_commit(&x_empty[xs]);
+        }
+        __syncwarp();
+        xs += x_step;
+        if (xs >= XS) {
+          xs -= XS;
+          xph ^= 1u;
+        }
+        s += kStep;
+        if (s >= S) {
+          s -= S;
+          ph ^= 1u;
+        }
+        // Look at the next chunk's barrier only now: the answer takes ~70 cycles, during which an in-order
+        // thread issues nothing, and here the tensor core already has this chunk's work.
+        tok_a = mbar_test(&a_full[s], ph);
       }
-      if (!ok) break;
-      if (!DUAL && leader) {
-        umma_commit(&empty[s]);
-        umma_commit(&x_empty[xs]);
-      }
+      if (!RUNS || run_end == kc_len || !ok) break;
+      // the run's sums are complete when its products are, and the accumulators the next run's when they have been read
+      if (leader) umma_commit(acc_full);
       __syncwarp();
-      xs += x_step;
-      if (xs >= XS) {
-        xs -= XS;
-        xph ^= 1u;
+      ok = mbar_wait_spin(acc_free, run & 1);
+      if (!ok) {
+        give_up(DERR_TMEM);
+        break;
       }
-      s += kStep;
-      if (s >= S) {
-        s -= S;
-        ph ^= 1u;
-      }
-      // Look at the next chunk's barrier only now: the answer takes ~70 cycles, during which an in-order
-      // thread issues nothing, and here the tensor core already has this chunk's work.
-      tok_a = mbar_test(&a_full[s], ph);
-    }
-    if (!RUNS || run_end == kc_len || !ok) break;
-    // the run's sums are complete when its products are, and the accumulators the next run's when they have been read
-    if (leader) umma_commit(acc_full);
-    __syncwarp();
-    ok = mbar_wait_spin(acc_free, run & 1);
-    if (!ok) {
-      give_up(DERR_TMEM);
-      break;
-    }
-    tc_fence_after();
+      tc_fence_after();
     }
     if (shared_tail && ok) {                     // (slots of two boxes: a chunk each)
       ok = mbar_wait_spin(a_tail, 0) && mbar_wait_spin(x_tail, 0);
@@ -371,147 +371,147 @@ qgemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
     // RUNS: the first group takes a run behind its first chunk of the next one, while the run's last products go on, the second, which converted the
     // run's last chunk, at once
     for (int stop = RUNS ? min(p.run_kc + (group ? 0 : kUmmaGroups), kc_len) : kc_len;; stop = min(stop + p.run_kc, kc_len)) {
-    const int from = ck;
+      const int from = ck;
 #pragma unroll 1
-    for (; ck < stop; ck += kUmmaGroups) {
-      // (with two terms the stage is only waited for when the first half of the row is converted:
-      // the MMAs that last read it have that long to finish -- decode step at batch 64 8.27 -> 8.11 ms; with one term
-      // the conversion is too short for that and the early wait measured 3 % better)
-      constexpr bool kLateWait = TERMS == 2;
-      ok = mbar_wait_token(&raw_full[r], rph, tok_raw) && (kLateWait || mbar_wait_token(&stage_empty[s * kEmptyStep], ph ^ 1u, tok_empty));
-      if (!ok) { give_up(DERR_FULL_WAIT); break; }
-      const int s_cur = s, r_cur = r, within_cur = within;
-      const uint32_t ph_cur = ph;
-      s += kUmmaGroups;
-      if (s >= S) {
-        s -= S;
-        ph ^= 1u;
-      }
-      within += kUmmaGroups;
-      const bool leaves = within >= KT;           // this group's next tile lies in the next ring slot
-      if (leaves) {
-        within -= KT;
-        if (++r == RS) {
-          r = 0;
-          rph ^= 1u;
+      for (; ck < stop; ck += kUmmaGroups) {
+        // (with two terms the stage is only waited for when the first half of the row is converted:
+        // the MMAs that last read it have that long to finish -- decode step at batch 64 8.27 -> 8.11 ms; with one term
+        // the conversion is too short for that and the early wait measured 3 % better)
+        constexpr bool kLateWait = TERMS == 2;
+        ok = mbar_wait_token(&raw_full[r], rph, tok_raw) && (kLateWait || mbar_wait_token(&stage_empty[s * kEmptyStep], ph ^ 1u, tok_empty));
+        if (!ok) { give_up(DERR_FULL_WAIT); break; }
+        const int s_cur = s, r_cur = r, within_cur = within;
+        const uint32_t ph_cur = ph;
+        s += kUmmaGroups;
+        if (s >= S) {
+          s -= S;
+          ph ^= 1u;
         }
-      }
-      const uint8_t* slot = raw_s + (size_t)r_cur * 8 * KT * TB;
-      const int tile_line = (rbi * KT + within_cur) * kTileLines;      // the tile's first line in the slot
-      if (!kLateWait) tc_fence_after();          // the stage's columns were last read by MMAs whose commit was waited for
-      const int line = tile_line + (kIs8 ? 8 * h + 4 * c : 4 * h) + (g >> 1);
-      const uint8_t* wrow = slot + line * 128 + (kIs8 ? 0 : 8 * c);
-      const int chunk0 = ((g & 1) * 4) ^ (line & 7);
-      const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (64 * TERMS) + c * (32 * TERMS));
-      uint32_t sh = 0, sl = 0;
-      if constexpr (KIND != I8_ROW) {
-        // Two terms of Q4 with f16 scales: s_hi = the scale rounded to five significant bits and s_lo = the rest, which has
-        // five too (of 11, rounded to nearest).  The integers have three (or are -8), so both products are exact in bf16, and
-        // so is 24 * s: each term is one fma over 24 + q, half the instructions of the general form below.
-        // General form: the scale as s_hi + s_lo, two bf16 numbers (exact for an f16 scale: 11 = 8 + 3 significant bits).
-        // With t = q*s_lo (7 bits, exact in bf16), hi = fma(q, s_hi, t) is the exact product rounded once;
-        // lo = t - fma(q, -s_hi, hi) = q*scale - hi, both steps exact, so hi + lo reproduces the product.
-        // (f32 scales keep their first 16 significant bits this way, and with int8 values t itself is rounded to 8
-        // bits: hi + lo is then the product to within 2^-15 relative.)
-        float2 f;
-        const int s_line = tile_line + (kIs8 ? 16 : 8) + (KIND == Q4_F16 ? 0 : h);
-        if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(slot + s_line * 128 + (((4 * h + (g >> 1)) ^ (s_line & 7)) << 4) + 8 * (g & 1) + 4 * c));
-        else f = *reinterpret_cast<const float2*>(slot + s_line * 128 + ((g ^ (s_line & 7)) << 4) + 8 * c);
-        if constexpr (kExactSplit) {
-          const uint32_t h0 = (__float_as_uint(f.x) + 0x40000u) & 0xFFF80000u, h1 = (__float_as_uint(f.y) + 0x40000u) & 0xFFF80000u;
-          sh = prmt(h0, h1, 0x7632u);
-          sl = prmt(__float_as_uint(f.x - __uint_as_float(h0)), __float_as_uint(f.y - __uint_as_float(h1)), 0x7632u);
-        } else {
-        const __nv_bfloat162 shb = __floats2bfloat162_rn(f.x, f.y);
-        sh = *reinterpret_cast<const uint32_t*>(&shb);
-        const __nv_bfloat162 slb = __floats2bfloat162_rn(f.x - __uint_as_float(sh << 16), f.y - __uint_as_float(sh & 0xFFFF0000u));
-        sl = *reinterpret_cast<const uint32_t*>(&slb);
-        }
-      }
-      uint32_t wq[4][4];                         // [k quarter][word]: Q4 uses words 0, 1 (blocks 2c, 2c+1)
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        if constexpr (kIs8) {
-          const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((chunk0 ^ t) << 4));
-          wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = v.z; wq[t][3] = v.w;
-        } else {
-          const uint2 v = *reinterpret_cast<const uint2*>(wrow + ((chunk0 ^ t) << 4));
-          wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = 0u; wq[t][3] = 0u;
-        }
-      }
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        uint32_t hi[16], lo[16];
-        if constexpr (kExactSplit) {
-          const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u);
-          const uint32_t c_hi = bf16x2_mul(s_hi, 0xC1C0C1C0u), c_lo = bf16x2_mul(s_lo, 0xC1C0C1C0u);   // -24 s
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t v[4];                         // 24 + q of (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t
-            dequant_q4_word_24(wq[t][jj], v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              hi[4 * t + e] = bf16x2_fma(v[e], s_hi, c_hi);
-              lo[4 * t + e] = bf16x2_fma(v[e], s_lo, c_lo);
-            }
+        within += kUmmaGroups;
+        const bool leaves = within >= KT;           // this group's next tile lies in the next ring slot
+        if (leaves) {
+          within -= KT;
+          if (++r == RS) {
+            r = 0;
+            rph ^= 1u;
           }
-        } else {
-        const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u), minus_s_hi = s_hi ^ 0x80008000u;
+        }
+        const uint8_t* slot = raw_s + (size_t)r_cur * 8 * KT * TB;
+        const int tile_line = (rbi * KT + within_cur) * kTileLines;      // the tile's first line in the slot
+        if (!kLateWait) tc_fence_after();          // the stage's columns were last read by MMAs whose commit was waited for
+        const int line = tile_line + (kIs8 ? 8 * h + 4 * c : 4 * h) + (g >> 1);
+        const uint8_t* wrow = slot + line * 128 + (kIs8 ? 0 : 8 * c);
+        const int chunk0 = ((g & 1) * 4) ^ (line & 7);
+        const uint32_t a_t = tmem_d + ((uint32_t)(32 * q4) << 16) + (uint32_t)(p.a_col0 + s_cur * (64 * TERMS) + c * (32 * TERMS));
+        uint32_t sh = 0, sl = 0;
+        if constexpr (KIND != I8_ROW) {
+          // Two terms of Q4 with f16 scales: s_hi = the scale rounded to five significant bits and s_lo = the rest, which has
+          // five too (of 11, rounded to nearest).  The integers have three (or are -8), so both products are exact in bf16, and
+          // so is 24 * s: each term is one fma over 24 + q, half the instructions of the general form below.
+          // General form: the scale as s_hi + s_lo, two bf16 numbers (exact for an f16 scale: 11 = 8 + 3 significant bits).
+          // With t = q*s_lo (7 bits, exact in bf16), hi = fma(q, s_hi, t) is the exact product rounded once;
+          // lo = t - fma(q, -s_hi, hi) = q*scale - hi, both steps exact, so hi + lo reproduces the product.
+          // (f32 scales keep their first 16 significant bits this way, and with int8 values t itself is rounded to 8
+          // bits: hi + lo is then the product to within 2^-15 relative.)
+          float2 f;
+          const int s_line = tile_line + (kIs8 ? 16 : 8) + (KIND == Q4_F16 ? 0 : h);
+          if (KIND == Q4_F16) f = __half22float2(*reinterpret_cast<const __half2*>(slot + s_line * 128 + (((4 * h + (g >> 1)) ^ (s_line & 7)) << 4) + 8 * (g & 1) + 4 * c));
+          else f = *reinterpret_cast<const float2*>(slot + s_line * 128 + ((g ^ (s_line & 7)) << 4) + 8 * c);
+          if constexpr (kExactSplit) {
+            const uint32_t h0 = (__float_as_uint(f.x) + 0x40000u) & 0xFFF80000u, h1 = (__float_as_uint(f.y) + 0x40000u) & 0xFFF80000u;
+            sh = prmt(h0, h1, 0x7632u);
+            sl = prmt(__float_as_uint(f.x - __uint_as_float(h0)), __float_as_uint(f.y - __uint_as_float(h1)), 0x7632u);
+          } else {
+          const __nv_bfloat162 shb = __floats2bfloat162_rn(f.x, f.y);
+          sh = *reinterpret_cast<const uint32_t*>(&shb);
+          const __nv_bfloat162 slb = __floats2bfloat162_rn(f.x - __uint_as_float(sh << 16), f.y - __uint_as_float(sh & 0xFFFF0000u));
+          sl = *reinterpret_cast<const uint32_t*>(&slb);
+          }
+        }
+        uint32_t wq[4][4];                         // [k quarter][word]: Q4 uses words 0, 1 (blocks 2c, 2c+1)
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          uint32_t q[4];                         // (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t, exact ints
-          if constexpr (kIs8) dequant_i8_words(wq[t][2 * jj], wq[t][2 * jj + 1], q);
-          else dequant_q4_word(wq[t][jj], q);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if constexpr (KIND == I8_ROW) {
-              hi[4 * t + e] = q[e];
-            } else {
-              const uint32_t tt = bf16x2_mul(q[e], s_lo);
-              hi[4 * t + e] = bf16x2_fma(q[e], s_hi, tt);
-              if (TERMS == 2) lo[4 * t + e] = bf16x2_sub(tt, bf16x2_fma(q[e], minus_s_hi, hi[4 * t + e]));
-            }
+          if constexpr (kIs8) {
+            const uint4 v = *reinterpret_cast<const uint4*>(wrow + ((chunk0 ^ t) << 4));
+            wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = v.z; wq[t][3] = v.w;
+          } else {
+            const uint2 v = *reinterpret_cast<const uint2*>(wrow + ((chunk0 ^ t) << 4));
+            wq[t][0] = v.x; wq[t][1] = v.y; wq[t][2] = 0u; wq[t][3] = 0u;
           }
         }
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {
+          uint32_t hi[16], lo[16];
+          if constexpr (kExactSplit) {
+            const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u);
+            const uint32_t c_hi = bf16x2_mul(s_hi, 0xC1C0C1C0u), c_lo = bf16x2_mul(s_lo, 0xC1C0C1C0u);   // -24 s
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              uint32_t v[4];                         // 24 + q of (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t
+              dequant_q4_word_24(wq[t][jj], v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                hi[4 * t + e] = bf16x2_fma(v[e], s_hi, c_hi);
+                lo[4 * t + e] = bf16x2_fma(v[e], s_lo, c_lo);
+              }
+            }
+          } else {
+          const uint32_t s_hi = prmt(sh, sh, jj ? 0x3232u : 0x1010u), s_lo = prmt(sl, sl, jj ? 0x3232u : 0x1010u), minus_s_hi = s_hi ^ 0x80008000u;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            uint32_t q[4];                         // (k0,k1) (k2,k3) (k4,k5) (k6,k7) of k quarter t, exact ints
+            if constexpr (kIs8) dequant_i8_words(wq[t][2 * jj], wq[t][2 * jj + 1], q);
+            else dequant_q4_word(wq[t][jj], q);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if constexpr (KIND == I8_ROW) {
+                hi[4 * t + e] = q[e];
+              } else {
+                const uint32_t tt = bf16x2_mul(q[e], s_lo);
+                hi[4 * t + e] = bf16x2_fma(q[e], s_hi, tt);
+                if (TERMS == 2) lo[4 * t + e] = bf16x2_sub(tt, bf16x2_fma(q[e], minus_s_hi, hi[4 * t + e]));
+              }
+            }
+          }
+          }
+          if (kLateWait && jj == 0) {
+            // the stage's columns were last read by MMAs whose commit is waited for here
+            ok = __all_sync(0xffffffffu, mbar_wait_token(&stage_empty[s_cur * kEmptyStep], ph_cur ^ 1u, tok_empty));
+            tc_fence_after();
+          }
+          if (ok) {
+            tmem_st16(a_t + (uint32_t)(16 * jj), hi);
+            if (TERMS == 2) tmem_st16(a_t + (uint32_t)(32 + 16 * jj), lo);
+          }
         }
-        if (kLateWait && jj == 0) {
-          // the stage's columns were last read by MMAs whose commit is waited for here
-          ok = __all_sync(0xffffffffu, mbar_wait_token(&stage_empty[s_cur * kEmptyStep], ph_cur ^ 1u, tok_empty));
-          tc_fence_after();
+        if (!ok) { give_up(DERR_EMPTY_WAIT); break; }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {                                                // one arrival per warp
+          mbar_arrive(&a_full[s_cur]);
+          if (leaves) mbar_arrive(&raw_empty[r_cur]);   // done with this ring slot (nobody waits for the final ones)
         }
-        if (ok) {
-          tmem_st16(a_t + (uint32_t)(16 * jj), hi);
-          if (TERMS == 2) tmem_st16(a_t + (uint32_t)(32 + 16 * jj), lo);
+        if (ck + kUmmaGroups < kc_len) {               // early look at what this group's next stage waits for
+          tok_raw = leaves ? mbar_test(&raw_full[r], rph) : 1u;
+          tok_empty = mbar_test(&stage_empty[s * kEmptyStep], ph ^ 1u);
         }
       }
-      if (!ok) { give_up(DERR_EMPTY_WAIT); break; }
-      tmem_st_wait();
+      if (shared_tail && stop == kc_len && from < kc_len && group == 0 && lane == 0) mbar_arrive(a_tail);   // (the last chunk was this group's)
+      if (!RUNS || !ok || (run + 1) * p.run_kc >= kc_len) break;
+      ok = __all_sync(0xffffffffu, mbar_wait_spin(acc_full, run & 1));
+      if (!ok) break;
+      tc_fence_after();
+      for (int c0 = col0; c0 < ntok; c0 += kColStep) {
+        float v[16];
+        sum_accumulators(tmem_lanes, p, c0, p.run_kc, p.run_kc, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sums[(c0 + i) * kUmmaRows] = run ? sums[(c0 + i) * kUmmaRows] + v[i] : v[i];
+      }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {                                                // one arrival per warp
-        mbar_arrive(&a_full[s_cur]);
-        if (leaves) mbar_arrive(&raw_empty[r_cur]);   // done with this ring slot (nobody waits for the final ones)
-      }
-      if (ck + kUmmaGroups < kc_len) {               // early look at what this group's next stage waits for
-        tok_raw = leaves ? mbar_test(&raw_full[r], rph) : 1u;
-        tok_empty = mbar_test(&stage_empty[s * kEmptyStep], ph ^ 1u);
-      }
-    }
-    if (shared_tail && stop == kc_len && from < kc_len && group == 0 && lane == 0) mbar_arrive(a_tail);   // (the last chunk was this group's)
-    if (!RUNS || !ok || (run + 1) * p.run_kc >= kc_len) break;
-    ok = __all_sync(0xffffffffu, mbar_wait_spin(acc_full, run & 1));
-    if (!ok) break;
-    tc_fence_after();
-    for (int c0 = col0; c0 < ntok; c0 += kColStep) {
-      float v[16];
-      sum_accumulators(tmem_lanes, p, c0, p.run_kc, p.run_kc, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) sums[(c0 + i) * kUmmaRows] = run ? sums[(c0 + i) * kUmmaRows] + v[i] : v[i];
-    }
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(acc_free);
-    ++run;
+      if (lane == 0) mbar_arrive(acc_free);
+      ++run;
     }
     // ---- epilogue: D[128 features x ntok tokens] -> y[token][feature]
     if (ok && !*failed) ok = mbar_wait_spin(acc_full, run & 1);
